@@ -14,9 +14,10 @@
 #include <vector>
 
 #include "../../include/es_gb300.h"
+#include "es_cascade.h"
 #include "es_internal.h"
 
-typedef unsigned __int128 u128;
+typedef es_u128 u128;
 
 namespace {
 
@@ -37,14 +38,6 @@ int cuda_fail(cudaError_t e, const char* what) {
         cudaError_t _e = (call);                             \
         if (_e != cudaSuccess) return cuda_fail(_e, what);   \
     } while (0)
-
-u128 mk(uint64_t lo, uint64_t hi) { return ((u128)hi << 64) | lo; }
-uint32_t bitlen128(u128 x) {
-    uint32_t n = 0;
-    while (x) { ++n; x >>= 1; }
-    return n;
-}
-uint32_t mod_q(u128 x, uint32_t q) { return (uint32_t)(x % q); }
 
 struct DeviceFacts {
     int dev = -1;
@@ -73,8 +66,6 @@ int device_facts() {
     g_dev.prepared = true;
     return ES_OK;
 }
-
-size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 int check_tune(const es_tune& t) {
     if (t.layout > ES_LAYOUT_AUTO)
@@ -106,15 +97,31 @@ es_tune default_tune() {
 }  // namespace
 
 // ------------------------------------------------------------------------------------------
+namespace {
+
+// One set of device tables of a plan: the header and its arena.
+struct TableSet {
+    EsInst h{};
+    EsInst* d = nullptr;
+    unsigned char* arena = nullptr;
+    uint64_t bytes = 0;
+};
+
+struct ProdSet {
+    TableSet t;
+    std::vector<EsCascadeEntry> entries;
+};
+
+}  // namespace
+
 struct es_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     es_tune tune{};
-    EsInst h_inst{};
-    EsInst* d_inst = nullptr;
-    unsigned char* d_arena = nullptr;
-    size_t arena_bytes = 0;
-    uint64_t table_bytes = 0;
+    EsHostPlan plan;
+    EsInst geo{};                 // geometry only (rings, filter count, M)
+    TableSet caller;              // caller's cascade order: counting and scalar launches
+    ProdSet prod[ES_PMAX + 1];    // production cascade by inner tables
     std::vector<uint32_t> q;
     u128 M = 1;
     uint32_t tconst[ES_MAX_FILTERS] = {0};
@@ -188,9 +195,9 @@ SmemPlan plan_smem(uint32_t small_max, uint32_t nf_max, const es_tune& tune, uin
     // per-warp stage counters exist only in counting launches; shared memory is kept small so
     // that the CUDA driver's carveout leaves the rest of the SM's 256 KB to L1 (the phase tables),
     // unless the launch stages those tables in shared memory itself
-    const uint32_t counters = tune.count_stages ? (uint32_t)align_up(4ull * nf_max * warps, 16) : 0u;
+    const uint32_t counters = tune.count_stages ? (uint32_t)es_align_up(4ull * nf_max * warps, 16) : 0u;
     p.stage_off = small_max;
-    p.cnt_off = p.stage_off + (uint32_t)align_up(4ull * stage_words, 16);
+    p.cnt_off = p.stage_off + (uint32_t)es_align_up(4ull * stage_words, 16);
     p.queue_off = p.cnt_off + counters;
     p.bytes = p.queue_off + queues;
     return p;
@@ -204,9 +211,6 @@ uint32_t staged_words(uint32_t layout, uint32_t mask_words) {
     if (layout == ES_LAYOUT_SMEM_PAIR) return 2u * mask_words;
     return 0u;
 }
-
-// Launches per batch: four width classes, each split into staged and unstaged plans.
-constexpr uint32_t kMaxSubs = 8;
 
 // Word-mask bytes of the inner-stage tables that fit the L1 beside the scan's own shared memory.
 constexpr uint32_t kL1TableBudget = 180u * 1024u;
@@ -275,6 +279,34 @@ uint64_t units_of(const EsInst& I, uint64_t cb, uint64_t ce, uint32_t strip) {
     return (rows + 31) / 32 * ((I.r2 + strip - 1) / strip);
 }
 
+// Launches that count no stages run the production cascade, in every layout but the scalar one
+// (the layouts are forms of the caller's cascade; none changes which candidates pass).
+bool is_production(const es_tune& t) { return !t.count_stages && t.layout != ES_LAYOUT_SCALAR; }
+
+// Inner tables of a production launch.
+uint32_t prod_tables(const es_tune& t) { return std::min<uint32_t>(std::max<uint32_t>(t.mask_filters, 1), ES_PMAX); }
+
+// The production cascade's block constants from the caller's.
+void prod_tconst(const ProdSet& S, const uint32_t* tconst, uint32_t* out) {
+    for (size_t i = 0; i < S.entries.size(); ++i) {
+        const EsCascadeEntry& e = S.entries[i];
+        uint64_t r = 0;
+        for (const EsCascadeEntry::Part& p : e.parts) {
+            const uint64_t x = tconst[p.f] % p.d;
+            r = (r + x * p.unit) % e.q;
+        }
+        out[i] = (uint32_t)r;
+    }
+}
+
+// tconst[j] = (t mod q)(M mod q) mod q
+void block_tconst(const es_ctx* c, uint64_t t, uint32_t* out) {
+    for (size_t f = 0; f < c->q.size(); ++f) {
+        const uint64_t q = c->q[f];
+        out[f] = (uint32_t)((t % q) * (uint64_t)(c->M % q) % q);
+    }
+}
+
 }  // namespace
 
 void es_set_last_error(const char* msg) { g_err = msg ? msg : ""; }
@@ -314,7 +346,8 @@ int es_device_name(char* out, uint32_t cap) {
 int es_ctx_destroy(es_ctx* c) {
     if (!c) return ES_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    cudaFree(c->d_arena);
+    cudaFree(c->caller.arena);
+    for (ProdSet& p : c->prod) cudaFree(p.t.arena);
     cudaFree(c->d_counts);
     cudaFree(c->d_surv);
     cudaFree(c->d_surv_n);
@@ -327,169 +360,131 @@ int es_ctx_destroy(es_ctx* c) {
     return ES_OK;
 }
 
-int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
-    if (!d || !out) return fail(ES_ERR_ARG, "null descriptor or output pointer");
-    *out = nullptr;
-    es_tune tune = tune_in ? *tune_in : default_tune();
-    if (int e = check_tune(tune)) return e;
-    if (d->flags != 0) return fail(ES_ERR_ARG, "descriptor flags must be 0");
-    const u128 M = mk(d->M_lo, d->M_hi);
-    if (M == 0 || bitlen128(M) > 126) return fail(ES_ERR_RANGE, "wheel modulus must be in [1, 2^126)");
-    if (d->n_filters > ES_MAX_FILTERS)
-        return fail(ES_ERR_RANGE, "too many residual filters (max " + std::to_string(ES_MAX_FILTERS) + ")");
-    if (d->n_rings > ES_MAX_RINGS - 3) return fail(ES_ERR_RANGE, "too many wheel rings");
-    if (d->n_rings && (!d->radix || !d->term_lo || !d->term_hi))
-        return fail(ES_ERR_ARG, "null ring arrays");
-    if (d->n_filters && (!d->filter_q || !d->allowed)) return fail(ES_ERR_ARG, "null filter arrays");
-    if (int e = device_facts()) return e;
+// Uploads one table set: the header, the small block, the inner-stage tables and the bit tables
+// (ring terms too) in one arena.
+static int upload_set(es_ctx* c, TableSet& T, const std::vector<unsigned char>& small, const std::vector<uint32_t>& masks,
+                      const std::vector<uint32_t>& pairs, const std::vector<uint32_t>& bits) {
+    const EsHostPlan& P = c->plan;
+    size_t aoff = 0;
+    auto atake = [&](size_t bytes) { size_t o = aoff; aoff = es_align_up(aoff + bytes, 256); return o; };
+    const size_t a_inst = atake(sizeof(EsInst));
+    const size_t a_small = atake(small.size());
+    const size_t a_masks = atake(4ull * std::max<size_t>(masks.size(), 4));
+    const size_t a_pairs = atake(4ull * std::max<size_t>(pairs.size(), 4));
+    const size_t a_bits = atake(4ull * std::max<size_t>(bits.size(), 4));
+    const size_t a_terms = atake(16ull * P.terms.size());
+    const size_t a_roff = atake(4ull * P.roff.size());
+    const size_t a_radix = atake(4ull * P.radix.size());
+    std::vector<unsigned char> img(aoff, 0);
+    memcpy(&img[a_small], small.data(), small.size());
+    if (!masks.empty()) memcpy(&img[a_masks], masks.data(), 4ull * masks.size());
+    if (!pairs.empty()) memcpy(&img[a_pairs], pairs.data(), 4ull * pairs.size());
+    if (!bits.empty()) memcpy(&img[a_bits], bits.data(), 4ull * bits.size());
+    for (size_t i = 0; i < P.terms.size(); ++i) {
+        uint64_t lo = (uint64_t)P.terms[i], hi = (uint64_t)(P.terms[i] >> 64);
+        memcpy(&img[a_terms + 16 * i], &lo, 8);
+        memcpy(&img[a_terms + 16 * i + 8], &hi, 8);
+    }
+    memcpy(&img[a_roff], P.roff.data(), 4ull * P.roff.size());
+    memcpy(&img[a_radix], P.radix.data(), 4ull * P.radix.size());
+    unsigned char* arena = nullptr;
+    ES_CUDA(cudaMalloc(&arena, aoff), "cudaMalloc(arena)");
+    EsInst& I = T.h;
+    I.small = arena + a_small;
+    I.masks = reinterpret_cast<const uint32_t*>(arena + a_masks);
+    I.pairs = reinterpret_cast<const uint32_t*>(arena + a_pairs);
+    I.allowed = reinterpret_cast<const uint32_t*>(arena + a_bits);
+    I.ring_terms = reinterpret_cast<const uint64_t*>(arena + a_terms);
+    I.ring_off = reinterpret_cast<const uint32_t*>(arena + a_roff);
+    I.radix = reinterpret_cast<const uint32_t*>(arena + a_radix);
+    memcpy(&img[a_inst], &I, sizeof(EsInst));
+    const cudaError_t ce = cudaMemcpy(arena, img.data(), aoff, cudaMemcpyHostToDevice);
+    if (ce != cudaSuccess) {
+        cudaFree(arena);
+        return cuda_fail(ce, "table upload");
+    }
+    T.arena = arena;
+    T.d = reinterpret_cast<EsInst*>(arena + a_inst);
+    T.bytes = aoff;
+    return ES_OK;
+}
 
-    // ---- rings (padded to >= 3 with radix-1 rings whose only term is 0) -------------------
-    std::vector<uint32_t> radix;
-    std::vector<u128> terms;
-    std::vector<uint32_t> roff;
-    uint64_t R = 1;
-    size_t pos = 0;
-    for (uint32_t j = 0; j < d->n_rings; ++j) {
-        const uint32_t r = d->radix[j];
-        if (r == 0 || r > 65535) return fail(ES_ERR_RANGE, "ring radix must be in [1, 65535]");
-        roff.push_back((uint32_t)terms.size());
-        radix.push_back(r);
-        for (uint32_t i = 0; i < r; ++i, ++pos) {
-            const u128 v = mk(d->term_lo[pos], d->term_hi[pos]);
-            if (v >= M) return fail(ES_ERR_ARG, "ring term not reduced mod M");
-            terms.push_back(v);
-        }
-        if (R > (1ull << 62) / r) return fail(ES_ERR_RANGE, "residues per block exceed 2^62");
-        R *= r;
-    }
-    while (radix.size() < 3) {
-        roff.push_back((uint32_t)terms.size());
-        radix.push_back(1);
-        terms.push_back(0);
-    }
-    const uint32_t nr = (uint32_t)radix.size();
-    const uint32_t r0 = radix[0], r1 = radix[1], r2 = radix[2];
-    const uint32_t nf = d->n_filters;
+// Tables of the caller's cascade order (counting launches and the scalar layout).
+static int build_caller(es_ctx* c) {
+    const EsHostPlan& P = c->plan;
+    TableSet T;
+    EsInst& I = T.h;
+    I = c->geo;
+    const u128 M = P.M;
+    const uint32_t r0 = I.r0, r1 = I.r1, r2 = I.r2, W = I.W, nf = I.n_filters, sh = I.sh;
     const uint32_t FB = std::min<uint32_t>(ES_FMAX, nf);
-    const uint32_t W = (r0 + 31) / 32;
-
-    es_ctx* c = new (std::nothrow) es_ctx();
-    if (!c) return fail(ES_ERR_NOMEM, "host allocation");
-    c->tune = tune;
-    c->M = M;
-    c->q.assign(d->filter_q, d->filter_q + nf);
-
-    // ---- filters ------------------------------------------------------------------------
     std::vector<EsFilterC> fc(nf);
-    std::vector<uint32_t> bit_off(nf + 1, 0);
-    for (uint32_t f = 0; f < nf; ++f) {
-        const uint32_t q = c->q[f];
-        if (q < 2 || q >= ES_MAX_Q) {
-            es_ctx_destroy(c);
-            return fail(ES_ERR_RANGE, "filter modulus must be in [2, 2^20)");
-        }
-        bit_off[f + 1] = bit_off[f] + (q + 31) / 32;
-        fc[f].q = q;
-        fc[f].corr = (uint32_t)((q - mod_q(M, q)) % q);
-        fc[f].w1 = mod_q((u128)1 << 32, q);
-        fc[f].w2 = mod_q((u128)1 << 64, q);
-        fc[f].w3 = mod_q((u128)1 << 96, q);
-        fc[f].off = bit_off[f];
-        fc[f].rcp = (uint64_t)(((u128)1 << 64) / q);
-    }
-    auto admissible = [&](uint32_t f, uint32_t r) -> uint32_t {
-        return (d->allowed[bit_off[f] + (r >> 5)] >> (r & 31u)) & 1u;
-    };
-
-    // ---- inner ring: sorted slots, keys, buckets ----------------------------------------
-    std::vector<uint32_t> order(r0);
-    for (uint32_t i = 0; i < r0; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(),
-                     [&](uint32_t a, uint32_t b) { return terms[roff[0] + a] < terms[roff[0] + b]; });
-    std::vector<u128> S0(r0);
-    for (uint32_t i = 0; i < r0; ++i) S0[i] = terms[roff[0] + order[i]];
-    const uint32_t bl = bitlen128(M);
-    const uint32_t sh = bl > 32 ? bl - 32 : 0;
-    const uint32_t kbits = bitlen128(M >> sh);
+    for (uint32_t f = 0; f < nf; ++f) fc[f] = es_filter_consts(M, P.q[f], P.bit_off[f]);
+    const EsSortedRing R = es_sort_inner(P);
+    const uint32_t kbits = es_bitlen(M >> sh);
     const uint32_t bsh = kbits > ES_NBUCKET_LOG2 ? kbits - ES_NBUCKET_LOG2 : 0;
     std::vector<uint32_t> K0(r0);
-    for (uint32_t i = 0; i < r0; ++i) K0[i] = (uint32_t)(S0[i] >> sh);
+    for (uint32_t i = 0; i < r0; ++i) K0[i] = (uint32_t)(R.S0[i] >> sh);
     // bucket b: the first sorted slot whose key is >= b << bsh, and the keys of that slot and
     // the next two (0xffffffff past the end), so that one 16-byte load settles the split
     std::vector<uint32_t> BK(4ull * (ES_NBUCKET + 1));
-    for (uint32_t bkt = 0; bkt <= ES_NBUCKET; ++bkt) {
+    for (uint32_t bkt = 0, n = 0; bkt <= ES_NBUCKET; ++bkt) {
         const uint64_t lim = (uint64_t)bkt << bsh;
-        uint32_t n = 0;
         while (n < r0 && (uint64_t)K0[n] < lim) ++n;
         BK[4 * bkt] = n;
         for (uint32_t j = 0; j < 3; ++j) BK[4 * bkt + 1 + j] = n + j < r0 ? K0[n + j] : 0xffffffffu;
     }
-
     // ---- small block ----------------------------------------------------------------------
-    EsInst& I = c->h_inst;
-    size_t off = 0;
-    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 16); return (uint32_t)o; };
-    I.o_T1 = take(16ull * r1);
-    I.o_TQ1 = take(4ull * ES_FMAX * r1);
-    I.o_D2 = take(16ull * r2);
-    I.o_DQ2 = take(4ull * ES_FMAX * r2);
-    I.o_S0 = take(16ull * (r0 + 1));   // + sentinel S0[r0] = M
-    I.o_K0 = take(4ull * (r0 + 1));    // + sentinel K0[r0] = 0xffffffff
-    I.o_I0 = take(4ull * r0);
-    I.o_Q0 = take(4ull * ES_FMAX * r0);
-    I.o_BK = take(16ull * (ES_NBUCKET + 1));
-    I.o_FC = take(sizeof(EsFilterC) * std::max<uint32_t>(nf, 1));
-    I.o_K1 = take(4ull * r1);
-    const size_t small_bytes = off;
-    std::vector<unsigned char> small(small_bytes, 0);
-    auto put128 = [&](uint32_t o, uint32_t i, u128 v) {
-        uint64_t lo = (uint64_t)v, hi = (uint64_t)(v >> 64);
-        memcpy(&small[o + 16ull * i], &lo, 8);
-        memcpy(&small[o + 16ull * i + 8], &hi, 8);
-    };
-    auto put32 = [&](uint32_t o, uint32_t i, uint32_t v) { memcpy(&small[o + 4ull * i], &v, 4); };
+    EsSmallBlock S;
+    I.o_T1 = S.take(16ull * r1);
+    I.o_TQ1 = S.take(4ull * ES_FMAX * r1);
+    I.o_D2 = S.take(16ull * r2);
+    I.o_DQ2 = S.take(4ull * ES_FMAX * r2);
+    I.o_S0 = S.take(16ull * (r0 + 1));   // + sentinel S0[r0] = M
+    I.o_K0 = S.take(4ull * (r0 + 1));    // + sentinel K0[r0] = 0xffffffff
+    I.o_I0 = S.take(4ull * r0);
+    I.o_Q0 = S.take(4ull * ES_FMAX * r0);
+    I.o_BK = S.take(16ull * (ES_NBUCKET + 1));
+    I.o_FC = S.take(sizeof(EsFilterC) * std::max<uint32_t>(nf, 1));
+    I.o_K1 = S.take(4ull * r1);
     for (uint32_t i = 0; i < r1; ++i) {
-        const u128 v = terms[roff[1] + i];
-        put128(I.o_T1, i, v);
-        put32(I.o_K1, i, (uint32_t)(v >> sh));
-        for (uint32_t f = 0; f < FB; ++f) put32(I.o_TQ1, i * ES_FMAX + f, mod_q(v, c->q[f]));
+        const u128 v = P.terms[P.roff[1] + i];
+        S.put128(I.o_T1, i, v);
+        S.put32(I.o_K1, i, (uint32_t)(v >> sh));
+        for (uint32_t f = 0; f < FB; ++f) S.put32(I.o_TQ1, i * ES_FMAX + f, es_mod(v, P.q[f]));
     }
     for (uint32_t i = 0; i < r2; ++i) {
-        const u128 a = terms[roff[2] + i], b = terms[roff[2] + (i + 1) % r2];
-        const u128 dlt = b >= a ? b - a : b + (M - a);
-        put128(I.o_D2, i, dlt);
-        for (uint32_t f = 0; f < FB; ++f) put32(I.o_DQ2, i * ES_FMAX + f, mod_q(dlt, c->q[f]));
+        const u128 dlt = es_ring2_delta(P, i);
+        S.put128(I.o_D2, i, dlt);
+        for (uint32_t f = 0; f < FB; ++f) S.put32(I.o_DQ2, i * ES_FMAX + f, es_mod(dlt, P.q[f]));
     }
     for (uint32_t i = 0; i < r0; ++i) {
-        put128(I.o_S0, i, S0[i]);
-        put32(I.o_K0, i, K0[i]);
-        put32(I.o_I0, i, order[i]);
-        for (uint32_t f = 0; f < FB; ++f) put32(I.o_Q0, f * r0 + i, mod_q(S0[i], c->q[f]));
+        S.put128(I.o_S0, i, R.S0[i]);
+        S.put32(I.o_K0, i, K0[i]);
+        S.put32(I.o_I0, i, R.digit[i]);
+        for (uint32_t f = 0; f < FB; ++f) S.put32(I.o_Q0, (size_t)f * r0 + i, es_mod(R.S0[i], P.q[f]));
     }
-    put128(I.o_S0, r0, M);             // stops the tie scan: M < thr never holds (thr <= M)
-    put32(I.o_K0, r0, 0xffffffffu);    // stops the key scan: never < t32
-    memcpy(&small[I.o_BK], BK.data(), 16ull * (ES_NBUCKET + 1));
-    if (nf) memcpy(&small[I.o_FC], fc.data(), sizeof(EsFilterC) * nf);
+    S.put128(I.o_S0, r0, M);             // stops the tie scan: M < thr never holds (thr <= M)
+    S.put32(I.o_K0, r0, 0xffffffffu);    // stops the key scan: never < t32
+    memcpy(&S.b[I.o_BK], BK.data(), 16ull * (ES_NBUCKET + 1));
+    if (nf) memcpy(&S.b[I.o_FC], fc.data(), sizeof(EsFilterC) * nf);
 
     // ---- word-mask phase tables for the first FB filters ---------------------------------
-    // rows of RS words: W, except three-word rings, whose rows are padded to four words so that
-    // one 16-byte load reads a row
-    const uint32_t RS = W == 3 ? 4u : W;
+    const uint32_t RS = es_row_words(W);
     std::vector<uint32_t> mask_off(ES_FMAX + 1, 0);
     for (uint32_t f = 0; f < ES_FMAX; ++f)
-        mask_off[f + 1] = mask_off[f] + (f < FB ? (uint32_t)align_up((uint64_t)c->q[f] * RS, 4) : 0u);
+        mask_off[f + 1] = mask_off[f] + (f < FB ? (uint32_t)es_align_up((uint64_t)P.q[f] * RS, 4) : 0u);
     std::vector<uint32_t> masks(std::max<uint32_t>(mask_off[ES_FMAX], 4), 0u);
+    std::vector<uint8_t> adm;
     for (uint32_t f = 0; f < FB; ++f) {
-        const uint32_t q = c->q[f];
-        uint32_t* P = masks.data() + mask_off[f];
+        const uint32_t q = P.q[f];
+        adm.assign(q, 0);
+        for (uint32_t r = 0; r < q; ++r) adm[r] = (P.allowed[P.bit_off[f] + (r >> 5)] >> (r & 31u)) & 1u;
+        uint32_t* D = masks.data() + mask_off[f];
         for (uint32_t i = 0; i < r0; ++i) {
-            const uint32_t a = mod_q(S0[i], q);
-            const uint32_t wd = i >> 5, bit = 1u << (i & 31u);
-            uint32_t r = a;
-            for (uint32_t ph = 0; ph < q; ++ph) {
-                if (admissible(f, r)) P[(uint64_t)ph * RS + wd] |= bit;
-                if (++r == q) r = 0;
-            }
+            const uint32_t a = es_mod(R.S0[i], q), wd = i >> 5, at = i & 31u;
+            for (uint32_t ph = 0; ph < q - a; ++ph) D[(uint64_t)ph * RS + wd] |= (uint32_t)adm[ph + a] << at;
+            for (uint32_t ph = q - a; ph < q; ++ph) D[(uint64_t)ph * RS + wd] |= (uint32_t)adm[ph + a - q] << at;
         }
     }
     // pair tables (inner rings of at most two words): phase row phi holds P_f[phi] and then the
@@ -499,75 +494,81 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     if (W <= 2) {
         pairs.assign(2ull * masks.size(), 0u);
         for (uint32_t f = 0; f < FB; ++f) {
-            const uint32_t q = c->q[f], corr = fc[f].corr;
-            const uint32_t* P = masks.data() + mask_off[f];
+            const uint32_t q = P.q[f], corr = fc[f].corr;
+            const uint32_t* D0 = masks.data() + mask_off[f];
             uint32_t* D = pairs.data() + 2ull * mask_off[f];
             for (uint32_t ph = 0; ph < q; ++ph) {
-                const uint32_t ph1 = (uint32_t)(((uint64_t)ph + corr) % q);
+                const uint32_t ph1 = ph + corr >= q ? ph + corr - q : ph + corr;
                 for (uint32_t wd = 0; wd < W; ++wd) {
-                    D[(uint64_t)ph * 2 * W + wd] = P[(uint64_t)ph * W + wd];
-                    D[(uint64_t)ph * 2 * W + W + wd] = P[(uint64_t)ph1 * W + wd];
+                    D[(uint64_t)ph * 2 * W + wd] = D0[(uint64_t)ph * W + wd];
+                    D[(uint64_t)ph * 2 * W + W + wd] = D0[(uint64_t)ph1 * W + wd];
                 }
             }
         }
     }
-
-    // ---- arena ----------------------------------------------------------------------------
-    size_t aoff = 0;
-    auto atake = [&](size_t bytes) { size_t o = aoff; aoff = align_up(aoff + bytes, 256); return o; };
-    const size_t a_inst = atake(sizeof(EsInst));
-    const size_t a_small = atake(small_bytes);
-    const size_t a_masks = atake(4ull * masks.size());
-    const size_t a_pairs = atake(4ull * std::max<size_t>(pairs.size(), 4));
-    const size_t a_bits = atake(4ull * std::max<uint32_t>(bit_off[nf], 4));
-    const size_t a_terms = atake(16ull * terms.size());
-    const size_t a_roff = atake(4ull * nr);
-    const size_t a_radix = atake(4ull * nr);
-    c->arena_bytes = aoff;
-    std::vector<unsigned char> img(aoff, 0);
-    memcpy(&img[a_small], small.data(), small_bytes);
-    memcpy(&img[a_masks], masks.data(), 4ull * masks.size());
-    if (!pairs.empty()) memcpy(&img[a_pairs], pairs.data(), 4ull * pairs.size());
-    if (bit_off[nf]) memcpy(&img[a_bits], d->allowed, 4ull * bit_off[nf]);
-    for (size_t i = 0; i < terms.size(); ++i) {
-        uint64_t lo = (uint64_t)terms[i], hi = (uint64_t)(terms[i] >> 64);
-        memcpy(&img[a_terms + 16 * i], &lo, 8);
-        memcpy(&img[a_terms + 16 * i + 8], &hi, 8);
-    }
-    memcpy(&img[a_roff], roff.data(), 4ull * nr);
-    memcpy(&img[a_radix], radix.data(), 4ull * nr);
-
-    cudaError_t ce = cudaMalloc(&c->d_arena, aoff);
-    if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "cudaMalloc(arena)"); }
-    I.M_lo = (uint64_t)M;
-    I.M_hi = (uint64_t)(M >> 64);
-    I.n_outer = R / r0;
-    I.n_cycles = I.n_outer / r1;
-    I.k = d->k;
-    I.n_rings = nr;
-    I.r0 = r0; I.W = W; I.r1 = r1; I.r2 = r2;
-    I.n_filters = nf;
     I.F_built = FB;
-    I.sh = sh;
     I.bsh = bsh;
-    I.tail_mask = (r0 % 32) ? ((1u << (r0 % 32)) - 1u) : 0xffffffffu;
-    I.km = (uint32_t)(M >> sh);
-    I.small_bytes = (uint32_t)small_bytes;
+    I.small_bytes = (uint32_t)S.b.size();
     for (uint32_t f = 0; f <= ES_FMAX; ++f) I.mask_off[f] = mask_off[f];
     I.mask_stride = RS;
-    I.small = c->d_arena + a_small;
-    I.masks = reinterpret_cast<const uint32_t*>(c->d_arena + a_masks);
-    I.pairs = reinterpret_cast<const uint32_t*>(c->d_arena + a_pairs);
-    I.allowed = reinterpret_cast<const uint32_t*>(c->d_arena + a_bits);
-    I.ring_terms = reinterpret_cast<const uint64_t*>(c->d_arena + a_terms);
-    I.ring_off = reinterpret_cast<const uint32_t*>(c->d_arena + a_roff);
-    I.radix = reinterpret_cast<const uint32_t*>(c->d_arena + a_radix);
-    memcpy(&img[a_inst], &I, sizeof(EsInst));
-    c->d_inst = reinterpret_cast<EsInst*>(c->d_arena + a_inst);
-    c->table_bytes = aoff;
+    if (int e = upload_set(c, T, S.b, masks, pairs, P.allowed)) return e;
+    c->caller = T;
+    return ES_OK;
+}
 
-    ce = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaMemcpy(c->d_arena, img.data(), aoff, cudaMemcpyHostToDevice);
+// Tables of the production cascade with F inner tables.
+static int build_prod(es_ctx* c, uint32_t F) {
+    EsProdImage img;
+    // beside the staged tables: the static shared memory, and the slots of the largest CTA's warps
+    es_prod_image(c->plan, c->geo, F, (uint32_t)g_dev.smem_optin - 2048u - 16u * ES_QUEUE_BYTES, img);
+    TableSet T;
+    T.h = img.inst;
+    if (int e = upload_set(c, T, img.small, img.tabs, {}, img.bits)) return e;
+    c->prod[F].t = T;
+    c->prod[F].entries = std::move(img.entries);
+    return ES_OK;
+}
+
+// Builds the table sets that launches of this shape read, unless they are there already.
+static int ensure_tables(es_ctx* c, const es_tune& t) {
+    try {
+        const uint32_t F = prod_tables(t);
+        if (!c->prod[F].t.d)
+            if (int e = build_prod(c, F)) return e;   // es_search_blocks_static never counts
+        if (!is_production(t) && !c->caller.d)
+            if (int e = build_caller(c)) return e;
+    } catch (const std::bad_alloc&) {
+        return fail(ES_ERR_NOMEM, "host allocation");
+    }
+    return ES_OK;
+}
+
+int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
+    if (!d || !out) return fail(ES_ERR_ARG, "null descriptor or output pointer");
+    *out = nullptr;
+    es_tune tune = tune_in ? *tune_in : default_tune();
+    if (int e = check_tune(tune)) return e;
+    std::string bad;
+    if (int code = es_check_desc(*d, bad)) return fail(code, bad);
+    if (int e = device_facts()) return e;
+
+    es_ctx* c = new (std::nothrow) es_ctx();
+    if (!c) return fail(ES_ERR_NOMEM, "host allocation");
+    std::string why;
+    if (int code = es_parse_plan(*d, c->plan, c->geo, why)) {
+        es_ctx_destroy(c);
+        return fail(code, why);
+    }
+    const uint32_t nf = d->n_filters;
+    c->tune = tune;
+    c->M = c->plan.M;
+    c->q = c->plan.q;
+    int e = ensure_tables(c, tune);
+    if (e) {
+        es_ctx_destroy(c);
+        return e;
+    }
+    cudaError_t ce = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaEventCreate(&c->ev0);
     if (ce == cudaSuccess) ce = cudaEventCreate(&c->ev1);
     if (ce == cudaSuccess) ce = cudaMalloc(&c->d_counts, 8ull * std::max<uint32_t>(nf, 1));
@@ -582,15 +583,66 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     c->d_min = c->d_surv_n + 3;
     ce = cudaMemset(c->d_found, 0xff, 8);
     if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "context setup"); }
-    int e = es_set_capacity(c, 1u << 20);
+    e = es_set_capacity(c, 1u << 20);
     if (e) { es_ctx_destroy(c); return e; }
     *out = c;
+    return ES_OK;
+}
+
+int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes, es_cascade_info* info, void* small,
+                     uint64_t small_cap, uint32_t* tabs, uint64_t tabs_cap, uint32_t* parts, uint64_t parts_cap) {
+    if (!d || !info) return fail(ES_ERR_ARG, "null argument");
+    if (tables < 1 || tables > ES_PMAX) return fail(ES_ERR_ARG, "tables must be in 1..6");
+    std::string why;
+    EsHostPlan P;
+    EsInst geo{};
+    if (int code = es_check_desc(*d, why)) return fail(code, why);
+    if (int code = es_parse_plan(*d, P, geo, why)) return fail(code, why);
+    EsProdImage img;
+    try {
+        es_prod_image(P, geo, tables, smem_bytes, img);
+    } catch (const std::bad_alloc&) {
+        return fail(ES_ERR_NOMEM, "host allocation");
+    }
+    const EsInst& I = img.inst;
+    memset(info, 0, sizeof(*info));
+    info->n_entries = I.n_filters;
+    info->row_bytes = I.row_bytes;
+    info->key_shift = I.sh;
+    info->bucket_shift = I.bsh;
+    info->band = I.band;
+    info->o_row1 = I.o_R1;
+    info->row1_bytes = tables <= 3 ? 16u : 32u;
+    info->o_terms1 = I.o_T1;
+    info->o_sorted = I.o_S0;
+    info->o_digits = I.o_I0;
+    info->o_buckets = I.o_BK;
+    info->small_bytes = img.small.size();
+    info->tab_words = img.tabs.size();
+    for (uint32_t i = 0; i < tables; ++i) {
+        info->tab_base[i] = I.tab_base[i];
+        info->tab_wrap[i] = I.tab_wrap[i];
+    }
+    uint64_t np = 0;
+    for (uint32_t i = 0; i < img.entries.size(); ++i)
+        for (const EsCascadeEntry::Part& p : img.entries[i].parts) {
+            if (parts && 3 * np + 2 < parts_cap) {
+                parts[3 * np] = i;
+                parts[3 * np + 1] = p.f;
+                parts[3 * np + 2] = p.d;
+            }
+            ++np;
+        }
+    info->n_parts = np;
+    if (small && small_cap >= img.small.size()) memcpy(small, img.small.data(), img.small.size());
+    if (tabs && tabs_cap >= img.tabs.size()) memcpy(tabs, img.tabs.data(), 4ull * img.tabs.size());
     return ES_OK;
 }
 
 int es_ctx_set_tune(es_ctx* c, const es_tune* t) {
     if (!c || !t) return fail(ES_ERR_ARG, "null argument");
     if (int e = check_tune(*t)) return e;
+    if (int e = ensure_tables(c, *t)) return e;
     c->tune = *t;
     return ES_OK;
 }
@@ -604,10 +656,13 @@ int es_ctx_get_tune(const es_ctx* c, es_tune* t) {
 int es_ctx_info(const es_ctx* c, uint64_t* n_outer, uint32_t* r0, uint32_t* n_filters,
                 uint64_t* table_bytes) {
     if (!c) return fail(ES_ERR_ARG, "null context");
-    if (n_outer) *n_outer = c->h_inst.n_outer;
-    if (r0) *r0 = c->h_inst.r0;
-    if (n_filters) *n_filters = c->h_inst.n_filters;
-    if (table_bytes) *table_bytes = c->table_bytes;
+    if (n_outer) *n_outer = c->geo.n_outer;
+    if (r0) *r0 = c->geo.r0;
+    if (n_filters) *n_filters = c->geo.n_filters;
+    if (table_bytes) {
+        *table_bytes = c->caller.bytes;
+        for (const ProdSet& p : c->prod) *table_bytes += p.t.bytes;
+    }
     return ES_OK;
 }
 
@@ -623,7 +678,7 @@ int es_set_capacity(es_ctx* c, uint64_t cap) {
 
 int es_set_block(es_ctx* c, const uint32_t* tconst, uint32_t n, uint64_t t) {
     if (!c) return fail(ES_ERR_ARG, "null context");
-    if (n != c->h_inst.n_filters || (n && !tconst))
+    if (n != c->geo.n_filters || (n && !tconst))
         return fail(ES_ERR_ARG, "tconst length must equal the number of filters");
     for (uint32_t f = 0; f < n; ++f) {
         if (tconst[f] >= c->q[f]) return fail(ES_ERR_ARG, "tconst[j] must be < q_j");
@@ -642,18 +697,21 @@ int es_reset_survivors(es_ctx* c) {
 
 int es_reset_counts(es_ctx* c) {
     if (!c) return fail(ES_ERR_ARG, "null context");
-    ES_CUDA(cudaMemsetAsync(c->d_counts, 0, 8ull * std::max<uint32_t>(c->h_inst.n_filters, 1),
+    ES_CUDA(cudaMemsetAsync(c->d_counts, 0, 8ull * std::max<uint32_t>(c->geo.n_filters, 1),
                             c->stream), "memset");
     return ES_OK;
 }
 
 static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_list) {
-    const EsInst& I = c->h_inst;
     const es_tune& tn = c->tune;
+    const bool prod = is_production(tn);
+    const uint32_t PF = prod_tables(tn);
+    const TableSet& T = prod ? c->prod[PF].t : c->caller;
+    const EsInst& I = T.h;
     EsLaunch L;
     memset(&L, 0, sizeof(L));
     EsItem& it = L.item0;
-    it.inst = c->d_inst;
+    it.inst = T.d;
     it.tconst = nullptr;
     it.list = d_list;
     it.counts = tn.count_stages ? c->d_counts : nullptr;
@@ -673,9 +731,11 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
     it.n_units = d_list ? (n_work + per_unit - 1) / per_unit : units_of(I, it.c_begin, it.c_end, tn.strip);
     it.group = 0;
     it.inst_id = 0;
-    const uint32_t F = stage_filters(tn.layout, tn.mask_filters, I.n_filters, I.F_built);
-    const uint32_t layout = launch_layout(tn.layout, I.W, I.small_bytes, I.n_filters, tn, I.mask_off[F]);
-    const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, I.n_filters, tn, staged_words(layout, I.mask_off[F]));
+    const uint32_t F = prod ? PF : stage_filters(tn.layout, tn.mask_filters, I.n_filters, I.F_built);
+    const uint32_t layout = prod ? ES_LAYOUT_PROD
+                                 : launch_layout(tn.layout, I.W, I.small_bytes, I.n_filters, tn, I.mask_off[F]);
+    const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, I.n_filters, tn,
+                                  prod ? I.tab_words : staged_words(layout, I.mask_off[F]));
     it.caller = 0;
     L.items = nullptr;
     L.n_items = 1;
@@ -694,7 +754,10 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
     L.cnt_off = sp.cnt_off;
     L.queue_off = sp.queue_off;
     L.stage_off = sp.stage_off;
-    memcpy(L.tconst0, c->tconst, 4ull * I.n_filters);
+    if (prod)
+        prod_tconst(c->prod[PF], c->tconst, L.tconst0);
+    else
+        memcpy(L.tconst0, c->tconst, 4ull * I.n_filters);
     if (it.n_units == 0) return ES_OK;
     int grid = 0;
     if (int e = grid_for(layout, tn.count_stages, I.W, F, tn, sp.bytes, it.n_units, &grid)) return e;
@@ -707,7 +770,7 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
 
 int es_launch(es_ctx* c, uint64_t ostart, uint64_t ocount) {
     if (!c) return fail(ES_ERR_ARG, "null context");
-    if (ostart > c->h_inst.n_outer || ocount > c->h_inst.n_outer - ostart)
+    if (ostart > c->geo.n_outer || ocount > c->geo.n_outer - ostart)
         return fail(ES_ERR_RANGE, "outer range outside [0, R/r0)");
     return ctx_launch(c, ostart, ostart + ocount, nullptr);
 }
@@ -715,7 +778,7 @@ int es_launch(es_ctx* c, uint64_t ostart, uint64_t ocount) {
 int es_launch_list(es_ctx* c, const uint64_t* outer, uint64_t n) {
     if (!c || (n && !outer)) return fail(ES_ERR_ARG, "null argument");
     for (uint64_t i = 0; i < n; ++i)
-        if (outer[i] >= c->h_inst.n_outer) return fail(ES_ERR_RANGE, "outer index outside [0, R/r0)");
+        if (outer[i] >= c->geo.n_outer) return fail(ES_ERR_RANGE, "outer index outside [0, R/r0)");
     if (n == 0) return ES_OK;
     ES_CUDA(cudaStreamSynchronize(c->stream), "sync");
     if (n > c->list_cap) {
@@ -773,7 +836,7 @@ int es_read_survivors(es_ctx* c, uint64_t* idx_out, uint64_t cap, uint64_t* n) {
 
 int es_stage_counts(es_ctx* c, uint64_t* counts, uint32_t n) {
     if (!c || (n && !counts)) return fail(ES_ERR_ARG, "null argument");
-    if (n != c->h_inst.n_filters) return fail(ES_ERR_ARG, "counts length must equal the filter count");
+    if (n != c->geo.n_filters) return fail(ES_ERR_ARG, "counts length must equal the filter count");
     ES_CUDA(cudaStreamSynchronize(c->stream), "kernel execution");
     if (n) ES_CUDA(cudaMemcpy(counts, c->d_counts, 8ull * n, cudaMemcpyDeviceToHost), "copy");
     return ES_OK;
@@ -838,8 +901,14 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     if (!b) return fail(ES_ERR_NOMEM, "host allocation");
     b->tune = tune;
     b->ctxs.assign(ctxs, ctxs + n_ctx);
-    for (uint32_t i = 0; i < n_ctx; ++i)
+    const bool prod = is_production(tune);
+    const uint32_t PF = prod_tables(tune);
+    for (uint32_t i = 0; i < n_ctx; ++i) {
         if (!ctxs[i]) { es_batch_destroy(b); return fail(ES_ERR_ARG, "null context in batch"); }
+        if (int e = ensure_tables(ctxs[i], tune)) { es_batch_destroy(b); return e; }
+    }
+    // the table set a plan's items run on
+    auto tables = [&](const es_ctx* c) -> const TableSet& { return prod ? c->prod[PF].t : c->caller; };
     // width class of a plan: the kernel instance its inner ring uses
     auto width_class = [](uint32_t W) -> uint32_t { return W <= 2 ? W : (W <= 4 ? 4u : 0u); };
     std::vector<uint32_t> h_tc;
@@ -852,14 +921,14 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         if (s.ctx_index >= n_ctx) { es_batch_destroy(b); return fail(ES_ERR_ARG, "item ctx_index out of range"); }
         if (s.group >= n_items) { es_batch_destroy(b); return fail(ES_ERR_ARG, "item group must be < n_items"); }
         const es_ctx* c = ctxs[s.ctx_index];
-        const EsInst& I = c->h_inst;
+        const EsInst& I = c->geo;
         if (s.o_begin > s.o_end || s.o_end > I.n_outer) {
             es_batch_destroy(b);
             return fail(ES_ERR_RANGE, "item outer range outside [0, R/r0)");
         }
         EsItem& it = b->h_items[i];
         memset(&it, 0, sizeof(it));
-        it.inst = c->d_inst;
+        it.inst = tables(c).d;
         it.list = nullptr;
         it.t = s.t;
         it.o_begin = s.o_begin;
@@ -870,13 +939,13 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         it.group = s.group;
         it.inst_id = s.ctx_index;
         it.caller = i;
-        // per-block constants tconst[j] = (t mod q)(M mod q) mod q
+        // per-block constants, in the order of the table set's entries
         it.tconst = reinterpret_cast<const uint32_t*>((uintptr_t)h_tc.size());  // patched below
-        for (uint32_t f = 0; f < I.n_filters; ++f) {
-            const uint64_t q = c->q[f];
-            const uint64_t mq = (uint64_t)(c->M % q);
-            h_tc.push_back((uint32_t)((s.t % q) * mq % q));
-        }
+        uint32_t caller_tc[ES_MAX_FILTERS], entry_tc[ES_MAX_ENTRIES];
+        block_tconst(c, s.t, caller_tc);
+        if (prod) prod_tconst(c->prod[PF], caller_tc, entry_tc);
+        h_tc.insert(h_tc.end(), prod ? entry_tc : caller_tc,
+                    prod ? entry_tc + c->prod[PF].entries.size() : caller_tc + I.n_filters);
         while (h_tc.size() % 4) h_tc.push_back(0);
         b->count_off[i] = cwords;
         cwords += std::max<uint32_t>(I.n_filters, 1);
@@ -884,13 +953,13 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     }
     b->n_groups = max_group + 1;
     b->counts_words = cwords;
-    // launch order: items grouped by width class (stable), one launch per class; with
-    // ES_LAYOUT_AUTO a one- or two-word class splits further into the plans whose inner-stage
+    // launch order: items grouped by width class (stable), one launch per class; counting launches
+    // with ES_LAYOUT_AUTO split a one- or two-word class further into the plans whose inner-stage
     // tables fit shared memory (staged) and the rest
     auto class_key = [&](uint32_t item) -> uint32_t {
-        const EsInst& I = ctxs[items[item].ctx_index]->h_inst;
+        const EsInst& I = tables(ctxs[items[item].ctx_index]).h;
         uint32_t key = 2u * width_class(I.W);
-        if (tune.layout == ES_LAYOUT_AUTO && (I.W == 1 || I.W == 2)) {
+        if (!prod && tune.layout == ES_LAYOUT_AUTO && (I.W == 1 || I.W == 2)) {
             const uint32_t Fi = stage_filters(tune.layout, tune.mask_filters, I.n_filters, I.F_built);
             if (launch_layout(ES_LAYOUT_AUTO, I.W, (uint32_t)I.small_bytes, I.n_filters, tune, I.mask_off[Fi]) ==
                 ES_LAYOUT_SMEM)
@@ -910,14 +979,14 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     if (ce == cudaSuccess) ce = cudaMalloc(&b->d_items_launch, sizeof(EsItem) * n_items);
     if (ce == cudaSuccess) ce = cudaMalloc(&b->d_tconst, 4ull * std::max<size_t>(h_tc.size(), 4));
     if (ce == cudaSuccess) ce = cudaMalloc(&b->d_counts, 8ull * cwords);
-    // scalars: [0] survivor count, [1..4] unit counters of the launches, then group_found[G],
+    // scalars: [0] survivor count, [1..n_items] unit counters of the launches, then group_found[G],
     // group_min[4G], item_next[n_items]
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_surv_n, 8ull * (1 + kMaxSubs + 5ull * b->n_groups + n_items));
+    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_surv_n, 8ull * (1 + 5ull * b->n_groups + 2ull * n_items));
     b->surv_cap = ctxs[0]->surv_cap;
     if (ce == cudaSuccess) ce = cudaMalloc(&b->d_surv, sizeof(es_survivor) * b->surv_cap);
     if (ce != cudaSuccess) { es_batch_destroy(b); return cuda_fail(ce, "batch setup"); }
     b->d_unit = b->d_surv_n + 1;
-    b->d_found = b->d_surv_n + 1 + kMaxSubs;
+    b->d_found = b->d_surv_n + 1 + n_items;
     b->d_min = b->d_found + b->n_groups;
     b->d_item_next = b->d_min + 4ull * b->n_groups;
     b->n_items = n_items;
@@ -930,20 +999,29 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     std::vector<EsItem> launch_items(n_items);
     uint32_t pos = 0;
     while (pos < n_items) {
-        const uint32_t cls = width_class(ctxs[items[order[pos]].ctx_index]->h_inst.W);
-        uint32_t end = pos;
-        uint32_t small_max = 0, nf_max = 1, F = tune.mask_filters, first_ctx = items[order[pos]].ctx_index;
+        const uint32_t first_ctx = items[order[pos]].ctx_index;
+        const uint32_t cls = width_class(ctxs[first_ctx]->geo.W);
+        uint32_t end = pos, small_max = 0, nf_max = 1, stage_max = 0;
+        uint32_t F = prod ? PF : tune.mask_filters;
         bool one_ctx = true;
-        uint32_t words = ctxs[first_ctx]->h_inst.W;
+        uint32_t words = ctxs[first_ctx]->geo.W;
         uint64_t units = 0;
         while (end < n_items && keys[order[end]] == keys[order[pos]]) {
             const uint32_t ci = items[order[end]].ctx_index;
-            const es_ctx* c = ctxs[ci];
-            small_max = std::max<uint32_t>(small_max, c->h_inst.small_bytes);
-            nf_max = std::max<uint32_t>(nf_max, c->h_inst.n_filters);
-            F = std::min(F, stage_filters(tune.layout, tune.mask_filters, c->h_inst.n_filters, c->h_inst.F_built));
+            const EsInst& I = tables(ctxs[ci]).h;
+            const uint32_t small = std::max<uint32_t>(small_max, I.small_bytes);
+            if (prod) {
+                // plans that fit a CTA's shared memory one by one may not fit it together
+                const uint32_t stage = std::max(stage_max, I.tab_words);
+                if (end > pos && plan_smem(small, 1, tune, stage).bytes > (uint32_t)g_dev.smem_optin - 1024u) break;
+                stage_max = stage;
+            } else {
+                F = std::min(F, stage_filters(tune.layout, tune.mask_filters, I.n_filters, I.F_built));
+            }
+            small_max = small;
+            nf_max = std::max<uint32_t>(nf_max, I.n_filters);
             if (ci != first_ctx) one_ctx = false;
-            if (c->h_inst.W != words) words = 0;   // the generic instance reads each plan's width
+            if (I.W != words) words = 0;   // the generic instance reads each plan's width
             EsItem it = b->h_items[order[end]];
             it.unit_begin = units;
             units += it.n_units;
@@ -952,11 +1030,16 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         }
         es_batch::Sub sub;
         sub.words = cls == 0 ? 0u : (cls == 4 && words == 0 ? 4u : (words ? words : cls));
-        uint32_t mask_words = 0;   // the largest inner-stage word-mask tables among the class's plans
-        for (uint32_t j = pos; j < end; ++j)
-            mask_words = std::max<uint32_t>(mask_words, ctxs[items[order[j]].ctx_index]->h_inst.mask_off[F]);
-        sub.layout = launch_layout(tune.layout, sub.words, small_max, nf_max, tune, mask_words);
-        const SmemPlan sp = plan_smem(small_max, nf_max, tune, staged_words(sub.layout, mask_words));
+        if (prod) {
+            sub.layout = ES_LAYOUT_PROD;
+        } else {
+            uint32_t mask_words = 0;   // the largest inner-stage word-mask tables among the class's plans
+            for (uint32_t j = pos; j < end; ++j)
+                mask_words = std::max<uint32_t>(mask_words, tables(ctxs[items[order[j]].ctx_index]).h.mask_off[F]);
+            sub.layout = launch_layout(tune.layout, sub.words, small_max, nf_max, tune, mask_words);
+            stage_max = staged_words(sub.layout, mask_words);
+        }
+        const SmemPlan sp = plan_smem(small_max, nf_max, tune, stage_max);
         EsLaunch& L = sub.L;
         memset(&L, 0, sizeof(L));
         L.items = b->d_items_launch + pos;
@@ -996,7 +1079,7 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
 }
 
 static int batch_enqueue(es_batch* b) {
-    ES_CUDA(cudaMemsetAsync(b->d_surv_n, 0, 8ull * (1 + kMaxSubs), b->stream), "memset");   // count + unit counters
+    ES_CUDA(cudaMemsetAsync(b->d_surv_n, 0, 8ull * (1 + b->n_items), b->stream), "memset");   // count + unit counters
     ES_CUDA(cudaMemsetAsync(b->d_found, 0xff, 8ull * b->n_groups, b->stream), "memset");
     ES_CUDA(cudaMemsetAsync(b->d_item_next, 0, 8ull * b->n_items, b->stream), "memset");
     if (b->counts_words)
@@ -1070,7 +1153,7 @@ int es_batch_group_min(es_batch* b, uint32_t group, int* found, uint64_t* t, uin
 int es_batch_item_counts(es_batch* b, uint32_t item, uint64_t* counts, uint32_t n) {
     if (!b || (n && !counts)) return fail(ES_ERR_ARG, "null argument");
     if (item >= b->h_items.size()) return fail(ES_ERR_ARG, "item out of range");
-    const uint32_t nf = b->ctxs[b->h_items[item].inst_id]->h_inst.n_filters;
+    const uint32_t nf = b->ctxs[b->h_items[item].inst_id]->geo.n_filters;
     if (n != nf) return fail(ES_ERR_ARG, "counts length must equal the item's filter count");
     if (!b->ran) return fail(ES_ERR_STATE, "batch has not run");
     ES_CUDA(cudaStreamSynchronize(b->stream), "kernel execution");
@@ -1141,13 +1224,13 @@ int es_int_peak_mixed(double* ops_per_s, double* ms_out) { return int_peak_probe
 // caller passes the inputs (the context's plan tables, built earlier) and the outputs (a
 // survivor buffer, its count and the 4-word minimum).  The launch's scratch -- work counter,
 // search flag, per-block item descriptors and block constants -- lives in the file-scope
-// array below, of fixed size ES_STATIC_MAX_BLOCKS blocks x ES_MAX_FILTERS filters (about
-// 57 KB); every GPU that loads this library keeps it until the process exits.
+// array below, of fixed size ES_STATIC_MAX_BLOCKS blocks x ES_MAX_ENTRIES entries (about
+// 60 KB); every GPU that loads this library keeps it until the process exits.
 namespace {
 
 constexpr size_t kStaticItemsOff = 256;
 constexpr size_t kStaticTconstOff = kStaticItemsOff + sizeof(EsItem) * ES_STATIC_MAX_BLOCKS;
-constexpr size_t kStaticBytes = kStaticTconstOff + 4ull * ES_STATIC_MAX_BLOCKS * ES_MAX_FILTERS;
+constexpr size_t kStaticBytes = kStaticTconstOff + 4ull * ES_STATIC_MAX_BLOCKS * ES_MAX_ENTRIES;
 
 // [0,8) work counter, [8,16) least block with a good survivor, items, per-block constants
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
@@ -1158,7 +1241,7 @@ static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
 constexpr int kMaxDevices = 64;
 unsigned char* g_static_ptr[kMaxDevices] = {nullptr};
 EsItem g_static_items[ES_STATIC_MAX_BLOCKS];
-uint32_t g_static_tconst[ES_STATIC_MAX_BLOCKS * ES_MAX_FILTERS];
+uint32_t g_static_tconst[ES_STATIC_MAX_BLOCKS * ES_MAX_ENTRIES];
 std::mutex g_static_mu;
 
 }  // namespace
@@ -1173,8 +1256,13 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
         return fail(ES_ERR_RANGE, "n_blocks must be in [1, " + std::to_string(ES_STATIC_MAX_BLOCKS) +
                                       "] for the static-scratch search");
     if (t0 > UINT64_MAX - n_blocks) return fail(ES_ERR_RANGE, "block range overflows");
-    const EsInst& I = c->h_inst;
-    if (I.n_filters > ES_MAX_FILTERS) return fail(ES_ERR_RANGE, "too many filters");
+    // the search never counts: the production cascade, or the scalar layout on request
+    es_tune tn = c->tune;
+    tn.count_stages = 0;
+    const bool prod = is_production(tn);
+    const uint32_t PF = prod_tables(tn);
+    const TableSet& T = prod ? c->prod[PF].t : c->caller;
+    const EsInst& I = T.h;
     cudaStream_t st = (cudaStream_t)stream;
     // The descriptors below are copied from host staging arrays that the next call overwrites; a
     // captured copy would read them only when the graph runs, so capture is refused.
@@ -1199,13 +1287,10 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
     EsItem* d_items = reinterpret_cast<EsItem*>(base + kStaticItemsOff);
     uint32_t* d_tc = reinterpret_cast<uint32_t*>(base + kStaticTconstOff);
 
-    const es_tune& tn = c->tune;
     const uint32_t nf = I.n_filters;
-    const uint32_t F = stage_filters(tn.layout, tn.mask_filters, nf, I.F_built);
-    es_tune tn0 = tn;
-    tn0.count_stages = 0;   // the static search never counts
-    const uint32_t layout = launch_layout(tn.layout, I.W, I.small_bytes, nf, tn0, I.mask_off[F]);
-    const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, nf, tn0, staged_words(layout, I.mask_off[F]));
+    const uint32_t F = prod ? PF : stage_filters(tn.layout, tn.mask_filters, nf, I.F_built);
+    const uint32_t layout = prod ? ES_LAYOUT_PROD : (uint32_t)ES_LAYOUT_SCALAR;
+    const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, nf, tn, prod ? I.tab_words : 0u);
     uint64_t cbeg = 0;
     const uint64_t ncyc = cycles_of(I, 0, I.n_outer, &cbeg);
     const uint64_t nu = units_of(I, cbeg, cbeg + ncyc, tn.strip);
@@ -1213,8 +1298,8 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
         const uint64_t t = t0 + i;
         EsItem& it = g_static_items[i];
         memset(&it, 0, sizeof(it));
-        it.inst = c->d_inst;
-        it.tconst = d_tc + (size_t)i * ES_MAX_FILTERS;
+        it.inst = T.d;
+        it.tconst = d_tc + (size_t)i * ES_MAX_ENTRIES;
         it.t = t;
         it.o_begin = 0;
         it.o_end = I.n_outer;
@@ -1223,14 +1308,18 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
         it.unit_begin = nu * i;
         it.n_units = nu;
         it.caller = i;
-        for (uint32_t f = 0; f < nf; ++f) {
-            const uint64_t q = c->q[f];
-            g_static_tconst[(size_t)i * ES_MAX_FILTERS + f] = (uint32_t)((t % q) * (uint64_t)(c->M % q) % q);
+        uint32_t* tc = g_static_tconst + (size_t)i * ES_MAX_ENTRIES;
+        if (prod) {
+            uint32_t caller_tc[ES_MAX_FILTERS];
+            block_tconst(c, t, caller_tc);
+            prod_tconst(c->prod[PF], caller_tc, tc);
+        } else {
+            block_tconst(c, t, tc);
         }
     }
     ES_CUDA(cudaMemcpyAsync(d_items, g_static_items, sizeof(EsItem) * n_blocks, cudaMemcpyHostToDevice, st),
             "copy items");
-    ES_CUDA(cudaMemcpyAsync(d_tc, g_static_tconst, 4ull * ES_MAX_FILTERS * n_blocks, cudaMemcpyHostToDevice, st),
+    ES_CUDA(cudaMemcpyAsync(d_tc, g_static_tconst, 4ull * ES_MAX_ENTRIES * n_blocks, cudaMemcpyHostToDevice, st),
             "copy block constants");
     ES_CUDA(cudaMemsetAsync(d_unit, 0, 8, st), "memset");
     ES_CUDA(cudaMemsetAsync(d_found, 0xff, 8, st), "memset");

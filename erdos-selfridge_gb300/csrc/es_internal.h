@@ -29,6 +29,10 @@
 #define ES_QUEUE_BYTES 2304   // per-warp shared slot: entry queue, lane records, tail context
 #define ES_MAX_RINGS 64
 #define ES_MAX_FILTERS 192   // pi(1024) = 172 residual primes at most
+#define ES_PMAX 6            // inner tables of the production cascade, at most
+#define ES_PRES 4            // residue-stage filters of the production cascade
+#define ES_MAX_ENTRIES (ES_MAX_FILTERS + ES_PMAX + ES_PRES)   // entries of a cascade, with fill-ins
+#define ES_PBUCKET_LOG2 11   // carry-split buckets of the production cascade
 
 struct EsFilterC {
     uint32_t q;      // modulus p^t_p (< 2^20)
@@ -56,6 +60,18 @@ struct EsInst {
     uint32_t km;          // M >> sh (32-bit key of M)
     // byte offsets inside the small block
     uint32_t o_T1, o_TQ1, o_D2, o_DQ2, o_S0, o_K0, o_I0, o_Q0, o_BK, o_FC, o_K1;
+    // production cascade (es_prod_kernel.cuh): F inner tables, ES_PRES residue filters, the tail
+    uint32_t F;           // inner tables (0 in a caller-order table set)
+    uint32_t o_R1;        // [r1 + 1] ring-1 rows: key, then the inner tables' scaled term residues
+    uint32_t o_TQr;       // [r1] term residues of the residue-stage filters
+    uint32_t o_DQr;       // [r2] step residues of the residue-stage filters
+    uint32_t o_Qr;        // [r0] inner-ring residues of the residue-stage filters
+    uint32_t ssh;         // 32 - bsh: bucket entries hold the key's low bits above the slot
+    uint32_t band;        // key distance below which the split is found exactly, << ssh
+    uint32_t row_bytes;   // bytes of a table row
+    uint32_t tab_base[ES_PMAX];   // byte offset of each table's phase-0 row in the staged block
+    int32_t tab_wrap[ES_PMAX];    // byte distance from a row to the row a wrap past M selects
+    uint32_t tab_words;   // words of all inner tables
     // word offsets of the fast (word-mask) tables, F_built + 1 entries (prefix sums)
     uint32_t mask_off[ES_FMAX + 1];
     uint32_t mask_stride;            // words per phase row of P_f: W, or 4 for W = 3 (16-byte rows)
@@ -106,18 +122,26 @@ struct EsLaunch {
     uint32_t stage_off;               // byte offset of the staged tables (ES_LAYOUT_SMEM, _SMEM_PAIR)
     // single-plan launches carry their one item and block constants by value
     EsItem item0;
-    uint32_t tconst0[ES_MAX_FILTERS];
+    uint32_t tconst0[ES_MAX_ENTRIES];
 };
 
-// Scan kernel instances by layout (es_scan_wm.cu / es_scan_wmc.cu, es_scan_pair.cu, es_scan_sc.cu,
-// es_scan_sm.cu, es_scan_sp.cu).
+// Internal layout code of the production cascade: launches that do not count stages, in every
+// layout but the scalar one.
+#define ES_LAYOUT_PROD 16
+
+// Scan kernel instances: the production cascade by inner-ring words (es_prod1.cu, es_prod2.cu,
+// es_prod4.cu, es_prod0.cu), and the caller's cascade order by layout (counting launches:
+// es_scan_wmc.cu, es_scan_pair.cu, es_scan_sm.cu, es_scan_sp.cu; es_scan_sc.cu both).
 typedef void (*ScanFn)(const EsLaunch);
-ScanFn es_pick_wordmask_fast(uint32_t words, uint32_t mask_filters);
-ScanFn es_pick_wordmask_count(uint32_t words, uint32_t mask_filters);
-ScanFn es_pick_pair(int count, uint32_t words, uint32_t mask_filters);
+ScanFn es_pick_prod1(uint32_t tables);
+ScanFn es_pick_prod2(uint32_t tables);
+ScanFn es_pick_prod4(uint32_t tables);
+ScanFn es_pick_prod0(uint32_t tables);
+ScanFn es_pick_wordmask(uint32_t words, uint32_t mask_filters);
+ScanFn es_pick_pair(uint32_t words, uint32_t mask_filters);
 ScanFn es_pick_scalar(int count, uint32_t mask_filters);
-ScanFn es_pick_smem(int count, uint32_t words, uint32_t mask_filters);
-ScanFn es_pick_smem_pair(int count, uint32_t words, uint32_t mask_filters);
+ScanFn es_pick_smem(uint32_t words, uint32_t mask_filters);
+ScanFn es_pick_smem_pair(uint32_t words, uint32_t mask_filters);
 
 // Host-side launchers implemented in es_scan.cu (return a cudaError_t value).
 int es_scan_prepare(int smem_optin_bytes);

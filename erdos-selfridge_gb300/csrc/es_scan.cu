@@ -1,14 +1,17 @@
 // Dispatch of the scan kernel instances, the block-ordered min-reduction and the integer-pipe
-// peak probe of the GB300 Erdős–Selfridge CRT-wheel sieve (sm_103a).  The scan kernel itself is
-// es_scan_kernel.cuh, instantiated per layout in es_scan_wm.cu / es_scan_wmc.cu (word masks,
-// production and counting launches), es_scan_pair.cu, es_scan_sc.cu, es_scan_sm.cu (word masks
-// staged in shared memory) and es_scan_sp.cu (pair tables staged in shared memory).
+// peak probe of the GB300 Erdős–Selfridge CRT-wheel sieve (sm_103a).  The production scan kernel is
+// es_prod_kernel.cuh (es_prod1.cu, es_prod2.cu, es_prod4.cu, es_prod0.cu); es_scan_kernel.cuh runs
+// the caller's cascade for counting launches, instantiated per layout in es_scan_wmc.cu (word
+// masks), es_scan_pair.cu, es_scan_sm.cu (word masks staged in shared memory) and es_scan_sp.cu
+// (pair tables staged in shared memory), and the scalar layout in es_scan_sc.cu.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "../../include/es_gb300.h"
 #include "es_internal.h"
@@ -128,16 +131,24 @@ __global__ void __launch_bounds__(256) es_int_peak_kernel(unsigned long long* si
 }
 
 ScanFn pick(int layout, int count, uint32_t words, uint32_t f) {
+    if (layout == ES_LAYOUT_PROD) {
+        // words == 0 (a batch whose plans differ in width) takes the instance for any width
+        if (words == 1) return es_pick_prod1(f);
+        if (words == 2) return es_pick_prod2(f);
+        if (words == 3 || words == 4) return es_pick_prod4(f);
+        return es_pick_prod0(f);
+    }
     if (layout == ES_LAYOUT_SCALAR) return es_pick_scalar(count, f);
+    if (!count) return nullptr;   // the caller's cascade by tables serves counting launches only
     // staged tables exist for inner rings of one or two words (the host resolves any other
     // ring to the word-mask layout before it asks)
-    if (layout == ES_LAYOUT_SMEM) return (words == 1 || words == 2) ? es_pick_smem(count, words, f) : nullptr;
-    if (layout == ES_LAYOUT_SMEM_PAIR) return (words == 1 || words == 2) ? es_pick_smem_pair(count, words, f) : nullptr;
+    if (layout == ES_LAYOUT_SMEM) return (words == 1 || words == 2) ? es_pick_smem(words, f) : nullptr;
+    if (layout == ES_LAYOUT_SMEM_PAIR) return (words == 1 || words == 2) ? es_pick_smem_pair(words, f) : nullptr;
     // pair tables exist for inner rings of one or two words.  words == 0 (a batch whose plans
     // differ in width) and wider rings take the generic word-mask instance, which reads each
     // plan's own width: a fixed-width instance would index past a narrower plan's tables.
-    if (layout == ES_LAYOUT_PAIR && (words == 1 || words == 2)) return es_pick_pair(count, words, f);
-    return count ? es_pick_wordmask_count(words, f) : es_pick_wordmask_fast(words, f);
+    if (layout == ES_LAYOUT_PAIR && (words == 1 || words == 2)) return es_pick_pair(words, f);
+    return es_pick_wordmask(words, f);
 }
 
 }  // namespace
@@ -146,18 +157,25 @@ ScanFn pick(int layout, int count, uint32_t words, uint32_t f) {
 int es_scan_prepare(int smem_optin_bytes) {
     const uint32_t fs[8] = {0, 1, 2, 3, 4, 5, 6, 8};
     const uint32_t ws[4] = {1, 2, 3, 5};   // every word-count instance: 1, 2, 3-4, generic
-    for (int layout = 0; layout < 5; ++layout)
-        for (int count = 0; count < 2; ++count)
-            for (uint32_t w : ws)
-                for (uint32_t f : fs) {
-                    if ((layout == ES_LAYOUT_SMEM || layout == ES_LAYOUT_SMEM_PAIR) && w > 2) continue;
-                    const ScanFn fn = pick(layout, count, w, f);
-                    if (!fn) return (int)cudaErrorInvalidDeviceFunction;
-                    cudaError_t e = cudaFuncSetAttribute(fn,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         smem_optin_bytes);
-                    if (e != cudaSuccess) return (int)e;
-                }
+    std::vector<ScanFn> all;
+    for (uint32_t w : ws) {
+        for (uint32_t f = 1; f <= ES_PMAX; ++f) all.push_back(pick(ES_LAYOUT_PROD, 0, w, f));
+        for (uint32_t f : fs) {
+            for (int count = 0; count < 2; ++count) all.push_back(pick(ES_LAYOUT_SCALAR, count, w, f));
+            all.push_back(pick(ES_LAYOUT_WORDMASK, 1, w, f));
+            all.push_back(pick(ES_LAYOUT_PAIR, 1, w, f));
+            if (w > 2) continue;
+            all.push_back(pick(ES_LAYOUT_SMEM, 1, w, f));
+            all.push_back(pick(ES_LAYOUT_SMEM_PAIR, 1, w, f));
+        }
+    }
+    std::sort(all.begin(), all.end());
+    all.erase(std::unique(all.begin(), all.end()), all.end());
+    for (const ScanFn fn : all) {
+        if (!fn) return (int)cudaErrorInvalidDeviceFunction;
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_bytes);
+        if (e != cudaSuccess) return (int)e;
+    }
     return 0;
 }
 

@@ -192,6 +192,12 @@ __device__ __forceinline__ void copy_words(uint32_t* dst, const uint32_t* __rest
     for (uint32_t i = (n4 << 2) + threadIdx.x; i < nwords; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
+// The plan's header into shared memory, a word per thread.
+__device__ __forceinline__ void load_inst(EsInst& si, const EsInst* inst) {
+    for (uint32_t i = threadIdx.x; i < sizeof(EsInst) / 4u; i += blockDim.x)
+        reinterpret_cast<uint32_t*>(&si)[i] = __ldg(reinterpret_cast<const uint32_t*>(inst) + i);
+}
+
 // Everything the flush, the cascade tail and the emit need for one warp-unit.  It lives in the
 // warp's slot in shared memory, written once per warp-unit and read only on the flush path, so
 // none of it occupies registers across the ring-1 sweep.
@@ -830,7 +836,7 @@ __global__ void __launch_bounds__(ES_LB_THREADS, ES_LB_MINB) es_scan_kernel(cons
 
     if (L.direct) {
         // ---- stage the one plan, then warps claim warp-units on their own ---------------
-        if (tid == 0) si = *items[0].inst;
+        load_inst(si, items[0].inst);
         __syncthreads();
         copy_words(reinterpret_cast<uint32_t*>(smem), reinterpret_cast<const uint32_t*>(si.small), si.small_bytes >> 2);
         if (LAYOUT == ES_LAYOUT_SMEM)   // the inner-stage filters' phase tables (16-byte aligned)
@@ -889,7 +895,7 @@ __global__ void __launch_bounds__(ES_LB_THREADS, ES_LB_MINB) es_scan_kernel(cons
         const EsItem& item = items[item_id];
         if (item.inst_id != cur_inst) {
             // restage: the header and the small tables of this item's plan
-            if (tid == 0) si = *item.inst;
+            load_inst(si, item.inst);
             __syncthreads();
             copy_words(reinterpret_cast<uint32_t*>(smem), reinterpret_cast<const uint32_t*>(si.small),
                        si.small_bytes >> 2);

@@ -56,6 +56,15 @@ class BatchItem(C.Structure):
                 ("o_begin", C.c_uint64), ("o_end", C.c_uint64)]
 
 
+class CascadeInfo(C.Structure):
+    _fields_ = [("small_bytes", C.c_uint64), ("tab_words", C.c_uint64), ("n_parts", C.c_uint64),
+                ("n_entries", C.c_uint32), ("row_bytes", C.c_uint32), ("key_shift", C.c_uint32),
+                ("bucket_shift", C.c_uint32), ("band", C.c_uint32), ("o_row1", C.c_uint32),
+                ("row1_bytes", C.c_uint32), ("o_terms1", C.c_uint32), ("o_sorted", C.c_uint32),
+                ("o_digits", C.c_uint32), ("o_buckets", C.c_uint32), ("reserved", C.c_uint32),
+                ("tab_base", C.c_uint32 * 6), ("tab_wrap", C.c_int32 * 6)]
+
+
 SURVIVOR_DTYPE = np.dtype([("idx", "<u8"), ("s_lo", "<u8"), ("s_hi", "<u8"), ("t", "<u8"),
                            ("item", "<u4"), ("good", "<u4")])
 assert SURVIVOR_DTYPE.itemsize == C.sizeof(Survivor)
@@ -79,6 +88,7 @@ def lib() -> C.CDLL:
         "es_abi_version": ([], i32),
         "es_device_info": ([C.POINTER(i32), C.POINTER(i32), C.POINTER(i32), pu64], i32),
         "es_device_name": ([C.c_char_p, u32], i32),
+        "es_cascade_image": ([C.POINTER(PlanDesc), u32, u32, C.POINTER(CascadeInfo), P, u64, P, u64, P, u64], i32),
         "es_ctx_create": ([C.POINTER(PlanDesc), C.POINTER(Tune), C.POINTER(P)], i32),
         "es_ctx_destroy": ([P], i32),
         "es_ctx_set_tune": ([P, C.POINTER(Tune)], i32),

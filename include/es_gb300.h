@@ -127,6 +127,22 @@ int es_device_info(int* sm_count, int* cc_major, int* cc_minor, uint64_t* smem_o
 /* The current device's name (NUL-terminated, truncated to cap bytes): part of the tuner's cache key. */
 int es_device_name(char* out, uint32_t cap);
 
+/* Host only, no device needed: the tables of a plan's production cascade (the cascade of launches
+ * that count no stages) with 1..6 inner tables in smem_bytes of shared memory, for inspection and
+ * tests.  `small` and `tabs` are filled when they are large enough; parts gets triples (entry,
+ * filter, modulus): entry e tests n mod modulus against the filter's admissible set projected to
+ * it.  Entries 0..tables-1 are the inner tables, the next four the residue stage. */
+typedef struct es_cascade_info {
+    uint64_t small_bytes, tab_words, n_parts;
+    uint32_t n_entries, row_bytes, key_shift, bucket_shift, band;
+    uint32_t o_row1, row1_bytes, o_terms1, o_sorted, o_digits, o_buckets, reserved;
+    uint32_t tab_base[6];
+    int32_t tab_wrap[6];
+} es_cascade_info;
+int es_cascade_image(const es_plan_desc* desc, uint32_t tables, uint32_t smem_bytes, es_cascade_info* info,
+                     void* small, uint64_t small_cap, uint32_t* tabs, uint64_t tabs_cap, uint32_t* parts,
+                     uint64_t parts_cap);
+
 /* ---- context: one plan on the device ---------------------------------------------------- */
 /* Replaces GpuSieve.__init__ (sieve/gpu_sieve_v9.py:426-498): copies term tables, filter bit
  * tables, and builds every derived table (sorted inner ring, carry-split keys, ring-1/ring-2
