@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -122,6 +123,7 @@ struct es_ctx {
     EsInst geo{};                 // geometry only (rings, filter count, M)
     TableSet caller;              // caller's cascade order: counting and scalar launches
     ProdSet prod[ES_PMAX + 1];    // production cascade by inner tables
+    uint32_t own_tables[ES_PMAX + 1] = {0};   // by tables asked for: tables of this plan's own launches
     std::vector<uint32_t> q;
     u128 M = 1;
     uint32_t tconst[ES_MAX_FILTERS] = {0};
@@ -283,8 +285,43 @@ uint64_t units_of(const EsInst& I, uint64_t cb, uint64_t ce, uint32_t strip) {
 // (the layouts are forms of the caller's cascade; none changes which candidates pass).
 bool is_production(const es_tune& t) { return !t.count_stages && t.layout != ES_LAYOUT_SCALAR; }
 
+// The shape a production launch runs: the largest CTA that a caller can ask for stands for the
+// largest that the production kernel takes.
+es_tune prod_shape(es_tune t) {
+    if (t.threads == 512)
+        t.threads = ES_PROD_THREADS;
+    else if (t.threads > 512)
+        t.threads = 1024;   // no kernel takes it: the launch is refused
+    return t;
+}
+
+// Ring-1 cycles per lane and warp-unit of a production launch of `steps` warp-wide cycles, at most
+// the caller's.  A unit costs about half a cycle to set up, and the launch ends when its last unit
+// does: with W steps per resident warp, W (1 + 0.5 / s) + 0.6 s is least at s = sqrt(0.8 W).
+// Measured (k = 300): 2^30 positions 126 us at 8, 118 at 4; 2^34 positions 1485 at 8, 1563 at 4;
+// k = 384, 2^28 positions 189 us at 8, 74 at 2.
+uint32_t prod_strip(uint64_t steps, const es_tune& t) {
+    const double per_warp = (double)steps / ((double)g_dev.sms * (t.threads / 32u));
+    return std::min(t.strip, std::max(1u, (uint32_t)(std::sqrt(0.8 * per_warp) + 0.5)));
+}
+
+// Warp-wide ring-1 cycles of [cb, ce) (rows of 32 lanes x ring-2 digits).
+uint64_t steps_of(const EsInst& I, uint64_t cb, uint64_t ce) {
+    if (ce <= cb) return 0;
+    if (I.r2 <= 1) return (ce - cb + 31) / 32;
+    return ((ce + I.r2 - 1) / I.r2 - cb / I.r2 + 31) / 32 * I.r2;
+}
+
 // Inner tables of a production launch.
 uint32_t prod_tables(const es_tune& t) { return std::min<uint32_t>(std::max<uint32_t>(t.mask_filters, 1), ES_PMAX); }
+
+// Whether launches of this shape run the production cascade with PF tables: a plan whose rings are so
+// large that the cascade's tables do not fit one CTA runs the scalar layout instead.
+bool runs_production(const es_ctx* c, const es_tune& t, uint32_t PF) {
+    if (!is_production(t)) return false;
+    const EsInst& I = c->prod[PF].t.h;
+    return plan_smem(I.small_bytes, I.n_filters, prod_shape(t), I.tab_words).bytes <= (uint32_t)g_dev.smem_optin - 1024u;
+}
 
 // The production cascade's block constants from the caller's.
 void prod_tconst(const ProdSet& S, const uint32_t* tconst, uint32_t* out) {
@@ -363,7 +400,8 @@ int es_ctx_destroy(es_ctx* c) {
 // Uploads one table set: the header, the small block, the inner-stage tables and the bit tables
 // (ring terms too) in one arena.
 static int upload_set(es_ctx* c, TableSet& T, const std::vector<unsigned char>& small, const std::vector<uint32_t>& masks,
-                      const std::vector<uint32_t>& pairs, const std::vector<uint32_t>& bits) {
+                      const std::vector<uint32_t>& pairs, const std::vector<uint32_t>& bits,
+                      const std::vector<u128>& terms) {
     const EsHostPlan& P = c->plan;
     size_t aoff = 0;
     auto atake = [&](size_t bytes) { size_t o = aoff; aoff = es_align_up(aoff + bytes, 256); return o; };
@@ -372,7 +410,7 @@ static int upload_set(es_ctx* c, TableSet& T, const std::vector<unsigned char>& 
     const size_t a_masks = atake(4ull * std::max<size_t>(masks.size(), 4));
     const size_t a_pairs = atake(4ull * std::max<size_t>(pairs.size(), 4));
     const size_t a_bits = atake(4ull * std::max<size_t>(bits.size(), 4));
-    const size_t a_terms = atake(16ull * P.terms.size());
+    const size_t a_terms = atake(16ull * std::max<size_t>(terms.size(), 1));
     const size_t a_roff = atake(4ull * P.roff.size());
     const size_t a_radix = atake(4ull * P.radix.size());
     std::vector<unsigned char> img(aoff, 0);
@@ -380,8 +418,8 @@ static int upload_set(es_ctx* c, TableSet& T, const std::vector<unsigned char>& 
     if (!masks.empty()) memcpy(&img[a_masks], masks.data(), 4ull * masks.size());
     if (!pairs.empty()) memcpy(&img[a_pairs], pairs.data(), 4ull * pairs.size());
     if (!bits.empty()) memcpy(&img[a_bits], bits.data(), 4ull * bits.size());
-    for (size_t i = 0; i < P.terms.size(); ++i) {
-        uint64_t lo = (uint64_t)P.terms[i], hi = (uint64_t)(P.terms[i] >> 64);
+    for (size_t i = 0; i < terms.size(); ++i) {
+        uint64_t lo = (uint64_t)terms[i], hi = (uint64_t)(terms[i] >> 64);
         memcpy(&img[a_terms + 16 * i], &lo, 8);
         memcpy(&img[a_terms + 16 * i + 8], &hi, 8);
     }
@@ -511,31 +549,56 @@ static int build_caller(es_ctx* c) {
     I.small_bytes = (uint32_t)S.b.size();
     for (uint32_t f = 0; f <= ES_FMAX; ++f) I.mask_off[f] = mask_off[f];
     I.mask_stride = RS;
-    if (int e = upload_set(c, T, S.b, masks, pairs, P.allowed)) return e;
+    if (int e = upload_set(c, T, S.b, masks, pairs, P.allowed, P.terms)) return e;
     c->caller = T;
     return ES_OK;
 }
 
-// Tables of the production cascade with F inner tables.
-static int build_prod(es_ctx* c, uint32_t F) {
-    EsProdImage img;
+// The host image of the production cascade with F inner tables.
+static void prod_image(const es_ctx* c, uint32_t F, EsProdImage& img) {
     // beside the staged tables: the static shared memory, and the slots of the largest CTA's warps
-    es_prod_image(c->plan, c->geo, F, (uint32_t)g_dev.smem_optin - 2048u - 16u * ES_QUEUE_BYTES, img);
+    es_prod_image(c->plan, c->geo, F,
+                  (uint32_t)g_dev.smem_optin - 2048u - ES_PROD_THREADS / 32u * ES_QUEUE_BYTES, img);
+}
+
+static int upload_prod(es_ctx* c, uint32_t F, EsProdImage& img) {
     TableSet T;
     T.h = img.inst;
-    if (int e = upload_set(c, T, img.small, img.tabs, {}, img.bits)) return e;
+    if (int e = upload_set(c, T, img.small, img.tabs, {}, img.bits, img.sums)) return e;
     c->prod[F].t = T;
     c->prod[F].entries = std::move(img.entries);
     return ES_OK;
 }
 
-// Builds the table sets that launches of this shape read, unless they are there already.
-static int ensure_tables(es_ctx* c, const es_tune& t) {
+// Candidates per warp-wide ring-1 digit above which a plan's own launches take one more inner table
+// than asked for: the queue's passes then cost more than the table.  k = 260 (4.2 candidates with four
+// tables), 2^32 positions: 498 us, with five 447; k = 378 (5.2): 1439 and 1336; k = 379 (3.0): 1842 and
+// 1857; k = 390 (1.1): 1603 and 1653.
+constexpr double kMoreTables = 3.5;
+
+// Builds the table sets that launches of this shape read, unless they are there already: the
+// plan's own launches (own), or those of a batch of several plans, which share a table count.
+static int ensure_tables(es_ctx* c, const es_tune& t, bool own) {
     try {
-        const uint32_t F = prod_tables(t);
-        if (!c->prod[F].t.d)
-            if (int e = build_prod(c, F)) return e;   // es_search_blocks_static never counts
-        if (!is_production(t) && !c->caller.d)
+        uint32_t F = prod_tables(t);
+        if (own && !c->own_tables[F]) {
+            EsProdImage img;
+            prod_image(c, F, img);
+            uint32_t use = F;
+            if (F < ES_PMAX && 32.0 * c->geo.r0 * img.rate > kMoreTables) prod_image(c, use = F + 1, img);
+            if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)
+                if (int e = upload_prod(c, use, img)) return e;
+            c->own_tables[F] = use;
+        }
+        if (own) F = c->own_tables[F];
+        if (!c->prod[F].t.d) {
+            EsProdImage img;
+            prod_image(c, F, img);
+            if (int e = upload_prod(c, F, img)) return e;
+        }
+        es_tune s = t;
+        s.count_stages = 0;
+        if ((!is_production(t) || !runs_production(c, s, F)) && !c->caller.d)
             if (int e = build_caller(c)) return e;
     } catch (const std::bad_alloc&) {
         return fail(ES_ERR_NOMEM, "host allocation");
@@ -563,7 +626,7 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     c->tune = tune;
     c->M = c->plan.M;
     c->q = c->plan.q;
-    int e = ensure_tables(c, tune);
+    int e = ensure_tables(c, tune, true);
     if (e) {
         es_ctx_destroy(c);
         return e;
@@ -642,7 +705,7 @@ int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes
 int es_ctx_set_tune(es_ctx* c, const es_tune* t) {
     if (!c || !t) return fail(ES_ERR_ARG, "null argument");
     if (int e = check_tune(*t)) return e;
-    if (int e = ensure_tables(c, *t)) return e;
+    if (int e = ensure_tables(c, *t, true)) return e;
     c->tune = *t;
     return ES_OK;
 }
@@ -703,9 +766,11 @@ int es_reset_counts(es_ctx* c) {
 }
 
 static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_list) {
-    const es_tune& tn = c->tune;
-    const bool prod = is_production(tn);
-    const uint32_t PF = prod_tables(tn);
+    es_tune tn = c->tune;
+    const uint32_t PF = c->own_tables[prod_tables(tn)];
+    const bool prod = runs_production(c, tn, PF);
+    if (prod) tn = prod_shape(tn);
+    if (!prod && !tn.count_stages) tn.layout = ES_LAYOUT_SCALAR;
     const TableSet& T = prod ? c->prod[PF].t : c->caller;
     const EsInst& I = T.h;
     EsLaunch L;
@@ -726,6 +791,7 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
         n_work = cycles_of(I, ob, oe, &it.c_begin);
         it.c_end = it.c_begin + n_work;
     }
+    if (prod) tn.strip = prod_strip(d_list ? (n_work + 31) / 32 : steps_of(I, it.c_begin, it.c_end), tn);
     const uint64_t per_unit = 32ull * tn.strip;
     it.unit_begin = 0;
     it.n_units = d_list ? (n_work + per_unit - 1) / per_unit : units_of(I, it.c_begin, it.c_end, tn.strip);
@@ -901,14 +967,15 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     if (!b) return fail(ES_ERR_NOMEM, "host allocation");
     b->tune = tune;
     b->ctxs.assign(ctxs, ctxs + n_ctx);
-    const bool prod = is_production(tune);
-    const uint32_t PF = prod_tables(tune);
     for (uint32_t i = 0; i < n_ctx; ++i) {
         if (!ctxs[i]) { es_batch_destroy(b); return fail(ES_ERR_ARG, "null context in batch"); }
-        if (int e = ensure_tables(ctxs[i], tune)) { es_batch_destroy(b); return e; }
+        if (int e = ensure_tables(ctxs[i], tune, n_ctx == 1)) { es_batch_destroy(b); return e; }
     }
+    const uint32_t PF = n_ctx == 1 ? ctxs[0]->own_tables[prod_tables(tune)] : prod_tables(tune);
     // the table set a plan's items run on
-    auto tables = [&](const es_ctx* c) -> const TableSet& { return prod ? c->prod[PF].t : c->caller; };
+    auto tables = [&](const es_ctx* c) -> const TableSet& {
+        return runs_production(c, tune, PF) ? c->prod[PF].t : c->caller;
+    };
     // width class of a plan: the kernel instance its inner ring uses
     auto width_class = [](uint32_t W) -> uint32_t { return W <= 2 ? W : (W <= 4 ? 4u : 0u); };
     std::vector<uint32_t> h_tc;
@@ -935,7 +1002,6 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         it.o_end = s.o_end;
         const uint64_t ncyc = s.o_end > s.o_begin ? cycles_of(I, s.o_begin, s.o_end, &it.c_begin) : 0;
         it.c_end = it.c_begin + ncyc;
-        it.n_units = units_of(I, it.c_begin, it.c_end, tune.strip);
         it.group = s.group;
         it.inst_id = s.ctx_index;
         it.caller = i;
@@ -943,6 +1009,7 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         it.tconst = reinterpret_cast<const uint32_t*>((uintptr_t)h_tc.size());  // patched below
         uint32_t caller_tc[ES_MAX_FILTERS], entry_tc[ES_MAX_ENTRIES];
         block_tconst(c, s.t, caller_tc);
+        const bool prod = runs_production(c, tune, PF);
         if (prod) prod_tconst(c->prod[PF], caller_tc, entry_tc);
         h_tc.insert(h_tc.end(), prod ? entry_tc : caller_tc,
                     prod ? entry_tc + c->prod[PF].entries.size() : caller_tc + I.n_filters);
@@ -959,7 +1026,8 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     auto class_key = [&](uint32_t item) -> uint32_t {
         const EsInst& I = tables(ctxs[items[item].ctx_index]).h;
         uint32_t key = 2u * width_class(I.W);
-        if (!prod && tune.layout == ES_LAYOUT_AUTO && (I.W == 1 || I.W == 2)) {
+        if (!tune.count_stages) return key + (runs_production(ctxs[items[item].ctx_index], tune, PF) ? 1u : 0u);
+        if (tune.layout == ES_LAYOUT_AUTO && (I.W == 1 || I.W == 2)) {
             const uint32_t Fi = stage_filters(tune.layout, tune.mask_filters, I.n_filters, I.F_built);
             if (launch_layout(ES_LAYOUT_AUTO, I.W, (uint32_t)I.small_bytes, I.n_filters, tune, I.mask_off[Fi]) ==
                 ES_LAYOUT_SMEM)
@@ -1002,10 +1070,13 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         const uint32_t first_ctx = items[order[pos]].ctx_index;
         const uint32_t cls = width_class(ctxs[first_ctx]->geo.W);
         uint32_t end = pos, small_max = 0, nf_max = 1, stage_max = 0;
+        const bool prod = runs_production(ctxs[first_ctx], tune, PF);
+        const uint32_t layout = prod || tune.count_stages ? tune.layout : (uint32_t)ES_LAYOUT_SCALAR;
         uint32_t F = prod ? PF : tune.mask_filters;
         bool one_ctx = true;
         uint32_t words = ctxs[first_ctx]->geo.W;
-        uint64_t units = 0;
+        uint64_t units = 0, steps = 0;
+        es_tune shape = prod ? prod_shape(tune) : tune;
         while (end < n_items && keys[order[end]] == keys[order[pos]]) {
             const uint32_t ci = items[order[end]].ctx_index;
             const EsInst& I = tables(ctxs[ci]).h;
@@ -1013,20 +1084,26 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
             if (prod) {
                 // plans that fit a CTA's shared memory one by one may not fit it together
                 const uint32_t stage = std::max(stage_max, I.tab_words);
-                if (end > pos && plan_smem(small, 1, tune, stage).bytes > (uint32_t)g_dev.smem_optin - 1024u) break;
+                if (end > pos && plan_smem(small, 1, shape, stage).bytes > (uint32_t)g_dev.smem_optin - 1024u) break;
                 stage_max = stage;
             } else {
-                F = std::min(F, stage_filters(tune.layout, tune.mask_filters, I.n_filters, I.F_built));
+                F = std::min(F, stage_filters(layout, tune.mask_filters, I.n_filters, I.F_built));
             }
             small_max = small;
             nf_max = std::max<uint32_t>(nf_max, I.n_filters);
             if (ci != first_ctx) one_ctx = false;
             if (I.W != words) words = 0;   // the generic instance reads each plan's width
-            EsItem it = b->h_items[order[end]];
+            const EsItem& it = b->h_items[order[end]];
+            steps += steps_of(I, it.c_begin, it.c_end);
+            ++end;
+        }
+        if (prod) shape.strip = prod_strip(steps, shape);
+        for (uint32_t j = pos; j < end; ++j) {
+            EsItem& it = launch_items[j];
+            it = b->h_items[order[j]];
+            it.n_units = units_of(ctxs[items[order[j]].ctx_index]->geo, it.c_begin, it.c_end, shape.strip);
             it.unit_begin = units;
             units += it.n_units;
-            launch_items[end] = it;
-            ++end;
         }
         es_batch::Sub sub;
         sub.words = cls == 0 ? 0u : (cls == 4 && words == 0 ? 4u : (words ? words : cls));
@@ -1036,16 +1113,16 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
             uint32_t mask_words = 0;   // the largest inner-stage word-mask tables among the class's plans
             for (uint32_t j = pos; j < end; ++j)
                 mask_words = std::max<uint32_t>(mask_words, tables(ctxs[items[order[j]].ctx_index]).h.mask_off[F]);
-            sub.layout = launch_layout(tune.layout, sub.words, small_max, nf_max, tune, mask_words);
+            sub.layout = launch_layout(layout, sub.words, small_max, nf_max, shape, mask_words);
             stage_max = staged_words(sub.layout, mask_words);
         }
-        const SmemPlan sp = plan_smem(small_max, nf_max, tune, stage_max);
+        const SmemPlan sp = plan_smem(small_max, nf_max, shape, stage_max);
         EsLaunch& L = sub.L;
         memset(&L, 0, sizeof(L));
         L.items = b->d_items_launch + pos;
         L.n_items = end - pos;
-        L.threads = tune.threads;
-        L.strip = tune.strip;
+        L.threads = shape.threads;
+        L.strip = shape.strip;
         L.mask_filters = F;
         L.total_units = units;
         L.nf_max = nf_max;
@@ -1060,7 +1137,7 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         L.cnt_off = sp.cnt_off;
         L.queue_off = sp.queue_off;
         L.stage_off = sp.stage_off;
-        if (int e = grid_for(sub.layout, tune.count_stages, sub.words, F, tune, sp.bytes,
+        if (int e = grid_for(sub.layout, tune.count_stages, sub.words, F, shape, sp.bytes,
                              std::max<uint64_t>(units, 1), &sub.grid)) {
             es_batch_destroy(b);
             return e;
@@ -1259,8 +1336,9 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
     // the search never counts: the production cascade, or the scalar layout on request
     es_tune tn = c->tune;
     tn.count_stages = 0;
-    const bool prod = is_production(tn);
-    const uint32_t PF = prod_tables(tn);
+    const uint32_t PF = c->own_tables[prod_tables(tn)];
+    const bool prod = runs_production(c, tn, PF);
+    if (prod) tn = prod_shape(tn);
     const TableSet& T = prod ? c->prod[PF].t : c->caller;
     const EsInst& I = T.h;
     cudaStream_t st = (cudaStream_t)stream;
@@ -1293,6 +1371,7 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
     const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, nf, tn, prod ? I.tab_words : 0u);
     uint64_t cbeg = 0;
     const uint64_t ncyc = cycles_of(I, 0, I.n_outer, &cbeg);
+    if (prod) tn.strip = prod_strip(steps_of(I, cbeg, cbeg + ncyc) * n_blocks, tn);
     const uint64_t nu = units_of(I, cbeg, cbeg + ncyc, tn.strip);
     for (uint32_t i = 0; i < n_blocks; ++i) {
         const uint64_t t = t0 + i;

@@ -176,7 +176,7 @@ struct Slot {
 
 }  // namespace
 
-EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, uint32_t table_bytes) {
+EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes) {
     const uint32_t nf = (uint32_t)P.q.size();
     const double budget = (double)(table_bytes / row_bytes);
     std::vector<EsPart> parts;
@@ -208,7 +208,7 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     if (parts.size() > 48) parts.resize(48);
     auto rows = [&](uint32_t d) {
         const uint32_t m = (uint32_t)(P.M % d);
-        return (double)es_table_rows(d, m ? d - m : 0u);
+        return (double)es_table_rows(d, m ? d - m : 0u, pair);
     };
     std::vector<Slot> slots;
     const uint32_t np = (uint32_t)parts.size();
@@ -289,6 +289,7 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
         C.inner.push_back(t);
     }
     C.inner.resize(F);
+    C.rate = std::exp(-std::max(best_value, 0.0));
     std::vector<uint32_t> order;
     for (uint32_t f = 0; f < nf; ++f)
         if (!settled[f]) order.push_back(f);
@@ -316,22 +317,26 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     I = geo;
     const u128 M = P.M;
     const uint32_t r0 = I.r0, r1 = I.r1, r2 = I.r2, W = I.W, nf = I.n_filters, sh = I.sh;
-    const uint32_t RS = es_row_words(W), row_bytes = 4u * RS;
+    const uint32_t RS = es_row_words(W);
+    const bool pair = es_pair_rows(W);
+    const uint32_t stride = pair ? 2u * RS : RS, row_bytes = 4u * stride;   // words, bytes from phase to phase
     const uint32_t n_max = nf + F + ES_PRES;
     const uint32_t row1 = F <= 3 ? 16u : 32u, ds = F <= 4 ? 4u : 8u;   // ring-1 row bytes, step row words
     EsSmallBlock S;
     I.o_T1 = S.take(16ull * r1);
     I.o_R1 = S.take((size_t)row1 * (r1 + 1));   // + a padding row: digits are swept in pairs
     I.o_TQr = S.take(16ull * r1);
-    I.o_D2 = S.take(16ull * r2);
-    I.o_DQ2 = S.take(4ull * ds * r2);
-    I.o_DQr = S.take(16ull * r2);
+    I.o_T2 = S.take(16ull * r2);
+    I.o_TQ2 = S.take(4ull * ds * r2);
+    I.o_TQ2r = S.take(16ull * r2);
     I.o_S0 = S.take(16ull * r0);
     I.o_I0 = S.take(4ull * r0);
     I.o_Qr = S.take(16ull * r0);
     I.o_BK = S.take(4ull << ES_PBUCKET_LOG2);
     I.o_FC = S.take(sizeof(EsFilterC) * n_max);
-    const EsCascade C = es_choose_cascade(P, F, row_bytes, table_bytes(geo.n_outer * r0, smem_bytes, S.b.size()));
+    const EsCascade C = es_choose_cascade(P, F, row_bytes, pair, table_bytes(geo.n_outer * r0, smem_bytes, S.b.size()));
+
+    out.rate = C.rate;
 
     // ---- entries: inner tables, residue stage, tail ----------------------------------------
     std::vector<EsCascadeEntry>& entries = out.entries;
@@ -398,17 +403,19 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
             for (uint32_t ph = 0; ph < d - a; ++ph) phase[(size_t)ph * RS + wd] |= (uint32_t)adm[ph + a] << at;
             for (uint32_t ph = d - a; ph < d; ++ph) phase[(size_t)ph * RS + wd] |= (uint32_t)adm[ph + a - d] << at;
         }
-        const bool up = corr <= d - corr;
-        const uint32_t lead = up ? 0u : d - corr, rows = es_table_rows(d, corr);
-        I.tab_base[i] = 4u * (uint32_t)tabs.size() + lead * row_bytes;
-        I.tab_wrap[i] = up ? (int32_t)(corr * row_bytes) : -(int32_t)((d - corr) * row_bytes);
+        const bool up = pair || corr <= d - corr;
+        const uint32_t lead = up ? 0u : d - corr, rows = es_table_rows(d, corr, pair);
         const size_t at = tabs.size();
-        tabs.resize(at + (size_t)rows * RS);
-        uint32_t ph = lead ? d - lead : 0u;   // the first row's phase (lead <= d)
+        I.tab_base[i] = 4u * (uint32_t)at + lead * row_bytes;
+        I.tab_wrap[i] = pair ? (int32_t)(4u * RS) : up ? (int32_t)(corr * row_bytes) : -(int32_t)((d - corr) * row_bytes);
+        tabs.resize(at + (size_t)rows * stride);
+        uint32_t ph = lead ? d - lead : 0u, ph1 = corr;   // the first row's phase (lead <= d), its wrapped one
         if (ph == d) ph = 0;
         for (uint32_t r = 0; r < rows; ++r) {
-            memcpy(&tabs[at + (size_t)r * RS], &phase[(size_t)ph * RS], row_bytes);
+            memcpy(&tabs[at + (size_t)r * stride], &phase[(size_t)ph * RS], 4u * RS);
+            if (pair) memcpy(&tabs[at + (size_t)r * stride + RS], &phase[(size_t)ph1 * RS], 4u * RS);
             if (++ph == d) ph = 0;
+            if (++ph1 == d) ph1 = 0;
         }
         while (tabs.size() % 4) tabs.push_back(0u);
     }
@@ -453,10 +460,10 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_TQr, 4 * i + f, es_mod(v, entries[F + f].q));
     }
     for (uint32_t i = 0; i < r2; ++i) {
-        const u128 dlt = es_ring2_delta(P, i);
-        S.put128(I.o_D2, i, dlt);
-        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_DQ2, i * ds + f, es_mod(dlt, entries[f].q));
-        for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_DQr, 4 * i + f, es_mod(dlt, entries[F + f].q));
+        const u128 v = P.terms[P.roff[2] + i];
+        S.put128(I.o_T2, i, v);
+        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_TQ2, i * ds + f, es_mod(v, entries[f].q));
+        for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_TQ2r, 4 * i + f, es_mod(v, entries[F + f].q));
     }
     for (uint32_t i = 0; i < r0; ++i) {
         S.put128(I.o_S0, i, R.S0[i]);
@@ -464,6 +471,31 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_Qr, 4 * i + f, es_mod(R.S0[i], entries[F + f].q));
     }
     memcpy(&S.b[I.o_FC], fc.data(), sizeof(EsFilterC) * fc.size());
+    // ---- sums over groups of rings >= 3 --------------------------------------------------------
+    // (two neighbouring groups hold more than ES_GROUP_SIZE sums between them and R < 2^62, so there
+    // are far fewer than ES_MAX_GROUPS)
+    out.sums.clear();
+    I.n_groups = 0;
+    for (uint32_t j = 3; j < I.n_rings;) {
+        uint64_t size = 1;
+        std::vector<u128> sum(1, 0);
+        do {
+            std::vector<u128> next;
+            next.reserve(sum.size() * P.radix[j]);
+            for (uint32_t d = 0; d < P.radix[j]; ++d)   // the group's first ring is the fastest digit
+                for (const u128 v : sum) {
+                    const u128 x = v + P.terms[P.roff[j] + d];
+                    next.push_back(x >= M ? x - M : x);
+                }
+            sum.swap(next);
+            size *= P.radix[j++];
+        } while (j < I.n_rings && size * P.radix[j] <= ES_GROUP_SIZE);
+        EsGroup& G = I.group[I.n_groups++];
+        G.size = (uint32_t)size;
+        G.magic = ~0ull / size;
+        G.off = (uint32_t)out.sums.size();
+        out.sums.insert(out.sums.end(), sum.begin(), sum.end());
+    }
     I.n_filters = (uint32_t)entries.size();
     I.F = F;
     I.bsh = bsh;

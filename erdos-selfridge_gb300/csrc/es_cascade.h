@@ -47,17 +47,25 @@ struct EsCascade {
     std::vector<std::vector<EsPart>> inner;
     std::vector<int> residue;
     std::vector<uint32_t> tail;
+    double rate = 1.0;    // share of the candidates that pass the inner tables
 };
 
-// Rows of an inner table of modulus d whose wrap correction is corr: phases up to 2 d - 2 come
-// unreduced, plus the nearer of +corr and corr - d for the wrapped row.
-inline uint32_t es_table_rows(uint32_t d, uint32_t corr) {
+// Inner rings of one word have the masks of a phase and of the phase a wrap past M selects side by
+// side in one row: one 8-byte load instead of two 4-byte ones, for rows twice as long (but none
+// beyond the 2 d - 1 unreduced phases).  Wider rings keep them apart, where the shorter tables let
+// more projections share one: k = 390 (two words), 2^34 positions, 2004 us with pair rows and 1686
+// without.
+inline bool es_pair_rows(uint32_t W) { return W <= 1; }
+
+// Rows of an inner table of modulus d whose wrap correction is corr: unreduced phases up to
+// 2 d - 2 and, where the wrapped masks are rows of their own, the nearer of +corr and corr - d.
+inline uint32_t es_table_rows(uint32_t d, uint32_t corr, bool pair) {
     const uint32_t ext = corr <= d - corr ? corr : d - corr;
-    return 2u * d - 1u + ext;
+    return 2u * d - 1u + (pair ? 0u : ext);
 }
 
 // Chooses F inner tables whose rows of row_bytes bytes fit table_bytes in all.
-EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, uint32_t table_bytes);
+EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes);
 
 // An entry of a production cascade: the residue of n mod q is needed.  Its block constant follows
 // from the caller's by CRT over the entry's parts (unit = 1 mod d of its own part, 0 mod the
@@ -73,8 +81,10 @@ struct EsCascadeEntry {
 // The tables of a plan's production cascade, as the device gets them.
 struct EsProdImage {
     EsInst inst{};
+    double rate = 1.0;    // share of the candidates that pass the inner tables
     std::vector<unsigned char> small;
     std::vector<uint32_t> tabs, bits;
+    std::vector<es_u128> sums;   // over the groups of rings >= 3
     std::vector<EsCascadeEntry> entries;
 };
 

@@ -34,6 +34,9 @@
 #define ES_MAX_ENTRIES (ES_MAX_FILTERS + ES_PMAX + ES_PRES)   // entries of a cascade, with fill-ins
 #define ES_PBUCKET_LOG2 11   // carry-split buckets of the production cascade
 
+// Largest CTA of a production launch: 20 warps of 96 registers (es_prod_kernel.cuh says why).
+#define ES_PROD_THREADS 640
+
 struct EsFilterC {
     uint32_t q;      // modulus p^t_p (< 2^20)
     uint32_t corr;   // (q - M mod q) mod q: residue correction when a sum wraps mod M
@@ -43,6 +46,15 @@ struct EsFilterC {
     uint32_t off;    // word offset of this filter's bit table
     uint64_t rcp;    // floor(2^64 / q): Barrett reciprocal for 64-bit residues
 };
+
+// Sums over a group of consecutive rings (>= 3), ring after ring mixed radix, first ring fastest.
+struct EsGroup {
+    uint64_t magic;   // floor((2^64 - 1) / size)
+    uint32_t size;    // product of the rings' radices
+    uint32_t off;     // first entry in the ring-term array
+};
+#define ES_MAX_GROUPS 32
+#define ES_GROUP_SIZE 2048   // rings are grouped while their product stays within this
 
 struct EsInst {
     uint64_t M_lo, M_hi;
@@ -64,14 +76,18 @@ struct EsInst {
     uint32_t F;           // inner tables (0 in a caller-order table set)
     uint32_t o_R1;        // [r1 + 1] ring-1 rows: key, then the inner tables' scaled term residues
     uint32_t o_TQr;       // [r1] term residues of the residue-stage filters
-    uint32_t o_DQr;       // [r2] step residues of the residue-stage filters
+    uint32_t o_T2;        // [r2] ring-2 terms
+    uint32_t o_TQ2;       // [r2] ring-2 term residues of the inner tables (rows of 4 or 8 words)
+    uint32_t o_TQ2r;      // [r2] ring-2 term residues of the residue-stage filters
     uint32_t o_Qr;        // [r0] inner-ring residues of the residue-stage filters
     uint32_t ssh;         // 32 - bsh: bucket entries hold the key's low bits above the slot
     uint32_t band;        // key distance below which the split is found exactly, << ssh
-    uint32_t row_bytes;   // bytes of a table row
+    uint32_t row_bytes;   // bytes from one phase's row to the next
     uint32_t tab_base[ES_PMAX];   // byte offset of each table's phase-0 row in the staged block
     int32_t tab_wrap[ES_PMAX];    // byte distance from a row to the row a wrap past M selects
     uint32_t tab_words;   // words of all inner tables
+    uint32_t n_groups;    // groups of rings >= 3, whose sums are ring_terms
+    EsGroup group[ES_MAX_GROUPS];
     // word offsets of the fast (word-mask) tables, F_built + 1 entries (prefix sums)
     uint32_t mask_off[ES_FMAX + 1];
     uint32_t mask_stride;            // words per phase row of P_f: W, or 4 for W = 3 (16-byte rows)

@@ -10,26 +10,35 @@
 //  * Every inner table lies in shared memory, whatever the filters' moduli (the cascade's tables
 //    are products of small projections), so one kernel serves every plan and no filter reads its
 //    phases through L2.
-//  * No residue is reduced in the sweep.  A table has a row for every unreduced phase
-//    BQ2 + TQ1 < 2 d, and beyond them (or before them) the rows that a wrap past M selects, so
-//    a lookup is: select BQ2 with or without the ring-1 wrap, add the digit's residue, load;
-//    add the wrap distance, load.  Residues are kept as byte offsets and BQ2 as the shared
-//    address itself.
+//  * No residue is reduced in the sweep: a table has a row for every unreduced phase
+//    BQ2 + TQ1 < 2 d.  In one-word rings a row holds the masks of both sides of the carry split
+//    (phase x and x + corr), so a lookup is: select BQ2 with or without the ring-1 wrap, add the
+//    digit's residue, load.  Wider rings have the wrapped row a fixed distance away.  Residues
+//    are kept as byte offsets and BQ2 as the shared address itself.
+//  * The tables after the first two are read only by lanes that still hold a candidate: a random
+//    gather costs shared-memory wavefronts by its active lanes.
 //  * The carry split is one 4-byte load: a bucket entry holds the first slot and the low bits of
 //    the one key that may lie in the bucket.  Buckets with more keys, key ties and keys within the
 //    rounding band take the exact 128-bit path out of line.
-//  * The masks of both sides of the carry split are gathered over all tables first and merged once.
+//  * A lane's record is b3, the sum of its terms of rings >= 3, and its residues.  They hold for
+//    the whole window, ring 2 is added where it is needed, and so the queue of candidates outlives
+//    a strip step: it is flushed 32 entries at a time and drained once per warp-unit.
+//  * b3 is decoded from tables of sums over groups of rings (es_cascade.cu), a few 64-bit
+//    divisions by reciprocal instead of one division per ring.
 //  * Lanes outside the scanned range sweep along and are dropped at the end of the cascade (only
 //    candidates that pass the residue stage get that far), so the sweep has no per-digit test for
 //    partial cycles.  An explicit list of outer indices gives each lane its own ring-1 digit and
 //    no sweep.
 //
-// What bounds it: instruction issue and shared-memory wavefronts (a random 4-byte gather of 32
-// lanes takes 3 to 4).  Measured through the drop-in calls against the caller's cascade by
-// word-mask or pair tables (the layouts of es_scan_kernel.cuh): k = 300, 2^34 positions 3,071 ->
-// 1,927 us (8.9 T candidates/s); the three-word k = 379 wheel, 2^34 positions, 5,508 -> 2,340 us;
-// both k = 390 wheels, 2^35 positions each, 17,115 -> 7,884 us (their caller-order tables, 1.75 MB
-// per wheel, came through L2).
+// CTA: one per SM, 20 warps at 96 registers.  16 warps at 128 registers leave the scheduler short of
+// ready warps (k = 300, 2^34 positions: 1469 against 1369 us), 24 at 80 spill in wide rings (k = 379:
+// 2209 against 1842 us).
+//
+// What bounds it: shared-memory wavefronts (l1tex 78 to 83 % busy) and instruction issue (63 % at
+// k = 300).  Through the drop-in calls, against the caller's cascade by word-mask or pair tables
+// (es_scan_kernel.cuh): k = 300, 2^34 positions 3068 -> 1559 us, 2^30 positions 320 -> 197 us; the
+// three-word k = 379 wheel, 2^34 positions, 5500 -> 1940 us; both k = 390 wheels, 2^35 positions
+// each, 17,068 -> 6297 us (their caller-order tables, 1.75 MB per wheel, came through L2).
 #pragma once
 #include "es_scan_kernel.cuh"
 
@@ -53,15 +62,19 @@ struct ProdCtx {
     uint64_t surv_cap;
     uint32_t kp1, nf, item_id, group, r0, r1;
     uint32_t lstride;                  // entries between the strips of consecutive lanes
+    uint64_t row0;                     // ring-2 row of lane 0 (where lanes stay on their rows)
+    uint32_t d2;                       // ring-2 digit of step 0
     uint32_t M_big;
 };
 
 struct ProdQueue {
     uint4 ent[ES_QCAP];
-    uint4 rec0[32];                    // per lane: b2 (limbs)
-    uint4 rec1[32];                    // per lane: b2 + block term mod the residue-stage filters
+    uint4 rec0[32];                    // per lane: b3 = sum of the terms of rings >= 3, mod M (limbs)
+    uint4 rec1[32];                    // per lane: b3 + block term mod the residue-stage filters
+    uint16_t own_d2[32];               // per lane: ring-2 digit, where lanes do not share it
     ProdCtx ctx;
 };
+#define ES_OWN_DIGIT 0xffffffffu       // ProdCtx::d2 where lanes do not share the ring-2 digit
 static_assert(sizeof(ProdQueue) <= ES_QUEUE_BYTES, "per-warp slot overflows its shared-memory share");
 
 __device__ __forceinline__ uint32_t shl_c(uint32_t v, uint32_t n) {   // shifts of 32 and more give 0
@@ -70,10 +83,44 @@ __device__ __forceinline__ uint32_t shl_c(uint32_t v, uint32_t n) {   // shifts 
     return r;
 }
 
+// Predicated loads: lanes whose `alive` is 0 load nothing and get an arbitrary value.
+__device__ __forceinline__ uint2 lds64_if(uint32_t a, uint32_t alive) {
+    uint2 v;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p ld.shared.v2.u32 {%0, %1}, [%2];\n\t}"
+        : "=r"(v.x), "=r"(v.y) : "r"(a), "r"(alive));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128_if(uint32_t a, uint32_t alive) {
+    uint4 v;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a), "r"(alive));
+    return v;
+}
+
+// b3 = sum_{j>=3} term_j[d_j] mod M for ring-2 row `row`, from the sums over groups of rings.
+__device__ __noinline__ U4 decode_row(const EsInst& si, uint64_t row, const U4 M) {
+    U4 acc{0u, 0u, 0u, 0u};
+    uint64_t rem = row;
+    for (uint32_t g = 0; g < si.n_groups; ++g) {
+        const EsGroup G = si.group[g];
+        // floor(rem / size) or one less (magic = floor((2^64 - 1) / size)), then corrected
+        uint64_t q = __umul64hi(rem, G.magic);
+        uint64_t d = rem - q * G.size;
+        if (d >= G.size) {
+            d -= G.size;
+            ++q;
+        }
+        rem = q;
+        uint32_t wm;
+        acc = addmod(acc, u4(__ldg(reinterpret_cast<const uint4*>(si.ring_terms) + (G.off + d))), M, wm);
+    }
+    return acc;
+}
+
 // The candidates that passed the residue stage: range test, n mod M in 128 bits, the rest of the
 // cascade by limb weights and Barrett, then the emit.
 __device__ __forceinline__ void prod_tail(const ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t f0,
-                                          uint32_t own, uint32_t d1, uint32_t slot, uint32_t step) {
+                                          const U4 b2, uint32_t own, uint32_t d1, uint32_t slot, uint32_t step) {
     const ProdCtx& C = Q->ctx;
     const uint64_t e = C.e_base + (uint64_t)own * C.lstride + step;
     if (e < C.e_min || e >= C.e_max) return;
@@ -81,7 +128,7 @@ __device__ __forceinline__ void prod_tail(const ProdQueue* Q, const unsigned cha
     if (oidx < C.o_begin || oidx >= C.o_end) return;
     const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
     uint32_t wm;
-    const U4 b = addmod(u4(Q->rec0[own]), u4(reinterpret_cast<const uint4*>(smem + si.o_T1)[d1]), C.M, wm);
+    const U4 b = addmod(b2, u4(reinterpret_cast<const uint4*>(smem + si.o_T1)[d1]), C.M, wm);
     const U4 s = addmod(b, u4(reinterpret_cast<const uint4*>(smem + si.o_S0)[slot]), C.M, wm);
     for (uint32_t f = f0; f < C.nf; ++f) {
         const EsFilterC fc = sFC[f];
@@ -110,12 +157,16 @@ __device__ __forceinline__ void prod_tail(const ProdQueue* Q, const unsigned cha
     if (good && C.group_found) atomicMin(C.group_found + C.group, (unsigned long long)C.t_blk);
 }
 
-// warp-uniform: one pass over up to 32 queued entries (the entry formats are those of
-// es_scan_kernel.cuh's flush; PD: two ring-1 digits per entry).  Each lane takes the lowest
-// candidate of its entry and puts the rest of the entry back.
+// warp-uniform: one pass over up to 32 queued entries.  Each lane takes the lowest candidate of its
+// entry and puts the rest of the entry back.  Entry formats: words (w, w + 1) of one ring-1 digit:
+// {bits of w, bits of w + 1, d1 | split << 16, lane | wrap << 5 | w << 6 | step << 17}; or, with PD
+// (one-word inner rings), the words of two consecutive digits d1, d1 + 1: {bits of d1, bits of
+// d1 + 1, d1 | split(d1) << 16 | split(d1 + 1) << 24, lane | wrap(d1) << 5 | wrap(d1 + 1) << 6 |
+// step << 17}.  Where lanes do not share the ring-2 digit it is in the lane's record (own_d2), and
+// the queue is drained before the next step.
 template <int F, bool PD>
 __device__ __forceinline__ void prod_flush(ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t lane,
-                                           uint32_t step, uint32_t& qhead, uint32_t& qsize) {
+                                           uint32_t& qhead, uint32_t& qsize) {
     __syncwarp();
     const uint32_t n = qsize < 32u ? qsize : 32u;
     const uint4 en = Q->ent[(qhead + lane) & (ES_QCAP - 1)];
@@ -135,33 +186,40 @@ __device__ __forceinline__ void prod_flush(ProdQueue* Q, const unsigned char* sm
     const uint32_t i = has ? __ffsll((long long)bits) - 1u : 0u;
     const uint32_t hw = PD ? (i >> 5) : 0u;        // PD: the candidate is in the second digit's word
     const uint32_t d1 = has ? (en.z & 0xffffu) + hw : 0u;
-    const uint32_t slot = has ? (PD ? (i & 31u) : ((en.w >> 6) << 5) + i) : 0u;
+    const uint32_t slot = has ? (PD ? (i & 31u) : (((en.w >> 6) & 0x7ffu) << 5) + i) : 0u;
     const uint32_t own = has ? (en.w & 31u) : 0u;
+    const uint32_t step = has ? en.w >> 17 : 0u;
     const bool wrap1 = has && ((en.w >> (5u + hw)) & 1u);
     const uint32_t split = PD ? (hw ? (en.z >> 24) : ((en.z >> 16) & 0xffu)) : (en.z >> 16);
     const bool cw = has && slot >= split;          // sorted slots from the split on wrap past M
     const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
     const uint32_t* allowed = si.allowed;
+    const uint32_t d2 = Q->ctx.d2 == ES_OWN_DIGIT ? Q->own_d2[own] : Q->ctx.d2 + step;
+    uint32_t wm2;
+    const U4 b2 = addmod(u4(Q->rec0[own]), u4(reinterpret_cast<const uint4*>(smem + si.o_T2)[d2]), ldv_M(si), wm2);
     const uint4 bq = Q->rec1[own];
+    const uint4 t2 = reinterpret_cast<const uint4*>(smem + si.o_TQ2r)[d2];
     const uint4 tq = reinterpret_cast<const uint4*>(smem + si.o_TQr)[d1];
     const uint4 sq = reinterpret_cast<const uint4*>(smem + si.o_Qr)[slot];
-    const uint32_t bqv[ES_PRES] = {bq.x, bq.y, bq.z, bq.w};
-    const uint32_t tqv[ES_PRES] = {tq.x, tq.y, tq.z, tq.w};
-    const uint32_t sqv[ES_PRES] = {sq.x, sq.y, sq.z, sq.w};
+    const uint32_t bqv[ES_PRES] = {bq.x + t2.x, bq.y + t2.y, bq.z + t2.z, bq.w + t2.w};
+    const uint32_t sqv[ES_PRES] = {sq.x + tq.x, sq.y + tq.y, sq.z + tq.z, sq.w + tq.w};
+    // n mod q = b3 + T2[d2] + T1[d1] + S0[slot] mod q, with -M mod q per wrap
+    const uint32_t wraps = (wm2 & 1u) + (wrap1 ? 1u : 0u) + (cw ? 1u : 0u);
     bool ok = has;
 #pragma unroll
     for (uint32_t j = 0; j < ES_PRES; ++j) {
         if (j == 0 || __any_sync(0xffffffffu, ok)) {
             const EsFilterC& fc = sFC[F + j];
-            const uint32_t q = fc.q, corr = fc.corr;
-            // n mod q = b2 + T1[d1] + S0[slot] mod q, with -M mod q per wrap
-            uint32_t x = red2(bqv[j] + tqv[j] + (wrap1 ? corr : 0u), q);
-            x = red2(x + sqv[j] + (cw ? corr : 0u), q);
+            const uint32_t q = fc.q;
+            uint32_t x = bqv[j] + sqv[j] + wraps * fc.corr;   // < 7 q
+            x = min(x, x - 4u * q);
+            x = min(x, x - 2u * q);
+            x = min(x, x - q);
             const uint32_t wv = __ldg(allowed + fc.off + (x >> 5));
             ok = ok && ((wv >> (x & 31u)) & 1u);
         }
     }
-    if (ok) prod_tail(Q, smem, si, F + ES_PRES, own, d1, slot, step);
+    if (ok) prod_tail(Q, smem, si, F + ES_PRES, b2, own, d1, slot, step);
     __syncwarp();
 }
 
@@ -169,25 +227,26 @@ __device__ __forceinline__ void prod_flush(ProdQueue* Q, const unsigned char* sm
 // every lane that has candidates, then flush while 32 entries wait
 template <int F, bool PD>
 __device__ __forceinline__ void prod_push(ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t lane,
-                                          uint32_t step, uint32_t& qhead, uint32_t& qsize, uint32_t has, uint32_t lo,
-                                          uint32_t hi, uint32_t ez, uint32_t ew) {
+                                          uint32_t& qhead, uint32_t& qsize, uint32_t has, uint32_t lo, uint32_t hi,
+                                          uint32_t ez, uint32_t ew) {
     if (lo | hi) {
         const uint32_t pos = (qhead + qsize + __popc(has & ((1u << lane) - 1u))) & (ES_QCAP - 1);
         Q->ent[pos] = make_uint4(lo, hi, ez, ew);
     }
     qsize += __popc(has);
     // each pass retires one candidate per lane, so this ends
-    while (qsize >= 32u) prod_flush<F, PD>(Q, smem, si, lane, step, qhead, qsize);
+    while (qsize >= 32u) prod_flush<F, PD>(Q, smem, si, lane, qhead, qsize);
 }
 
 // The exact ring-1 wrap and carry split of digit d1 for one lane, in 128 bits: b = b2 + T1[d1] mod
 // M, then the first sorted slot whose term is >= M - b.  Returns the slot, with the top bit set on a
 // wrap.  Out of line: it runs for a tiny share of (lane, digit) pairs.
 __device__ __noinline__ uint32_t prod_split(const ProdQueue* Q, const unsigned char* smem, const EsInst& si,
-                                            uint32_t lane, uint32_t d1) {
+                                            uint32_t lane, uint32_t d2, uint32_t d1) {
     const U4 M = ldv_M(si);
     uint32_t wm, br;
-    const U4 b = addmod(ldv128(&Q->rec0[lane]), ldv128(smem + si.o_T1 + 16u * d1), M, wm);
+    const U4 b2 = addmod(ldv128(&Q->rec0[lane]), ldv128(smem + si.o_T2 + 16u * d2), M, wm);
+    const U4 b = addmod(b2, ldv128(smem + si.o_T1 + 16u * d1), M, wm);
     const U4 thr = sub128(M, b, br);
     const uint4* S0 = reinterpret_cast<const uint4*>(smem + si.o_S0);
     uint32_t lo = 0, hi = si.r0;
@@ -228,29 +287,34 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
     constexpr uint32_t NW = WT == 0 ? 1u : (uint32_t)WT;   // inner words held at a time
     constexpr uint32_t NU = WT == 1 ? 2u : 1u;             // ring-1 digits per loop iteration
     constexpr bool PD = WT == 1;
-    const uint32_t* tcv = L.items ? item.tconst : L.tconst0;
     const uint32_t r1 = si.r1, r2 = si.r2;
     const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
-    const uint64_t* list = item.list;
+    const bool list = item.list != nullptr;
     // This unit's entries, decoded as in es_scan_kernel.cuh's scan_unit (units_of in es_abi.cu).
     const uint64_t u = w - item.unit_begin;
     const uint64_t c_lo = list ? item.o_begin : item.c_begin, c_hi = list ? item.o_end : item.c_end;
-    uint64_t e_base, e_lo;
-    uint32_t lstride, nsteps;
+    uint64_t e_base, e_lo, row0 = 0;
+    uint32_t lstride, nsteps, wlo = 0;
     if (!list && r2 > 1u) {
         const uint32_t J = (r2 + L.strip - 1u) / L.strip;
         const uint64_t rb = u / J;
         const uint32_t j = (uint32_t)(u - rb * J);
-        const uint32_t wlo = j * r2 / J;
+        wlo = j * r2 / J;
         nsteps = (j + 1u) * r2 / J - wlo;
         lstride = r2;
-        e_base = (item.c_begin / r2 + rb * 32ull) * r2 + wlo;
+        row0 = item.c_begin / r2 + rb * 32ull;
+        e_base = row0 * r2 + wlo;
     } else {
         nsteps = lstride = L.strip;
         e_base = c_lo + u * 32ull * L.strip;
     }
     e_lo = e_base + (uint64_t)lane * lstride;
-    const uint64_t e_min = max(e_lo, c_lo), e_hi = min(e_lo + nsteps, c_hi);
+    const bool rows = !list && r2 > 1u;   // each lane stays on its ring-2 row for the whole unit
+    // this lane's steps in range: [first, last); the unit takes as many steps as its longest lane
+    const uint64_t e_end = min(e_lo + nsteps, c_hi);
+    const uint32_t last = e_end > e_lo ? (uint32_t)(e_end - e_lo) : 0u;
+    const uint32_t first = e_lo >= c_lo ? 0u : (uint32_t)min(c_lo - e_lo, (uint64_t)nsteps);
+    nsteps = __reduce_max_sync(0xffffffffu, last);
     ProdCtx& C = Q->ctx;
     if (lane == 0) {
         C.M = U4{(uint32_t)si.M_lo, (uint32_t)(si.M_lo >> 32), (uint32_t)si.M_hi, (uint32_t)(si.M_hi >> 32)};
@@ -260,7 +324,7 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
         C.nf = si.n_filters;
         C.r0 = si.r0;
         C.r1 = r1;
-        C.tc = tcv;
+        C.tc = L.items ? item.tconst : L.tconst0;
         C.allowed_g = si.allowed;
         C.surv = L.surv;
         C.surv_n = L.surv_n;
@@ -270,87 +334,77 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
         C.group = item.group;
         C.t_blk = item.t;
         C.lstride = lstride;
-        C.list = reinterpret_cast<const unsigned long long*>(list);
+        C.d2 = rows ? wlo : ES_OWN_DIGIT;
+        C.row0 = row0;
+        C.list = reinterpret_cast<const unsigned long long*>(item.list);
         C.e_base = e_base;
         C.e_min = c_lo;
         C.e_max = c_hi;
         C.o_begin = list ? 0ull : item.o_begin;
         C.o_end = list ? ~0ull : item.o_end;
     }
-    // lanes that never reach a cycle of the range sweep with b2 = 0 (their candidates are dropped)
+    // lanes that never reach a cycle of the range sweep with b3 = 0 (their candidates are dropped)
     Q->rec0[lane] = make_uint4(0u, 0u, 0u, 0u);
     Q->rec1[lane] = make_uint4(0u, 0u, 0u, 0u);
+    Q->own_d2[lane] = 0;
     __syncwarp();
 
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t rb = si.row_bytes, KM = si.km, bsh = si.bsh, ssh = si.ssh, band = si.band;
     const uint32_t smask = ssh >= 32u ? 0xffffffffu : (1u << ssh) - 1u;
     const uint32_t bk = sbase + si.o_BK;
-    uint32_t qf[F], corr[F], base[F];
-    int32_t wrap[F];
+    int32_t wrap[F];   // (one- and two-word rings have the wrapped row in the row itself)
 #pragma unroll
-    for (int f = 0; f < F; ++f) {
-        qf[f] = sFC[f].q;
-        corr[f] = sFC[f].corr;
-        base[f] = sbase + L.stage_off + si.tab_base[f];
-        wrap[f] = si.tab_wrap[f];
-    }
-    uint32_t BQ2[F];
+    for (int f = 0; f < F; ++f) wrap[f] = si.tab_wrap[f];
+    uint32_t BQ3[F];   // b3 + block term mod the inner tables' moduli
 #pragma unroll
-    for (int f = 0; f < F; ++f) BQ2[f] = 0u;
-    uint32_t qhead = 0, qsize = 0, d2 = 0;
-    bool have = false;
-    uint64_t prev_c = 0;
+    for (int f = 0; f < F; ++f) BQ3[f] = 0u;
+    uint32_t qhead = 0, qsize = 0;
     for (uint32_t step = 0; step < nsteps; ++step) {
-        const uint64_t e = e_lo + step;
-        const bool live = e >= e_min && e < e_hi;
-        if (__ballot_sync(0xffffffffu, e < e_hi) == 0u) break;   // no lane has entries left
-        uint32_t lo1 = 0u;
+        uint32_t lo1 = 0u, d2 = rows ? wlo + step : 0u;
         const U4 Mv = ldv_M(si);
-        U4 b2 = ldv128(&Q->rec0[lane]);   // of the lane's last cycle (0 before the first decode)
-        if (live) {
-            uint64_t c = e;
-            if (list) {
-                const uint64_t o = __ldg(reinterpret_cast<const unsigned long long*>(list) + e);
-                c = o / r1;
-                lo1 = (uint32_t)(o - c * r1);
+        if (rows ? (step == 0u && first < last) : (step >= first && step < last)) {
+            const uint64_t e = Q->ctx.e_base + (uint64_t)lane * Q->ctx.lstride + step;
+            const uint32_t* tcv = Q->ctx.tc;
+            uint64_t row;
+            if (rows) {
+                row = Q->ctx.row0 + lane;
+            } else {
+                uint64_t c = e;
+                if (list) {
+                    const uint64_t o = __ldg(Q->ctx.list + e);
+                    c = o / r1;
+                    lo1 = (uint32_t)(o - c * r1);
+                }
+                row = c / r2;
+                d2 = (uint32_t)(c - row * r2);
+                Q->own_d2[lane] = (uint16_t)d2;
             }
-            // rings >= 2: one delta step while the ring-2 digit advances, else a decode
-            if (have && c == prev_c + 1 && d2 + 1u < r2) {
-                uint32_t wm;
-                b2 = addmod(b2, u4(reinterpret_cast<const uint4*>(smem + si.o_D2)[d2]), Mv, wm);
-                constexpr uint32_t DS = F <= 4 ? 4u : 8u;
-                const uint32_t* dq = reinterpret_cast<const uint32_t*>(smem + si.o_DQ2) + d2 * DS;
+            const U4 b3 = decode_row(si, row, Mv);
 #pragma unroll
-                for (int f = 0; f < F; ++f) BQ2[f] = red2(BQ2[f] + dq[f] + (corr[f] & wm), qf[f]);
-                const uint4 rq = Q->rec1[lane];
-                const uint4 dr = reinterpret_cast<const uint4*>(smem + si.o_DQr)[d2];
-                uint32_t rv[ES_PRES] = {rq.x + dr.x, rq.y + dr.y, rq.z + dr.z, rq.w + dr.w};
+            for (int f = 0; f < F; ++f) BQ3[f] = red1(mod128(b3, sFC[f]) + tcv[f], sFC[f].q);
+            uint32_t rv[ES_PRES];
 #pragma unroll
-                for (uint32_t j = 0; j < ES_PRES; ++j) rv[j] = red2(rv[j] + (sFC[F + j].corr & wm), sFC[F + j].q);
-                Q->rec0[lane] = make_uint4(b2.x, b2.y, b2.z, b2.w);
-                Q->rec1[lane] = make_uint4(rv[0], rv[1], rv[2], rv[3]);
-                ++d2;
-            } else if (!(have && c == prev_c)) {
-                b2 = decode_cycle(si, c, Mv, d2);
-#pragma unroll
-                for (int f = 0; f < F; ++f) BQ2[f] = red1(mod128(b2, sFC[f]) + tcv[f], qf[f]);
-                uint32_t rv[ES_PRES];
-#pragma unroll
-                for (uint32_t j = 0; j < ES_PRES; ++j) rv[j] = red1(mod128(b2, sFC[F + j]) + tcv[F + j], sFC[F + j].q);
-                Q->rec0[lane] = make_uint4(b2.x, b2.y, b2.z, b2.w);
-                Q->rec1[lane] = make_uint4(rv[0], rv[1], rv[2], rv[3]);
-                have = true;
-            }
-            prev_c = c;
+            for (uint32_t j = 0; j < ES_PRES; ++j) rv[j] = red1(mod128(b3, sFC[F + j]) + tcv[F + j], sFC[F + j].q);
+            Q->rec0[lane] = make_uint4(b3.x, b3.y, b3.z, b3.w);
+            Q->rec1[lane] = make_uint4(rv[0], rv[1], rv[2], rv[3]);
         }
+        uint32_t wm2;
+        const U4 b2 = addmod(ldv128(&Q->rec0[lane]), u4(reinterpret_cast<const uint4*>(smem + si.o_T2)[d2]), Mv, wm2);
         // shared addresses of the tables' rows at BQ2 without and with the ring-1 wrap
         uint32_t B[F], Bc[F];
+        constexpr uint32_t DS = F <= 4 ? 4u : 8u;
+        const uint32_t* tq2 = reinterpret_cast<const uint32_t*>(smem + si.o_TQ2) + d2 * DS;
 #pragma unroll
         for (int f = 0; f < F; ++f) {
-            B[f] = base[f] + rb * BQ2[f];
-            Bc[f] = base[f] + rb * red1(BQ2[f] + corr[f], qf[f]);
+            // (volatile loads: constants of the step are not worth registers in the sweep)
+            const uint32_t q = ldv32(&sFC[f].q), corr = ldv32(&sFC[f].corr);
+            const uint32_t base = sbase + L.stage_off + ldv32(&si.tab_base[f]);
+            const uint32_t BQ2 = red2(BQ3[f] + tq2[f] + (corr & wm2), q);
+            B[f] = base + rb * BQ2;
+            Bc[f] = base + rb * red1(BQ2 + corr, q);
         }
+        const uint32_t ews = lane | (step << 17);   // entry fields that belong to the step
         // A = M - b2 and its 32-bit key, once per ring-1 cycle
         uint32_t brA;
         const uint32_t KA = key32(sub128(Mv, b2, brA), si.sh);
@@ -386,7 +440,7 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
                 for (uint32_t v = 0; v < NU; ++v) {
                     // the padding row after the last digit has no term of its own
                     if (rare[v] && d1 + v < r1) {
-                        const uint32_t was = wm1[v], x = prod_split(Q, smem, si, lane, d1 + v);
+                        const uint32_t was = wm1[v], x = prod_split(Q, smem, si, lane, d2, d1 + v);
                         split[v] = x & 0x7fffffffu;
                         wm1[v] = (x >> 31) ? 0xffffffffu : 0u;
 #pragma unroll
@@ -417,61 +471,75 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
                     const uint32_t p0 = odd ? lo : x, p1 = odd ? x : 0u;
                     const uint32_t has = __ballot_sync(0xffffffffu, (p0 | p1) != 0u);
                     if (has)
-                        prod_push<F, PD>(Q, smem, si, lane, step, qhead, qsize, has, p0, p1, ent_z(d1, split[0]),
-                                         ent_w(lane, wm1[0], wd & ~1u));
+                        prod_push<F, PD>(Q, smem, si, lane, qhead, qsize, has, p0, p1, ent_z(d1, split[0]),
+                                         ent_w(ews, wm1[0], wd & ~1u));
                 }
             } else {
 #pragma unroll
-            for (uint32_t v = 0; v < NU; ++v) {
-                uint32_t m0[NW], m1[NW];
-#pragma unroll
-                for (int f = 0; f < F; ++f) {
-                    uint32_t x0[NW], x1[NW];
-                    if (WT == 1) {
-                        x0[0] = lds32(a[v][f]);
-                        x1[0] = lds32(a[v][f] + wrap[f]);
-                    } else if (WT == 2) {
-                        const uint2 y0 = lds64(a[v][f]), y1 = lds64(a[v][f] + wrap[f]);
-                        x0[0] = y0.x; x0[NW > 1 ? 1 : 0] = y0.y;
-                        x1[0] = y1.x; x1[NW > 1 ? 1 : 0] = y1.y;
-                    } else {
-                        const uint4 y0 = lds128(a[v][f]), y1 = lds128(a[v][f] + wrap[f]);
-                        x0[0] = y0.x; x0[NW > 1 ? 1 : 0] = y0.y; x0[NW > 2 ? 2 : 0] = y0.z; x0[NW > 3 ? 3 : 0] = y0.w;
-                        x1[0] = y1.x; x1[NW > 1 ? 1 : 0] = y1.y; x1[NW > 2 ? 2 : 0] = y1.z; x1[NW > 3 ? 3 : 0] = y1.w;
-                    }
+                for (uint32_t v = 0; v < NU; ++v) {
+                    // candidates on either side of the split that every table so far admits
+                    uint32_t m0[NW], m1[NW];
 #pragma unroll
                     for (uint32_t j = 0; j < NW; ++j) {
-                        m0[j] = f == 0 ? x0[j] : m0[j] & x0[j];
-                        m1[j] = f == 0 ? x1[j] : m1[j] & x1[j];
+                        m1[j] = shl_c(0xffffffffu, j == 0 ? split[v] : max(split[v], 32u * j) - 32u * j);
+                        m0[j] = ~m1[j];
+                    }
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        uint32_t x0[4], x1[4];
+                        if (WT == 1) {
+                            const uint2 y = f < 2 ? lds64(a[v][f]) : lds64_if(a[v][f], m0[0] | m1[0]);
+                            x0[0] = y.x;
+                            x1[0] = y.y;
+                        } else if (WT == 2) {
+                            const uint2 y0 = f < 2 ? lds64(a[v][f]) : lds64_if(a[v][f], m0[0] | m0[NW - 1]);
+                            const uint2 y1 =
+                                f < 2 ? lds64(a[v][f] + wrap[f]) : lds64_if(a[v][f] + wrap[f], m1[0] | m1[NW - 1]);
+                            x0[0] = y0.x; x0[1] = y0.y;
+                            x1[0] = y1.x; x1[1] = y1.y;
+                        } else {
+                            uint32_t l0 = 0u, l1 = 0u;
+#pragma unroll
+                            for (uint32_t j = 0; j < NW; ++j) {
+                                l0 |= m0[j];
+                                l1 |= m1[j];
+                            }
+                            const uint4 y0 = f < 2 ? lds128(a[v][f]) : lds128_if(a[v][f], l0);
+                            const uint4 y1 = f < 2 ? lds128(a[v][f] + wrap[f]) : lds128_if(a[v][f] + wrap[f], l1);
+                            x0[0] = y0.x; x0[1] = y0.y; x0[2] = y0.z; x0[3] = y0.w;
+                            x1[0] = y1.x; x1[1] = y1.y; x1[2] = y1.z; x1[3] = y1.w;
+                        }
+#pragma unroll
+                        for (uint32_t j = 0; j < NW; ++j) {
+                            m0[j] &= x0[j];
+                            m1[j] &= x1[j];
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < NW; ++j) bits[v][j] = m0[j] | m1[j];
+                }
+                if (WT == 1) {
+                    if (i + 1u >= nd) bits[NU - 1][0] = 0u;   // the padding row
+                    const uint32_t has = __ballot_sync(0xffffffffu, (bits[0][0] | bits[NU - 1][0]) != 0u);
+                    if (has)
+                        prod_push<F, PD>(Q, smem, si, lane, qhead, qsize, has, bits[0][0], bits[NU - 1][0],
+                                         d1 | (split[0] << 16) | (split[NU - 1] << 24),
+                                         ews | (wm1[0] & 32u) | (wm1[NU - 1] & 64u));
+                } else {
+#pragma unroll 1
+                    for (uint32_t j = 0; j < NW; j += 2) {   // (one copy of the push and flush)
+                        const uint32_t p0 = j ? bits[0][NW - 2] : bits[0][0], p1 = j ? bits[0][NW - 1] : bits[0][1];
+                        const uint32_t has = __ballot_sync(0xffffffffu, (p0 | p1) != 0u);
+                        if (has)
+                            prod_push<F, PD>(Q, smem, si, lane, qhead, qsize, has, p0, p1, ent_z(d1, split[0]),
+                                             ent_w(ews, wm1[0], j));
                     }
                 }
-#pragma unroll
-                for (uint32_t j = 0; j < NW; ++j) {
-                    const uint32_t cm = shl_c(0xffffffffu, j == 0 ? split[v] : max(split[v], 32u * j) - 32u * j);
-                    bits[v][j] = (m0[j] & ~cm) | (m1[j] & cm);
-                }
-            }
-            if (WT == 1) {
-                if (i + 1u >= nd) bits[NU - 1][0] = 0u;   // the padding row
-                const uint32_t has = __ballot_sync(0xffffffffu, (bits[0][0] | bits[NU - 1][0]) != 0u);
-                if (has)
-                    prod_push<F, PD>(Q, smem, si, lane, step, qhead, qsize, has, bits[0][0], bits[NU - 1][0],
-                                     d1 | (split[0] << 16) | (split[NU - 1] << 24),
-                                     lane | (wm1[0] & 32u) | (wm1[NU - 1] & 64u));
-            } else {
-#pragma unroll
-                for (uint32_t j = 0; j < NW; j += 2) {
-                    const uint32_t p0 = bits[0][j], p1 = bits[0][j + 1 < NW ? j + 1 : j];
-                    const uint32_t has = __ballot_sync(0xffffffffu, (p0 | p1) != 0u);
-                    if (has)
-                        prod_push<F, PD>(Q, smem, si, lane, step, qhead, qsize, has, p0, p1, ent_z(d1, split[0]),
-                                         ent_w(lane, wm1[0], j));
-                }
-            }
             }
         }
-        // the records change with the next strip step: drain the queue
-        while (qsize) prod_flush<F, PD>(Q, smem, si, lane, step, qhead, qsize);
+        // drain the queue after the last step, and where the lanes' records change with the next one
+        if (!rows || step + 1u == nsteps)
+            while (qsize) prod_flush<F, PD>(Q, smem, si, lane, qhead, qsize);
     }
     __syncwarp();
 }
@@ -503,7 +571,7 @@ __device__ __forceinline__ void stage_plan(const EsLaunch& L, EsInst& si, const 
 // Template: F = inner tables, WT = inner-ring words (1, 2; 4 for three and four, rows of 16 bytes;
 // 0 for wider rings).  Work distribution as in es_scan_kernel.
 template <int F, int WT>
-__global__ void __launch_bounds__(ES_LB_THREADS, ES_LB_MINB) es_prod_kernel(const __grid_constant__ EsLaunch L) {
+__global__ void __launch_bounds__(ES_PROD_THREADS, 1) es_prod_kernel(const __grid_constant__ EsLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ EsInst si;
     __shared__ uint32_t s_item;

@@ -77,8 +77,10 @@ def test_tables_match_definition(spec):
         inner = [entry.get(e, []) for e in range(F)]
         q = [int(np.prod([d for _, d in ps])) if ps else 2 for ps in inner]
         proj = [[(d, {x % d for x in filters[f][1]}) for f, d in ps] for ps in inner]
-        starts = [info.tab_base[i] + min(0, info.tab_wrap[i]) for i in range(F)] + [4 * info.tab_words]
-        W, RS = -(-r0 // 32), info.row_bytes // 4
+        starts = [info.tab_base[i] + min(0, info.tab_wrap[i]) for i in range(F)] + [4 * info.tab_words]   # table after table
+        W = -(-r0 // 32)
+        RS = 4 if W == 3 else W
+        assert info.row_bytes == (8 * RS if W <= 1 else 4 * RS)   # one word: both masks in a row
         sh, bsh, band = info.key_shift, info.bucket_shift, info.band
         ssh = 32 - bsh
         mask32 = 0xffffffff
@@ -113,7 +115,7 @@ def test_tables_match_definition(spec):
                         B = (B + corr) % q[i]
                     a = info.tab_base[i] + info.row_bytes * B + int(u32[row + 1 + i])
                     for at in (a, a + info.tab_wrap[i]):
-                        assert starts[i] <= at <= starts[i + 1] - info.row_bytes
+                        assert starts[i] <= at <= starts[i + 1] - 4 * RS
                     lo = tabs[a // 4:a // 4 + RS]
                     hi = tabs[(a + info.tab_wrap[i]) // 4:(a + info.tab_wrap[i]) // 4 + RS]
                     for s in range(RS * 32):
@@ -182,6 +184,34 @@ def test_production_scan_matches_c_oracle(native, spec):
             assert sorted(int(x) for x in ctx.survivors()) == sorted(ws), (F, strip, t, "list")
             ctx.close()
     assert outer >= 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spec", [(300, None), (390, "primary"), (379, "primary")], ids=lambda s: f"k{s[0]}")
+def test_production_windows_of_several_digits(native, spec):
+    """Ranges long enough for the launch to give a lane several ring-2 digits per unit (few warps,
+    so that the strip rule picks 4 to 8), whose queue outlives the steps: against the C oracle."""
+    import es_oracle as O
+    N = native
+    P = _plan(spec)
+
+    class Few:
+        pass
+    few = Few()
+    few.__dict__.update(P.__dict__, rest=P.rest[:6])
+    few.idx_to_n = P.idx_to_n
+    o = 1234567
+    n = (1 << 27) // P.radix[0]
+    want = O.scan_c(few, 1, o_range=(o, o + n))[0]
+    assert len(want) > 1000
+    for F, threads in ((3, 64), (4, 64), (4, 512), (6, 128)):
+        ctx = N.Context(few, N.make_tune(layout=5, mask_filters=F, strip=8, threads=threads, ctas_per_sm=1,
+                                         count_stages=0))
+        ctx.set_block(1)
+        ctx.reset()
+        ctx.launch(o, n)
+        assert sorted(int(x) for x in ctx.survivors()) == want, (F, threads)
+        ctx.close()
 
 
 @pytest.mark.gpu
