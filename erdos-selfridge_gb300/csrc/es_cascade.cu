@@ -161,13 +161,6 @@ double value_of(const std::vector<uint8_t>& proj, uint32_t d, uint32_t g) {
     return -std::log(((double)n / d) * ((double)g / ng));
 }
 
-// The admissible set of a filter (packed bits of q residues) as bytes, projected to d | q.
-void project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_t>& out) {
-    out.assign(d, 0);
-    for (uint32_t from = 0; from < q; from += d)
-        for (uint32_t j = 0; j < d; ++j) out[j] |= (bits[(from + j) >> 5] >> ((from + j) & 31u)) & 1u;
-}
-
 // A possible inner table: up to three parts.
 struct Slot {
     uint32_t n, part[3];
@@ -175,6 +168,12 @@ struct Slot {
 };
 
 }  // namespace
+
+void es_project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_t>& out) {
+    out.assign(d, 0);
+    for (uint32_t from = 0; from < q; from += d)
+        for (uint32_t j = 0; j < d; ++j) out[j] |= (bits[(from + j) >> 5] >> ((from + j) & 31u)) & 1u;
+}
 
 EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes) {
     const uint32_t nf = (uint32_t)P.q.size();
@@ -195,7 +194,7 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
                 full[f] = n ? -std::log((double)n / q) : 64.0;
                 if (full[f] > 1e-3 && 2.0 * d <= budget) parts.push_back(EsPart{f, d, full[f]});
             } else if (whole || 2.0 * d <= budget) {
-                project(bits, q, d, proj);
+                es_project(bits, q, d, proj);
                 const double v = value_of(proj, d, gcd32(d, gM));
                 if (whole) full[f] = v;
                 if (v > 1e-3 && 2.0 * d <= budget) parts.push_back(EsPart{f, d, v});
@@ -391,7 +390,7 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         adm.assign(d, 1);
         for (const EsCascadeEntry::Part& p : e.parts) {
             const uint32_t q = P.q[p.f];
-            project(P.allowed.data() + P.bit_off[p.f], q, p.d, one);
+            es_project(P.allowed.data() + P.bit_off[p.f], q, p.d, one);
             for (uint32_t r = 0, m = 0; r < d; ++r) {
                 adm[r] &= one[m];
                 if (++m == p.d) m = 0;

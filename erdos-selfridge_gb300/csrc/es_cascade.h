@@ -64,6 +64,9 @@ inline uint32_t es_table_rows(uint32_t d, uint32_t corr, bool pair) {
     return 2u * d - 1u + (pair ? 0u : ext);
 }
 
+// The admissible set of a filter (packed bits of q residues) as bytes, projected to d | q.
+void es_project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_t>& out);
+
 // Chooses F inner tables whose rows of row_bytes bytes fit table_bytes in all.
 EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes);
 

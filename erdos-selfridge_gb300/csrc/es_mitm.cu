@@ -11,13 +11,28 @@
 // number of n tested is counted.
 //
 // GB300-first organisation (not the reference's one-thread-per-s1 kernel with two full binary
-// searches): S2 is sorted once on the host and uploaded with a directory over the top bits of
-// its values (bucket b -> first index whose value >= b << shift), sized at about four entries
-// per bucket, so each search is one directory load and a binary search over a handful of entries
-// instead of log2|S2| dependent loads; warps claim chunks of s1 indices from an atomic counter
-// (persistent grid, no waits); s1 is decoded from its index by mixed radix with precomputed
-// 64-bit reciprocals; n mod q uses 32-bit limb weights and one Barrett step against packed bit
-// tables, exactly the exact tail of the block-sieve kernel.
+// searches):
+//  * S2 is sorted once on the host and uploaded with a directory over the top bits of its values
+//    (bucket b -> first index whose value >= b << shift), about one entry per bucket.  A run is
+//    walked from its bucket's first entry: the few entries below M - s1 are passed over, and it
+//    ends at the first n >= B, so no search is needed for either end.
+//  * S1 is swept in value order, tile by tile: with A the sums over the first rings of the large
+//    half (sorted on the host) and b those over the rest, the s1 = a + b of one slice [X, X') of
+//    [0, M) are, for every b, one circular range of A.  Warps claim up to 16 values of b of one slice
+//    from an atomic counter (persistent grid, no waits), search their ranges, a lane per end,
+//    and sweep them, so that the warps at work read one slice of S2 and its directory, which stay
+//    in L2, and a slice comes from memory once.  (In index order every s1 falls anywhere in S2.)
+//  * Runs have a handful of entries and differ from lane to lane, and four of five candidates
+//    fail the first filter: the walk only queues its candidates (per warp, in shared memory), and
+//    a full warp of them at a time goes through the cascade.  Two bit tables in shared memory come
+//    first, each over a product of projections of filters (es_cascade.h), so that one limb-weight
+//    and Barrett reduction tests several filters; the full cascade runs for what is left.
+//
+// What bounds it: instruction issue and the latency of the S2 reads.  With per-lane searches and
+// per-lane cascades the warps ran at 8.6 of 32 lanes: k = 150, bound 3E (1.2e7 s1, 1.7e7
+// candidates) took 930 us of kernel time (7.7e8 warp instructions) and takes 290 (2.1e8); k = 160, whose
+// S2 is twice the L2, 4.2 ms and 1.2 ms.  (More CTAs per SM are slower: 5 of 256 threads 507 against
+// 474 us a scan, 8 895 us.  Their shared memory is taken from the L1 that S2 and the directory use.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +44,7 @@
 #include <vector>
 
 #include "../../include/es_gb300.h"
+#include "es_cascade.h"
 #include "es_internal.h"
 #include "es_scan_kernel.cuh"
 
@@ -53,15 +69,25 @@ int mcuda(cudaError_t e, const char* what) {
     } while (0)
 
 constexpr uint32_t kMitmMaxRings = 32;
-constexpr uint32_t kMitmThreads = 256;
-constexpr uint32_t kMitmChunk = 8;   // s1 indices per lane per claimed chunk
+constexpr uint32_t kMitmThreads = 512;
+constexpr uint32_t kMitmChunk = 16;  // values of b per claimed unit, at most (two lanes each for its range)
+constexpr uint32_t kMitmQueue = 64;  // candidates queued per warp
+constexpr uint32_t kMitmTables = 2;  // merged bit tables ahead of the cascade
+constexpr uint32_t kMitmTableBits = 1u << 18;   // bits of both
+constexpr uint64_t kMitmGroup = 1u << 17;       // rings are grouped while their sums stay within this
+constexpr uint64_t kMitmRange = 64;             // values of A per b and slice, at least
+constexpr uint32_t kMitmSlicesLog2 = 12;        // slices at most
 
 struct MitmParams {
     const uint4* S2;              // sorted small half: {lo.x, lo.y, hi.x, hi.y} per entry
     const uint32_t* dir;          // [2^D + 1] first S2 index with value >= b << shift
-    const uint4* terms1;          // large half's terms, ring after ring
+    const uint4* A;               // large half: sorted sums over its first rings
+    const uint32_t* a_index;      // their indices (mixed radix, first ring fastest)
+    const uint4* sums1;           // sums over the groups of the other rings
+    const uint4* slices;          // [n_slices + 1] slice boundaries, 0 .. M
     const EsFilterC* filt;        // residual filters (q, limb weights, Barrett reciprocal, offset)
     const uint32_t* allowed;      // packed admissible-residue bits of every filter
+    const uint32_t* merged;       // the merged tables' bits
     uint4* out;                   // survivors {n_lo, n_hi} as uint4
     unsigned long long* counters; // [0] survivors, [1] candidates tested, [2] work counter
     uint64_t out_cap;
@@ -69,11 +95,13 @@ struct MitmParams {
     uint64_t s1_begin, s1_end;
     uint64_t M_lo, M_hi, B_lo, B_hi;
     uint32_t shift;               // directory bucket = value >> shift
-    uint32_t n_rings1;
+    uint32_t n_a, n_slices;
+    uint32_t chunk;               // values of b per claimed unit
+    uint32_t n_groups;
     uint32_t n_filters;
-    uint32_t radix1[kMitmMaxRings];
-    uint32_t off1[kMitmMaxRings];
-    unsigned long long magic1[kMitmMaxRings];   // ceil(2^64 / radix) (0 for radix 1)
+    uint32_t merged_words;
+    EsFilterC table[kMitmTables];   // merged moduli; off: word offset in the merged bits
+    EsGroup group[kMitmMaxRings];
 };
 
 __device__ __forceinline__ U4 ld_s2(const uint4* S2, uint64_t i) { return u4(__ldg(S2 + i)); }
@@ -88,91 +116,156 @@ __device__ __forceinline__ uint32_t bucket_of(const U4 v, uint32_t shift) {
     return (uint32_t)r;
 }
 
-// first index u with S2[u] >= v (n2 when none): the directory narrows it to one bucket
-__device__ __forceinline__ uint64_t lower_bound_s2(const MitmParams& P, const U4 v) {
-    const uint32_t b = bucket_of(v, P.shift);
-    uint64_t a = __ldg(P.dir + b), e = __ldg(P.dir + b + 1);
-    while (a < e) {
-        const uint64_t m = (a + e) >> 1;
-        if (lt128(ld_s2(P.S2, m), v)) a = m + 1; else e = m;
-    }
-    return a;
-}
-
-// s1 of index idx: mixed radix over the large half's rings, ring 0 fastest
-__device__ __forceinline__ U4 decode_s1(const MitmParams& P, uint64_t idx, const U4 M) {
+// b of index idx: mixed radix over the groups of rings after A's, the first fastest
+__device__ __forceinline__ U4 decode_b(const MitmParams& P, uint64_t idx, const U4 M) {
     U4 acc{0u, 0u, 0u, 0u};
     uint64_t rem = idx;
-    for (uint32_t j = 0; j < P.n_rings1; ++j) {
-        const uint32_t r = P.radix1[j];
-        uint64_t q;
-        if (r <= 1) {
-            q = rem;
-        } else if ((rem >> 48) == 0) {
-            q = __umul64hi(rem, P.magic1[j]);   // exact for rem < 2^48, r < 2^16
-        } else {
-            q = rem / r;
+    for (uint32_t g = 0; g < P.n_groups; ++g) {
+        const EsGroup G = P.group[g];
+        // floor(rem / size) or one less (magic = floor((2^64 - 1) / size)), then corrected
+        uint64_t q = __umul64hi(rem, G.magic);
+        uint64_t d = rem - q * G.size;
+        if (d >= G.size) {
+            d -= G.size;
+            ++q;
         }
-        const uint64_t d = rem - q * r;
         rem = q;
         uint32_t wm;
-        acc = addmod(acc, u4(__ldg(P.terms1 + P.off1[j] + d)), M, wm);
+        acc = addmod(acc, u4(__ldg(P.sums1 + (G.off + d))), M, wm);
     }
     return acc;
 }
 
+// first index of the sorted A with A[i] >= v (n_a when none)
+__device__ __forceinline__ uint32_t lower_bound_a(const MitmParams& P, const U4 v) {
+    uint32_t a = 0, e = P.n_a;
+    while (a < e) {
+        const uint32_t m = (a + e) >> 1;
+        if (lt128(u4(__ldg(P.A + m)), v)) a = m + 1; else e = m;
+    }
+    return a;
+}
+
+// warp-uniform: the first min(32, size) queued candidates through the cascade; survivors are emitted
+__device__ __forceinline__ void mitm_flush(const MitmParams& P, const uint4* queue, const uint32_t* bits, uint32_t lane,
+                                           uint32_t head, uint32_t size) {
+    __syncwarp();
+    bool ok = lane < size;
+    const U4 n = u4(queue[(head + lane) & (kMitmQueue - 1u)]);   // (stale beyond size: not used)
+    for (uint32_t i = 0; i < kMitmTables; ++i) {
+        const EsFilterC& fc = P.table[i];
+        const uint32_t r = mod128(n, fc);
+        ok = ok && ((bits[fc.off + (r >> 5)] >> (r & 31u)) & 1u);
+        if (!__any_sync(0xffffffffu, ok)) break;
+    }
+    if (ok) {
+        for (uint32_t f = 0; f < P.n_filters && ok; ++f) {
+            const EsFilterC fc = P.filt[f];
+            const uint32_t r = mod128(n, fc);
+            ok = (__ldg(P.allowed + fc.off + (r >> 5)) >> (r & 31u)) & 1u;
+        }
+        if (ok) {
+            const unsigned long long slot = atomicAdd(P.counters + 0, 1ull);
+            if (slot < P.out_cap) P.out[slot] = make_uint4(n.x, n.y, n.z, n.w);
+        }
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(kMitmThreads) es_mitm_kernel(const __grid_constant__ MitmParams P) {
+    extern __shared__ __align__(16) uint32_t bits[];   // the merged tables
+    __shared__ uint4 queues[kMitmThreads / 32][kMitmQueue];
     const uint32_t lane = threadIdx.x & 31u;
+    uint4* queue = queues[threadIdx.x >> 5];
+    for (uint32_t i = threadIdx.x; i < P.merged_words; i += kMitmThreads) bits[i] = __ldg(P.merged + i);
+    for (uint32_t i = lane; i < kMitmQueue; i += 32u) queue[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
     const U4 M{(uint32_t)P.M_lo, (uint32_t)(P.M_lo >> 32), (uint32_t)P.M_hi, (uint32_t)(P.M_hi >> 32)};
     const U4 B{(uint32_t)P.B_lo, (uint32_t)(P.B_lo >> 32), (uint32_t)P.B_hi, (uint32_t)(P.B_hi >> 32)};
-    const uint64_t total = P.s1_end - P.s1_begin;
-    const uint64_t per_claim = 32ull * kMitmChunk;
+    // the values of b that the s1 indices touch; the first and the last may take part of A only
+    const uint64_t b_lo = P.s1_begin / P.n_a, b_hi = (P.s1_end + P.n_a - 1) / P.n_a;
+    const uint64_t chunks = (b_hi - b_lo + P.chunk - 1) / P.chunk;
+    const uint32_t n2 = (uint32_t)P.n2;   // below 2^31
     unsigned long long tested = 0;
+    uint32_t head = 0, size = 0;
     for (;;) {
         unsigned long long c = 0;
         if (lane == 0) c = atomicAdd(P.counters + 2, 1ull);
         c = __shfl_sync(0xffffffffu, c, 0);
-        const uint64_t base = c * per_claim;
-        if (base >= total) break;
-        for (uint32_t it = 0; it < kMitmChunk; ++it) {
-            const uint64_t rel = base + (uint64_t)it * 32u + lane;
-            if (rel >= total) break;
-            const U4 s1 = decode_s1(P, P.s1_begin + rel, M);
-            // lo = (M - s1) mod M, hi = lo + B (mod M, wrapping past M when lo + B >= M)
-            uint32_t br;
-            U4 lo = sub128(M, s1, br);
-            if ((s1.x | s1.y | s1.z | s1.w) == 0u) lo = U4{0u, 0u, 0u, 0u};
-            const U4 hs = add128(lo, B);
-            const U4 hm = sub128(hs, M, br);
-            const bool wrap = br == 0u;            // lo + B >= M
-            const U4 hi = wrap ? hm : hs;
-            const uint64_t i0 = lower_bound_s2(P, lo);
-            const uint64_t j0 = lower_bound_s2(P, hi);
-            // the run: [i0, j0) without a wrap; [i0, n2) then [0, j0) with one
-            uint64_t u = i0;
-            const uint64_t end0 = wrap ? P.n2 : j0;
-            uint64_t todo = (end0 > i0 ? end0 - i0 : 0) + (wrap ? j0 : 0);
-            tested += todo;
-            while (todo) {
-                if (u >= end0 && wrap) u -= end0;   // continue at the front of S2
-                const U4 s2 = ld_s2(P.S2, u);
-                uint32_t wm;
-                const U4 n = addmod(s1, s2, M, wm);
-                bool ok = true;
-                for (uint32_t f = 0; f < P.n_filters && ok; ++f) {
-                    const EsFilterC fc = P.filt[f];
-                    const uint32_t r = mod128(n, fc);
-                    ok = (__ldg(P.allowed + fc.off + (r >> 5)) >> (r & 31u)) & 1u;
+        if (c >= chunks * P.n_slices) break;
+        const uint64_t slice = c / chunks, b0 = b_lo + (c - slice * chunks) * P.chunk;
+        // lanes 2 i and 2 i + 1: b0 + i, and where its range of A starts and ends.  The slice's upper
+        // boundary less b is taken mod M too: an end that is not above the start goes round.
+        const U4 bv = decode_b(P, min(b0 + (lane >> 1), b_hi - 1), M);
+        uint32_t br;
+        U4 v = sub128(u4(__ldg(P.slices + slice + (lane & 1u))), bv, br);
+        if (br) v = add128(v, M);
+        if (((v.x ^ M.x) | (v.y ^ M.y) | (v.z ^ M.z) | (v.w ^ M.w)) == 0u) v = U4{0u, 0u, 0u, 0u};
+        const uint32_t at = lower_bound_a(P, v);
+        const U4 other{__shfl_xor_sync(0xffffffffu, v.x, 1), __shfl_xor_sync(0xffffffffu, v.y, 1),
+                       __shfl_xor_sync(0xffffffffu, v.z, 1), __shfl_xor_sync(0xffffffffu, v.w, 1)};
+        const bool round = (lane & 1u) ? !lt128(other, v) : !lt128(v, other);
+        for (uint32_t i = 0; i < P.chunk && b0 + i < b_hi; ++i) {
+            const uint64_t b = b0 + i;
+            const U4 bs{__shfl_sync(0xffffffffu, bv.x, 2 * i), __shfl_sync(0xffffffffu, bv.y, 2 * i),
+                        __shfl_sync(0xffffffffu, bv.z, 2 * i), __shfl_sync(0xffffffffu, bv.w, 2 * i)};
+            const uint32_t start = __shfl_sync(0xffffffffu, at, 2 * i), stop = __shfl_sync(0xffffffffu, at, 2 * i + 1);
+            const uint32_t count = __shfl_sync(0xffffffffu, round, 2 * i) ? P.n_a - start + stop : stop - start;
+            const bool partial = b * P.n_a < P.s1_begin || (b + 1) * P.n_a > P.s1_end;
+            for (uint32_t from = 0; from < count; from += 32u) {
+                bool active = from + lane < count;
+                uint32_t ia = start + (active ? from + lane : from);
+                if (ia >= P.n_a) ia -= P.n_a;
+                if (partial) {
+                    const uint64_t index = b * P.n_a + __ldg(P.a_index + ia);
+                    active = active && index >= P.s1_begin && index < P.s1_end;
                 }
-                if (ok) {
-                    const unsigned long long slot = atomicAdd(P.counters + 0, 1ull);
-                    if (slot < P.out_cap) P.out[slot] = make_uint4(n.x, n.y, n.z, n.w);
+                uint32_t wa;
+                const U4 s1 = addmod(u4(__ldg(P.A + ia)), bs, M, wa);
+                // The run starts at the first entry >= lo = (M - s1) mod M.  Up to the end of S2,
+                // n = s2 - lo (below 0 for the entries passed over); past it, n = s2 + s1.
+                const bool zero = (s1.x | s1.y | s1.z | s1.w) == 0u;
+                U4 off = sub128(s1, M, br);   // -lo
+                if (zero) off = U4{0u, 0u, 0u, 0u};
+                const U4 lo = sub128(U4{0u, 0u, 0u, 0u}, off, br);
+                uint32_t u = __ldg(P.dir + bucket_of(lo, P.shift));
+                if (u == n2) {
+                    u = 0;
+                    off = s1;
                 }
-                ++u;
-                --todo;
+                uint32_t left = n2;        // entries the run may still take (B = M: all of S2)
+                U4 s2 = ld_s2(P.S2, u);
+                while (__any_sync(0xffffffffu, active)) {
+                    // the next entry, circularly, is on its way while this one is looked at
+                    const U4 n = add128(s2, off);
+                    ++u;
+                    if (u == n2) {
+                        u = 0;
+                        off = s1;
+                    }
+                    if (active) s2 = ld_s2(P.S2, u);
+                    const bool cand = active && lt128(n, B) && left != 0u;   // (a negative n is above B)
+                    left -= cand ? 1u : 0u;
+                    active = cand || (active && (int32_t)n.w < 0);
+                    const uint32_t has = __ballot_sync(0xffffffffu, cand);
+                    if (has) {
+                        if (cand) {
+                            queue[(head + size + __popc(has & ((1u << lane) - 1u))) & (kMitmQueue - 1u)] =
+                                make_uint4(n.x, n.y, n.z, n.w);
+                            ++tested;
+                        }
+                        size += __popc(has);   // at most 31 + 32
+                        if (size >= 32u) {
+                            mitm_flush(P, queue, bits, lane, head, 32u);
+                            head = (head + 32u) & (kMitmQueue - 1u);
+                            size -= 32u;
+                        }
+                    }
+                }
             }
         }
     }
+    if (size) mitm_flush(P, queue, bits, lane, head, size);
     for (uint32_t o = 16; o > 0; o >>= 1) tested += __shfl_down_sync(0xffffffffu, tested, o);
     if (lane == 0 && tested) atomicAdd(P.counters + 1, tested);
 }
@@ -184,9 +277,13 @@ struct es_mitm {
     MitmParams P{};
     uint4* d_S2 = nullptr;
     uint32_t* d_dir = nullptr;
-    uint4* d_terms1 = nullptr;
+    uint4* d_sums1 = nullptr;
     EsFilterC* d_filt = nullptr;
     uint32_t* d_allowed = nullptr;
+    uint32_t* d_merged = nullptr;
+    uint4* d_A = nullptr;
+    uint32_t* d_a_index = nullptr;
+    uint4* d_slices = nullptr;
     uint4* d_out = nullptr;
     unsigned long long* d_cnt = nullptr;
     unsigned long long* h_cnt = nullptr;
@@ -201,9 +298,13 @@ int es_mitm_destroy(es_mitm* m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     cudaFree(m->d_S2);
     cudaFree(m->d_dir);
-    cudaFree(m->d_terms1);
+    cudaFree(m->d_sums1);
     cudaFree(m->d_filt);
     cudaFree(m->d_allowed);
+    cudaFree(m->d_merged);
+    cudaFree(m->d_A);
+    cudaFree(m->d_a_index);
+    cudaFree(m->d_slices);
     cudaFree(m->d_out);
     cudaFree(m->d_cnt);
     if (m->h_cnt) cudaFreeHost(m->h_cnt);
@@ -328,19 +429,28 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     uint32_t bits = 0;   // values < M < 2^bits
     for (u128m x = M - 1; x; x >>= 1) ++bits;
     parallel_sort(S2, bits);
-    // directory over the top bits of values < M: about four entries per bucket
+    // directory over the top bits of values < M: about one entry per bucket
     uint32_t D = 8;
-    while (D < 26 && (1ull << (D + 2)) < n2) ++D;
+    while (D < 28 && (1ull << D) < n2) ++D;
     if (D > bits) D = bits;
     const uint32_t shift = bits - D;
     std::vector<uint32_t> dir((1ull << D) + 1);
     {
-        size_t i = 0;
-        for (uint64_t b = 0; b <= (1ull << D); ++b) {
-            const u128m lim = (u128m)b << shift;
-            while (i < S2.size() && S2[i] < lim) ++i;
-            dir[b] = (uint32_t)i;
-        }
+        // every core fills the buckets of its share of the entries: bucket b holds the first entry i
+        // with value >= b << shift, so entry i fills the buckets above entry i - 1's, up to its own
+        const unsigned T = n2 < (1u << 16) ? 1u : std::max(1u, std::min(64u, std::thread::hardware_concurrency()));
+        auto fill = [&](unsigned t) {
+            const size_t from = n2 * t / T, to = n2 * (t + 1) / T;
+            uint64_t b = from == 0 ? 0 : (uint64_t)(S2[from - 1] >> shift) + 1;
+            for (size_t i = from; i < to; ++i)
+                for (const uint64_t own = (uint64_t)(S2[i] >> shift); b <= own; ++b) dir[b] = (uint32_t)i;
+            if (t + 1 == T)
+                for (; b <= (1ull << D); ++b) dir[b] = (uint32_t)n2;
+        };
+        std::vector<std::thread> th;
+        for (unsigned t = 1; t < T; ++t) th.emplace_back(fill, t);
+        fill(0);
+        for (auto& x : th) x.join();
     }
     // ---- filters ---------------------------------------------------------------------------
     std::vector<EsFilterC> fc(d->n_filters);
@@ -362,27 +472,98 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     if (!m) return mfail(ES_ERR_NOMEM, "host allocation");
     m->n1 = n1;
     m->n2 = n2;
-    std::vector<uint4> h_S2(S2.size()), h_t1(std::max<size_t>(t1.size(), 1));
-    auto pack = [](u128m v) {
-        const uint64_t lo = (uint64_t)v, hi = (uint64_t)(v >> 64);
-        return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
-    };
-    for (size_t i = 0; i < S2.size(); ++i) h_S2[i] = pack(S2[i]);
-    for (size_t i = 0; i < t1.size(); ++i) h_t1[i] = pack(t1[i]);
+    // ---- merged tables: products of projections of filters, tested ahead of the cascade ---------
+    EsHostPlan hp;
+    hp.k = d->k;
+    hp.M = M;
+    hp.q.assign(d->filter_q, d->filter_q + d->n_filters);
+    hp.bit_off.assign(1, 0);
+    for (uint32_t f = 0; f < d->n_filters; ++f) hp.bit_off.push_back(hp.bit_off.back() + (hp.q[f] + 31) / 32);
+    if (d->n_filters) hp.allowed.assign(d->allowed, d->allowed + words);
+    // (rows of one byte, two per residue: kMitmTableBits residues in all)
+    const EsCascade cascade = es_choose_cascade(hp, kMitmTables, 1, true, 2u * kMitmTableBits);
+    std::vector<uint32_t> merged;
+    std::vector<uint8_t> one;
+    for (uint32_t i = 0; i < kMitmTables; ++i) {
+        uint32_t q = 1;
+        for (const EsPart& p : cascade.inner[i]) q *= p.d;
+        if (q == 1) q = 2;   // a fill-in that passes everything
+        const uint32_t off = (uint32_t)merged.size();
+        std::vector<uint8_t> adm(q, 1);
+        for (const EsPart& p : cascade.inner[i]) {
+            es_project(hp.allowed.data() + hp.bit_off[p.f], hp.q[p.f], p.d, one);
+            for (uint32_t r = 0, x = 0; r < q; ++r) {
+                adm[r] &= one[x];
+                if (++x == p.d) x = 0;
+            }
+        }
+        merged.resize(off + (q + 31) / 32, 0u);
+        for (uint32_t r = 0; r < q; ++r) merged[off + (r >> 5)] |= (uint32_t)adm[r] << (r & 31u);
+        m->P.table[i] = es_filter_consts(M, q, off);
+    }
+    // ---- large half: sums over groups of consecutive rings; the first group is A, sorted -----------
+    std::vector<u128m> A(1, 0), sums;
+    for (uint32_t j = 0, o = 0; j < d->n_rings1;) {
+        uint64_t size = 1;
+        const bool first = j == 0;
+        std::vector<u128m> sum(1, 0);
+        do {
+            std::vector<u128m> next;
+            next.reserve(sum.size() * r1[j]);
+            for (uint32_t i = 0; i < r1[j]; ++i)
+                for (const u128m v : sum) {
+                    const u128m x = v + t1[o + i];
+                    next.push_back(x >= M ? x - M : x);
+                }
+            sum.swap(next);
+            size *= r1[j];
+            o += r1[j++];
+        } while (j < d->n_rings1 && size * r1[j] <= kMitmGroup);
+        if (first) {
+            A.swap(sum);
+            continue;
+        }
+        EsGroup& G = m->P.group[m->P.n_groups++];
+        G.size = (uint32_t)size;
+        G.magic = ~0ull / size;
+        G.off = (uint32_t)sums.size();
+        sums.insert(sums.end(), sum.begin(), sum.end());
+    }
+    if (sums.empty()) sums.push_back(0);
+    std::vector<uint32_t> a_index(A.size());
+    for (size_t i = 0; i < A.size(); ++i) a_index[i] = (uint32_t)i;
+    std::sort(a_index.begin(), a_index.end(), [&](uint32_t x, uint32_t y) { return A[x] < A[y]; });
+    std::vector<u128m> a_sorted(A.size());
+    for (size_t i = 0; i < A.size(); ++i) a_sorted[i] = A[a_index[i]];
+    // slices of [0, M): a power of two of them, none so thin that a b's range of A is a few values
+    uint32_t sl = 0;
+    while (sl < kMitmSlicesLog2 && (A.size() >> (sl + 1)) >= kMitmRange) ++sl;
+    std::vector<u128m> slices;
+    for (uint64_t i = 0; i < (1ull << sl); ++i) slices.push_back((M >> sl) * i);
+    slices.push_back(M);
+    static_assert(sizeof(u128m) == sizeof(uint4), "values are uploaded as they are (little endian)");
     cudaError_t ce = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_S2, sizeof(uint4) * h_S2.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_S2, sizeof(uint4) * S2.size());
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_dir, 4ull * dir.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_terms1, sizeof(uint4) * h_t1.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_sums1, sizeof(uint4) * sums.size());
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_filt, sizeof(EsFilterC) * std::max<size_t>(fc.size(), 1));
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_allowed, 4ull * std::max<uint32_t>(words, 1));
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_cnt, 8ull * 4);
     if (ce == cudaSuccess) ce = cudaHostAlloc(&m->h_cnt, 8ull * 4, cudaHostAllocDefault);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_S2, h_S2.data(), sizeof(uint4) * h_S2.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_S2, S2.data(), sizeof(uint4) * S2.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(m->d_dir, dir.data(), 4ull * dir.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_terms1, h_t1.data(), sizeof(uint4) * h_t1.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_sums1, sums.data(), sizeof(uint4) * sums.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess && !fc.empty())
         ce = cudaMemcpy(m->d_filt, fc.data(), sizeof(EsFilterC) * fc.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess && words) ce = cudaMemcpy(m->d_allowed, d->allowed, 4ull * words, cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_A, sizeof(uint4) * A.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_a_index, 4ull * A.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_slices, sizeof(uint4) * slices.size());
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_A, a_sorted.data(), sizeof(uint4) * A.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_a_index, a_index.data(), 4ull * A.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_slices, slices.data(), sizeof(uint4) * slices.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_merged, 4ull * merged.size());
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_merged, merged.data(), 4ull * merged.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemset(m->d_cnt, 0, 8ull * 4);
     if (ce != cudaSuccess) {
         es_mitm_destroy(m);
@@ -391,7 +572,7 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     MitmParams& P = m->P;
     P.S2 = m->d_S2;
     P.dir = m->d_dir;
-    P.terms1 = m->d_terms1;
+    P.sums1 = m->d_sums1;
     P.filt = m->d_filt;
     P.allowed = m->d_allowed;
     P.counters = m->d_cnt;
@@ -399,17 +580,16 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     P.M_lo = d->M_lo;
     P.M_hi = d->M_hi;
     P.shift = shift;
-    P.n_rings1 = d->n_rings1;
     P.n_filters = d->n_filters;
-    uint32_t o = 0;
-    for (uint32_t j = 0; j < d->n_rings1; ++j) {
-        P.radix1[j] = r1[j];
-        P.off1[j] = o;
-        P.magic1[j] = r1[j] > 1 ? (unsigned long long)((~0ull) / r1[j]) + 1ull : 0ull;
-        o += r1[j];
-    }
+    P.merged = m->d_merged;
+    P.A = m->d_A;
+    P.a_index = m->d_a_index;
+    P.n_a = (uint32_t)A.size();
+    P.slices = m->d_slices;
+    P.n_slices = 1u << sl;
+    P.merged_words = (uint32_t)merged.size();
     int occ = 0;
-    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, es_mitm_kernel, kMitmThreads, 0);
+    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, es_mitm_kernel, kMitmThreads, 4ull * merged.size());
     if (ce != cudaSuccess || occ < 1) {
         es_mitm_destroy(m);
         return mcuda(ce == cudaSuccess ? cudaErrorInvalidConfiguration : ce, "MITM occupancy");
@@ -461,11 +641,15 @@ int es_mitm_scan(es_mitm* m, uint64_t B_lo, uint64_t B_hi, uint64_t s1_begin, ui
     P.s1_begin = s1_begin;
     P.s1_end = s1_end;
     ES_MCUDA(cudaMemsetAsync(m->d_cnt + 2, 0, 8, m->stream), "memset");
-    // persistent grid, no more CTAs than there are chunks of s1 indices for their warps
-    const uint64_t claims = (s1_end - s1_begin + 32ull * kMitmChunk - 1) / (32ull * kMitmChunk);
+    // persistent grid, no more CTAs than there are units for their warps
+    const uint64_t nb = (s1_end + P.n_a - 1) / P.n_a - s1_begin / P.n_a;
+    // (several units per warp where there is work for that)
+    const uint64_t warps = (uint64_t)m->grid * (kMitmThreads / 32);
+    P.chunk = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kMitmChunk, nb * P.n_slices / (4 * warps)));
+    const uint64_t claims = (nb + P.chunk - 1) / P.chunk * P.n_slices;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(m->grid, (claims + kMitmThreads / 32 - 1) /
                                                                               (kMitmThreads / 32)));
-    es_mitm_kernel<<<grid, kMitmThreads, 0, m->stream>>>(P);
+    es_mitm_kernel<<<grid, kMitmThreads, 4u * P.merged_words, m->stream>>>(P);
     ES_MCUDA(cudaGetLastError(), "MITM launch");
     return ES_OK;
 }
