@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -113,6 +114,73 @@ struct ProdSet {
     std::vector<EsCascadeEntry> entries;
 };
 
+// Device and pinned memory, stream and events of one batch.  A destroyed batch hands them to the
+// pool of its first context, which keeps one such set for the next batch: a block-ordered search
+// makes a batch per launch, and allocating and freeing these took 200 of its 254 us.
+struct BatchMem {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    unsigned char *dev = nullptr, *pin = nullptr;
+    size_t dev_cap = 0, pin_cap = 0;
+    es_survivor* surv = nullptr;
+    uint64_t surv_cap = 0;
+    BatchMem() = default;
+    BatchMem(const BatchMem&) = delete;
+    BatchMem& operator=(const BatchMem&) = delete;
+    ~BatchMem() {
+        cudaFree(dev);
+        cudaFree(surv);
+        if (pin) cudaFreeHost(pin);
+        if (ev0) cudaEventDestroy(ev0);
+        if (ev1) cudaEventDestroy(ev1);
+        if (stream) cudaStreamDestroy(stream);
+    }
+    cudaError_t need(size_t dev_bytes, size_t pin_bytes, uint64_t cap) {
+        cudaError_t e = cudaSuccess;
+        if (!stream) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess && !ev0) e = cudaEventCreate(&ev0);
+        if (e == cudaSuccess && !ev1) e = cudaEventCreate(&ev1);
+        if (e == cudaSuccess && dev_cap < dev_bytes) {
+            cudaFree(dev);
+            dev = nullptr;
+            dev_cap = 0;
+            e = cudaMalloc(&dev, dev_bytes * 2);
+            if (e == cudaSuccess) dev_cap = dev_bytes * 2;
+        }
+        if (e == cudaSuccess && pin_cap < pin_bytes) {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr;
+            pin_cap = 0;
+            e = cudaHostAlloc(&pin, pin_bytes * 2, cudaHostAllocDefault);
+            if (e == cudaSuccess) pin_cap = pin_bytes * 2;
+        }
+        if (e == cudaSuccess && surv_cap < cap) {
+            cudaFree(surv);
+            surv = nullptr;
+            surv_cap = 0;
+            e = cudaMalloc(&surv, sizeof(es_survivor) * cap);
+            if (e == cudaSuccess) surv_cap = cap;
+        }
+        return e;
+    }
+};
+
+// Shared by a context and the batches made on it, so that either may go first.
+struct BatchPool {
+    static constexpr size_t kKeep = 256u << 20;   // a larger set is freed instead of kept
+    std::mutex mu;
+    std::unique_ptr<BatchMem> idle;
+    std::unique_ptr<BatchMem> take() {
+        std::lock_guard<std::mutex> lock(mu);
+        return std::move(idle);
+    }
+    void give(std::unique_ptr<BatchMem> m) {
+        if (m->dev_cap + m->pin_cap + sizeof(es_survivor) * m->surv_cap > kKeep) return;
+        std::lock_guard<std::mutex> lock(mu);
+        if (!idle) idle = std::move(m);
+    }
+};
+
 }  // namespace
 
 struct es_ctx {
@@ -133,39 +201,46 @@ struct es_ctx {
     es_survivor* d_surv = nullptr;
     uint64_t surv_cap = 0;
     unsigned long long* d_surv_n = nullptr;
-    unsigned long long* d_unit = nullptr;
-    unsigned long long* d_found = nullptr;
+    unsigned long long* d_unit = nullptr;   // work counter, and CTAs done: 0 between launches
+    unsigned long long* d_done = nullptr;
     unsigned long long* d_min = nullptr;
     unsigned long long* h_pin = nullptr;  // pinned scalars for small readbacks
     uint64_t* d_list = nullptr;
     uint64_t list_cap = 0;
-    bool launched = false;
+    // the survivor count read since the last launch or reset, if any
+    bool count_known = false;
+    uint64_t count = 0;
+    std::shared_ptr<BatchPool> pool = std::make_shared<BatchPool>();
 };
 
 struct es_batch {
-    cudaStream_t stream = nullptr;
+    std::shared_ptr<BatchPool> pool;
+    std::unique_ptr<BatchMem> mem;
+    cudaStream_t stream = nullptr;        // mem's
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     es_tune tune{};
     std::vector<es_ctx*> ctxs;
     std::vector<EsItem> h_items;
-    std::vector<uint32_t> nf_of_item;
     uint32_t n_groups = 0;
     EsItem* d_items = nullptr;
+    EsItem* d_items_launch = nullptr;  // the items grouped by width class, as the launches see them
     uint32_t* d_tconst = nullptr;
-    unsigned long long* d_counts = nullptr;
-    uint64_t counts_words = 0;
     std::vector<uint64_t> count_off;
     es_survivor* d_surv = nullptr;
     uint64_t surv_cap = 0;
+    // one block of scalars: the group minima and the survivor count (copied to h_result at the end
+    // of a run), then the launches' unit counters, the items' and the stage counts; then found
+    unsigned long long* d_min = nullptr;         // [n_groups][4]
     unsigned long long* d_surv_n = nullptr;
-    unsigned long long* d_unit = nullptr;
-    unsigned long long* d_found = nullptr;
-    unsigned long long* d_min = nullptr;
-    unsigned long long* d_item_next = nullptr;   // per-item warp-unit counters (several plans)
+    unsigned long long* d_unit = nullptr;        // [n_items], one per launch
+    unsigned long long* d_item_next = nullptr;   // [n_items] next warp-unit (several plans)
+    unsigned long long* d_counts = nullptr;
+    unsigned long long* d_found = nullptr;       // [n_groups]
+    size_t zero_bytes = 0;                       // from d_surv_n up to d_found
+    unsigned long long* h_result = nullptr;      // pinned: minima, count
     uint32_t n_items = 0;
-    EsItem* d_items_launch = nullptr;  // the items grouped by width class, as the launches see them
     // One persistent launch per inner-ring width class (1, 2, 3-4 words, wider): each runs the
     // kernel instance specialised for its width instead of one generic instance for all.
     struct Sub {
@@ -295,14 +370,36 @@ es_tune prod_shape(es_tune t) {
     return t;
 }
 
-// Ring-1 cycles per lane and warp-unit of a production launch of `steps` warp-wide cycles, at most
-// the caller's.  A unit costs about half a cycle to set up, and the launch ends when its last unit
-// does: with W steps per resident warp, W (1 + 0.5 / s) + 0.6 s is least at s = sqrt(0.8 W).
-// Measured (k = 300): 2^30 positions 126 us at 8, 118 at 4; 2^34 positions 1485 at 8, 1563 at 4;
-// k = 384, 2^28 positions 189 us at 8, 74 at 2.
-uint32_t prod_strip(uint64_t steps, const es_tune& t) {
-    const double per_warp = (double)steps / ((double)g_dev.sms * (t.threads / 32u));
-    return std::min(t.strip, std::max(1u, (uint32_t)(std::sqrt(0.8 * per_warp) + 0.5)));
+// Longest unit, in ring-1 cycles per lane, of a plan at `strip` (windows of ring-2 digits are balanced).
+uint32_t longest_of(const EsInst& I, uint32_t strip) {
+    if (I.r2 <= 1) return strip;
+    const uint32_t J = (I.r2 + strip - 1) / strip;
+    return (I.r2 + J - 1) / J;
+}
+
+// Ring-1 cycles per lane and warp-unit of a launch of `steps` warp-wide cycles, at most the caller's;
+// units(s) is the number of units at s, longest(s) the longest of them.  A unit costs about half a
+// cycle to set up, so long ones are better; but a warp takes as long for a unit when the SM is half
+// empty as when it is full, so a launch of few waves takes whole ones.  Measured (3040 resident
+// warps): k = 300, 2^30 positions 103 us in 1.9 waves of 7 cycles, 117 in 4.4 of 3, 141 in 13.3 of 1;
+// 2^34 positions 1470 at 7, 1723 at 2; k = 384, 2^28 positions 67 us in 1.5 waves of 1, 127 in 0.2 of 8.
+template <class Units, class Longest>
+uint32_t launch_strip(uint64_t steps, const es_tune& t, const Units& units, const Longest& longest) {
+    const double warps = (double)g_dev.sms * (t.threads / 32u);
+    uint32_t best = 1;
+    double least = 0.0;
+    for (uint32_t s = 1; s <= std::min<uint32_t>(t.strip, 64); ++s) {
+        const uint64_t n = units(s);
+        if (n == 0) break;
+        const double waves = n / warps;
+        const double cost = (waves < 8.0 ? std::ceil(waves) : waves + 0.5) *
+                            ((waves < 4.0 ? longest(s) : (double)steps / n) + 0.5);
+        if (s == 1 || cost < least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
 }
 
 // Warp-wide ring-1 cycles of [cb, ce) (rows of 32 lanes x ring-2 digits).
@@ -310,6 +407,13 @@ uint64_t steps_of(const EsInst& I, uint64_t cb, uint64_t ce) {
     if (ce <= cb) return 0;
     if (I.r2 <= 1) return (ce - cb + 31) / 32;
     return ((ce + I.r2 - 1) / I.r2 - cb / I.r2 + 31) / 32 * I.r2;
+}
+
+void launch_tables(EsLaunch& L, const EsInst& I) {
+    L.small = I.small;
+    L.tabs = I.masks;
+    L.small_bytes = I.small_bytes;
+    L.tab_words = I.tab_words;
 }
 
 // Inner tables of a production launch.
@@ -640,12 +744,10 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     if (ce == cudaSuccess) ce = cudaMemset(c->d_counts, 0, 8ull * std::max<uint32_t>(nf, 1));
     if (ce == cudaSuccess) ce = cudaMemset(c->d_surv_n, 0, 8ull * 8);
     if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "context setup"); }
-    // d_surv_n block: [0] survivor count, [1] unit counter, [2] group found, [3..6] group min
+    // d_surv_n block: [0] survivor count, [1] unit counter, [2] CTAs done, [3..6] group min
     c->d_unit = c->d_surv_n + 1;
-    c->d_found = c->d_surv_n + 2;
+    c->d_done = c->d_surv_n + 2;
     c->d_min = c->d_surv_n + 3;
-    ce = cudaMemset(c->d_found, 0xff, 8);
-    if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "context setup"); }
     e = es_set_capacity(c, 1u << 20);
     if (e) { es_ctx_destroy(c); return e; }
     *out = c;
@@ -753,8 +855,8 @@ int es_set_block(es_ctx* c, const uint32_t* tconst, uint32_t n, uint64_t t) {
 
 int es_reset_survivors(es_ctx* c) {
     if (!c) return fail(ES_ERR_ARG, "null context");
+    c->count_known = false;
     ES_CUDA(cudaMemsetAsync(c->d_surv_n, 0, 8, c->stream), "memset");
-    ES_CUDA(cudaMemsetAsync(c->d_found, 0xff, 8, c->stream), "memset");
     return ES_OK;
 }
 
@@ -791,7 +893,12 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
         n_work = cycles_of(I, ob, oe, &it.c_begin);
         it.c_end = it.c_begin + n_work;
     }
-    if (prod) tn.strip = prod_strip(d_list ? (n_work + 31) / 32 : steps_of(I, it.c_begin, it.c_end), tn);
+    tn.strip = launch_strip(
+        d_list ? (n_work + 31) / 32 : steps_of(I, it.c_begin, it.c_end), tn,
+        [&](uint32_t w) {
+            return d_list ? (n_work + 32ull * w - 1) / (32ull * w) : units_of(I, it.c_begin, it.c_end, w);
+        },
+        [&](uint32_t w) { return d_list ? w : longest_of(I, w); });
     const uint64_t per_unit = 32ull * tn.strip;
     it.unit_begin = 0;
     it.n_units = d_list ? (n_work + per_unit - 1) / per_unit : units_of(I, it.c_begin, it.c_end, tn.strip);
@@ -812,6 +919,7 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
     L.nf_max = std::max<uint32_t>(I.n_filters, 1);
     L.direct = 1;
     L.unit_counter = c->d_unit;
+    L.ctas_done = c->d_done;
     L.surv = c->d_surv;
     L.surv_n = c->d_surv_n;
     L.surv_cap = c->surv_cap;
@@ -820,6 +928,7 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
     L.cnt_off = sp.cnt_off;
     L.queue_off = sp.queue_off;
     L.stage_off = sp.stage_off;
+    launch_tables(L, I);
     if (prod)
         prod_tconst(c->prod[PF], c->tconst, L.tconst0);
     else
@@ -827,10 +936,9 @@ static int ctx_launch(es_ctx* c, uint64_t ob, uint64_t oe, const uint64_t* d_lis
     if (it.n_units == 0) return ES_OK;
     int grid = 0;
     if (int e = grid_for(layout, tn.count_stages, I.W, F, tn, sp.bytes, it.n_units, &grid)) return e;
-    ES_CUDA(cudaMemsetAsync(c->d_unit, 0, 8, c->stream), "memset");
+    c->count_known = false;
     int e = es_launch_scan(L, (int)layout, (int)tn.count_stages, I.W, grid, c->stream);
     if (e) return cuda_fail((cudaError_t)e, "scan launch");
-    c->launched = true;
     return ES_OK;
 }
 
@@ -865,9 +973,13 @@ int es_sync(es_ctx* c) {
 
 int es_survivor_count(es_ctx* c, uint64_t* n) {
     if (!c || !n) return fail(ES_ERR_ARG, "null argument");
-    ES_CUDA(cudaMemcpyAsync(c->h_pin, c->d_surv_n, 8, cudaMemcpyDeviceToHost, c->stream), "copy");
-    ES_CUDA(cudaStreamSynchronize(c->stream), "kernel execution");
-    *n = c->h_pin[0];
+    if (!c->count_known) {
+        ES_CUDA(cudaMemcpyAsync(c->h_pin, c->d_surv_n, 8, cudaMemcpyDeviceToHost, c->stream), "copy");
+        ES_CUDA(cudaStreamSynchronize(c->stream), "kernel execution");
+        c->count = c->h_pin[0];
+        c->count_known = true;
+    }
+    *n = c->count;
     return ES_OK;
 }
 
@@ -942,15 +1054,7 @@ int es_batch_destroy(es_batch* b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
-    cudaFree(b->d_items);
-    cudaFree(b->d_items_launch);
-    cudaFree(b->d_tconst);
-    cudaFree(b->d_counts);
-    cudaFree(b->d_surv);
-    cudaFree(b->d_surv_n);
-    if (b->ev0) cudaEventDestroy(b->ev0);
-    if (b->ev1) cudaEventDestroy(b->ev1);
-    if (b->stream) cudaStreamDestroy(b->stream);
+    if (b->mem && b->pool) b->pool->give(std::move(b->mem));
     delete b;
     return ES_OK;
 }
@@ -1019,7 +1123,6 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         max_group = std::max<uint32_t>(max_group, s.group);
     }
     b->n_groups = max_group + 1;
-    b->counts_words = cwords;
     // launch order: items grouped by width class (stable), one launch per class; counting launches
     // with ES_LAYOUT_AUTO split a one- or two-word class further into the plans whose inner-stage
     // tables fit shared memory (staged) and the rest
@@ -1040,23 +1143,36 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     std::vector<uint32_t> order(n_items);
     for (uint32_t i = 0; i < n_items; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
-    cudaError_t ce = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaEventCreate(&b->ev0);
-    if (ce == cudaSuccess) ce = cudaEventCreate(&b->ev1);
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_items, sizeof(EsItem) * n_items);
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_items_launch, sizeof(EsItem) * n_items);
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_tconst, 4ull * std::max<size_t>(h_tc.size(), 4));
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_counts, 8ull * cwords);
-    // scalars: [0] survivor count, [1..n_items] unit counters of the launches, then group_found[G],
-    // group_min[4G], item_next[n_items]
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_surv_n, 8ull * (1 + 5ull * b->n_groups + 2ull * n_items));
+    // device block: items (caller order, launch order), constants (uploaded in one copy), scalars
+    const size_t items_bytes = es_align_up(sizeof(EsItem) * n_items, 16);
+    const size_t upload = 2 * items_bytes + es_align_up(4ull * h_tc.size(), 16);
+    const size_t n_scalars = 4ull * b->n_groups + 1 + 2ull * n_items + cwords + b->n_groups;
+    b->pool = ctxs[0]->pool;
+    b->mem = b->pool->take();
+    if (!b->mem) b->mem.reset(new (std::nothrow) BatchMem());
+    if (!b->mem) { es_batch_destroy(b); return fail(ES_ERR_NOMEM, "host allocation"); }
     b->surv_cap = ctxs[0]->surv_cap;
-    if (ce == cudaSuccess) ce = cudaMalloc(&b->d_surv, sizeof(es_survivor) * b->surv_cap);
-    if (ce != cudaSuccess) { es_batch_destroy(b); return cuda_fail(ce, "batch setup"); }
+    cudaError_t ce = b->mem->need(upload + 8 * n_scalars, upload + 8 * (4ull * b->n_groups + 1), b->surv_cap);
+    if (ce != cudaSuccess) {
+        b->mem.reset();
+        es_batch_destroy(b);
+        return cuda_fail(ce, "batch setup");
+    }
+    b->stream = b->mem->stream;
+    b->ev0 = b->mem->ev0;
+    b->ev1 = b->mem->ev1;
+    b->d_surv = b->mem->surv;
+    b->d_items = reinterpret_cast<EsItem*>(b->mem->dev);
+    b->d_items_launch = reinterpret_cast<EsItem*>(b->mem->dev + items_bytes);
+    b->d_tconst = reinterpret_cast<uint32_t*>(b->mem->dev + 2 * items_bytes);
+    b->d_min = reinterpret_cast<unsigned long long*>(b->mem->dev + upload);
+    b->d_surv_n = b->d_min + 4ull * b->n_groups;
     b->d_unit = b->d_surv_n + 1;
-    b->d_found = b->d_surv_n + 1 + n_items;
-    b->d_min = b->d_found + b->n_groups;
-    b->d_item_next = b->d_min + 4ull * b->n_groups;
+    b->d_item_next = b->d_unit + n_items;
+    b->d_counts = b->d_item_next + n_items;
+    b->d_found = b->d_counts + cwords;
+    b->zero_bytes = 8ull * (size_t)(b->d_found - b->d_surv_n);
+    b->h_result = reinterpret_cast<unsigned long long*>(b->mem->pin + upload);
     b->n_items = n_items;
     for (uint32_t i = 0; i < n_items; ++i) {
         EsItem& it = b->h_items[i];
@@ -1097,7 +1213,20 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
             steps += steps_of(I, it.c_begin, it.c_end);
             ++end;
         }
-        if (prod) shape.strip = prod_strip(steps, shape);
+        auto geo_of = [&](uint32_t j) -> const EsInst& { return ctxs[items[order[j]].ctx_index]->geo; };
+        shape.strip = launch_strip(
+            steps, shape,
+            [&](uint32_t w) {
+                uint64_t n = 0;
+                for (uint32_t j = pos; j < end; ++j)
+                    n += units_of(geo_of(j), b->h_items[order[j]].c_begin, b->h_items[order[j]].c_end, w);
+                return n;
+            },
+            [&](uint32_t w) {
+                uint32_t m = 0;
+                for (uint32_t j = pos; j < end; ++j) m = std::max(m, longest_of(geo_of(j), w));
+                return m;
+            });
         for (uint32_t j = pos; j < end; ++j) {
             EsItem& it = launch_items[j];
             it = b->h_items[order[j]];
@@ -1137,6 +1266,7 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         L.cnt_off = sp.cnt_off;
         L.queue_off = sp.queue_off;
         L.stage_off = sp.stage_off;
+        if (one_ctx) launch_tables(L, tables(ctxs[first_ctx]).h);
         if (int e = grid_for(sub.layout, tune.count_stages, sub.words, F, shape, sp.bytes,
                              std::max<uint64_t>(units, 1), &sub.grid)) {
             es_batch_destroy(b);
@@ -1145,22 +1275,19 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         b->subs.push_back(sub);
         pos = end;
     }
-    ce = cudaMemcpy(b->d_items, b->h_items.data(), sizeof(EsItem) * n_items, cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess)
-        ce = cudaMemcpy(b->d_items_launch, launch_items.data(), sizeof(EsItem) * n_items, cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess && !h_tc.empty())
-        ce = cudaMemcpy(b->d_tconst, h_tc.data(), 4ull * h_tc.size(), cudaMemcpyHostToDevice);
+    unsigned char* stage = b->mem->pin;   // not written again before this batch's memory is reused
+    memcpy(stage, b->h_items.data(), sizeof(EsItem) * n_items);
+    memcpy(stage + items_bytes, launch_items.data(), sizeof(EsItem) * n_items);
+    if (!h_tc.empty()) memcpy(stage + 2 * items_bytes, h_tc.data(), 4ull * h_tc.size());
+    ce = cudaMemcpyAsync(b->mem->dev, stage, upload, cudaMemcpyHostToDevice, b->stream);
     if (ce != cudaSuccess) { es_batch_destroy(b); return cuda_fail(ce, "batch upload"); }
     *out = b;
     return ES_OK;
 }
 
 static int batch_enqueue(es_batch* b) {
-    ES_CUDA(cudaMemsetAsync(b->d_surv_n, 0, 8ull * (1 + b->n_items), b->stream), "memset");   // count + unit counters
+    ES_CUDA(cudaMemsetAsync(b->d_surv_n, 0, b->zero_bytes, b->stream), "memset");
     ES_CUDA(cudaMemsetAsync(b->d_found, 0xff, 8ull * b->n_groups, b->stream), "memset");
-    ES_CUDA(cudaMemsetAsync(b->d_item_next, 0, 8ull * b->n_items, b->stream), "memset");
-    if (b->counts_words)
-        ES_CUDA(cudaMemsetAsync(b->d_counts, 0, 8ull * b->counts_words, b->stream), "memset");
     for (const es_batch::Sub& sub : b->subs) {
         if (!sub.L.total_units) continue;
         int e = es_launch_scan(sub.L, (int)sub.layout, (int)b->tune.count_stages, sub.words, sub.grid, b->stream);
@@ -1170,6 +1297,8 @@ static int batch_enqueue(es_batch* b) {
     int e = es_launch_min(b->d_surv, b->d_surv_n, b->surv_cap, b->d_items, b->n_groups, b->d_found,
                           b->d_min, b->stream);
     if (e) return cuda_fail((cudaError_t)e, "min launch");
+    ES_CUDA(cudaMemcpyAsync(b->h_result, b->d_min, 8ull * (4ull * b->n_groups + 1), cudaMemcpyDeviceToHost, b->stream),
+            "copy");
     return ES_OK;
 }
 
@@ -1213,8 +1342,7 @@ int es_batch_group_min(es_batch* b, uint32_t group, int* found, uint64_t* t, uin
     if (group >= b->n_groups) return fail(ES_ERR_ARG, "group out of range");
     if (!b->ran) return fail(ES_ERR_STATE, "batch has not run");
     ES_CUDA(cudaStreamSynchronize(b->stream), "kernel execution");
-    unsigned long long v[4];
-    ES_CUDA(cudaMemcpy(v, b->d_min + 4ull * group, 32, cudaMemcpyDeviceToHost), "copy");
+    const unsigned long long* v = b->h_result + 4ull * group;
     *found = (int)v[0];
     if (t) *t = v[1];
     if (s_lo) *s_lo = v[2];
@@ -1242,8 +1370,7 @@ int es_batch_survivors(es_batch* b, es_survivor* out, uint64_t cap, uint64_t* n)
     if (!b || !n) return fail(ES_ERR_ARG, "null argument");
     if (!b->ran) return fail(ES_ERR_STATE, "batch has not run");
     ES_CUDA(cudaStreamSynchronize(b->stream), "kernel execution");
-    unsigned long long cnt = 0;
-    ES_CUDA(cudaMemcpy(&cnt, b->d_surv_n, 8, cudaMemcpyDeviceToHost), "copy");
+    const unsigned long long cnt = b->h_result[4ull * b->n_groups];
     *n = cnt;
     if (cnt > b->surv_cap) return fail(ES_ERR_OVERFLOW, "survivor buffer overflow");
     if (cnt > cap) return fail(ES_ERR_OVERFLOW, "output buffer smaller than the survivor count");
@@ -1371,7 +1498,9 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
     const SmemPlan sp = plan_smem((uint32_t)I.small_bytes, nf, tn, prod ? I.tab_words : 0u);
     uint64_t cbeg = 0;
     const uint64_t ncyc = cycles_of(I, 0, I.n_outer, &cbeg);
-    if (prod) tn.strip = prod_strip(steps_of(I, cbeg, cbeg + ncyc) * n_blocks, tn);
+    tn.strip = launch_strip(steps_of(I, cbeg, cbeg + ncyc) * n_blocks, tn,
+                            [&](uint32_t w) { return units_of(I, cbeg, cbeg + ncyc, w) * n_blocks; },
+                            [&](uint32_t w) { return longest_of(I, w); });
     const uint64_t nu = units_of(I, cbeg, cbeg + ncyc, tn.strip);
     for (uint32_t i = 0; i < n_blocks; ++i) {
         const uint64_t t = t0 + i;
@@ -1423,6 +1552,7 @@ extern "C" int es_search_blocks_static(const es_ctx* c, uint64_t t0, uint32_t n_
     L.cnt_off = sp.cnt_off;
     L.queue_off = sp.queue_off;
     L.stage_off = sp.stage_off;
+    launch_tables(L, I);
     if (L.total_units) {
         int grid = 0;
         if (int e = grid_for(layout, 0, I.W, F, tn, sp.bytes, L.total_units, &grid)) return e;

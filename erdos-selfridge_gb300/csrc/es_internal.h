@@ -127,6 +127,7 @@ struct EsLaunch {
     uint32_t nf_max;               // largest filter count among the launch's plans
     uint32_t direct;               // 1: every item uses one plan (no CTA barriers after staging)
     unsigned long long* unit_counter;     // single-plan launches: next warp-unit
+    unsigned long long* ctas_done;        // or null: the launch's last CTA sets both counters back to 0
     unsigned long long* item_next;        // several plans: next warp-unit of each item
     struct es_survivor* surv;
     unsigned long long* surv_n;
@@ -136,6 +137,10 @@ struct EsLaunch {
     uint32_t cnt_off;                 // byte offset of the per-warp tail-stage counters in smem
     uint32_t queue_off;               // byte offset of the per-warp survivor queues in smem
     uint32_t stage_off;               // byte offset of the staged tables (ES_LAYOUT_SMEM, _SMEM_PAIR)
+    // production launches of one plan: its tables, so that staging them need not wait for the header
+    const unsigned char* small;
+    const uint32_t* tabs;
+    uint32_t small_bytes, tab_words;
     // single-plan launches carry their one item and block constants by value
     EsItem item0;
     uint32_t tconst0[ES_MAX_ENTRIES];

@@ -562,9 +562,14 @@ __device__ __forceinline__ void stage_words(unsigned char* dst, const void* src,
 
 __device__ __forceinline__ void stage_plan(const EsLaunch& L, EsInst& si, const EsInst* inst, unsigned char* smem) {
     load_inst(si, inst);
-    __syncthreads();
-    stage_words(smem, si.small, si.small_bytes >> 2);
-    stage_words(smem + L.stage_off, si.masks, si.tab_words);
+    if (L.small) {   // the launch has one plan and brings its table addresses
+        stage_words(smem, L.small, L.small_bytes >> 2);
+        stage_words(smem + L.stage_off, L.tabs, L.tab_words);
+    } else {
+        __syncthreads();
+        stage_words(smem, si.small, si.small_bytes >> 2);
+        stage_words(smem + L.stage_off, si.masks, si.tab_words);
+    }
     __syncthreads();
 }
 
@@ -583,14 +588,18 @@ __global__ void __launch_bounds__(ES_PROD_THREADS, 1) es_prod_kernel(const __gri
     const unsigned long long total = L.total_units;
 
     if (L.direct) {
-        // one plan: stage it, then warps claim warp-units on their own
+        // one plan: stage it, then warps claim warp-units on their own (the first claim is on its way
+        // meanwhile).  With no more units than warps each warp has one at most and claims once.
+        unsigned long long w = 0;
+        if (lane == 0) w = atomicAdd(L.unit_counter, 1ull);
+        const bool single = total <= (unsigned long long)gridDim.x * (blockDim.x >> 5);
         stage_plan(L, si, items[0].inst, smem);
-        for (;;) {
-            unsigned long long w = 0;
+        for (bool first = true;; first = false) {
+            if (!first && single) break;
             uint32_t it_id = 0;
             int skip = 0;
             if (lane == 0) {
-                w = atomicAdd(L.unit_counter, 1ull);
+                if (!first) w = atomicAdd(L.unit_counter, 1ull);
                 if (w < total) {
                     uint32_t lo = 0, hi = L.n_items;
                     while (hi - lo > 1) {
@@ -612,6 +621,7 @@ __global__ void __launch_bounds__(ES_PROD_THREADS, 1) es_prod_kernel(const __gri
             if (skip) continue;
             prod_unit<F, WT>(L, si, smem, Q, lane, w, items[it_id]);
         }
+        leave(L);
         return;
     }
 

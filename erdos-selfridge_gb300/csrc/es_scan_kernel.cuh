@@ -805,6 +805,20 @@ __device__ __forceinline__ void scan_unit(const EsLaunch& L, const EsInst& si, u
     }
 }
 
+// The end of a single-plan launch: the last CTA sets its counters back to 0 for the next launch on
+// the stream (no memset between launches).
+__device__ __forceinline__ void leave(const EsLaunch& L) {
+    if (!L.ctas_done) return;
+    __syncthreads();   // every warp of the CTA has made its last claim
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(L.ctas_done, 1ull) + 1ull == gridDim.x) {
+            *L.unit_counter = 0ull;
+            *L.ctas_done = 0ull;
+        }
+    }
+}
+
 // Work distribution.  A warp-unit is 32 lanes x up to `strip` ring-1 cycles (or list entries)
 // of one item (lanes on consecutive ring-2 rows, see scan_unit).  Single-plan launches: the CTA stages the plan's tables once, then each
 // warp claims warp-units from the global counter on its own -- no CTA barrier after staging.
@@ -871,6 +885,7 @@ __global__ void __launch_bounds__(ES_LB_THREADS, ES_LB_MINB) es_scan_kernel(cons
             if (skip) continue;
             scan_unit<F, LAYOUT, COUNT, WT>(L, si, smem, Q, wcnt, wcnt_saddr, lane, w, items[it_id], it_id);
         }
+        leave(L);
         return;
     }
 

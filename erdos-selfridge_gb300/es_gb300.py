@@ -103,6 +103,28 @@ def block_from_tconst(rest_q, rest_Mmodq, tc) -> int:
     return t_mod
 
 
+class _BlockRecovery:
+    """block_from_tconst with the CRT coefficients of one plan worked out once."""
+
+    def __init__(self, rest_q, rest_Mmodq):
+        self.steps, mod = [], 1     # (filter, q, inverse of M mod q, inverse of the modulus so far, that modulus)
+        for j, q in enumerate(rest_q):
+            m = rest_Mmodq[j]
+            if math.gcd(m, q) != 1 or math.gcd(mod, q) != 1:
+                continue
+            self.steps.append((j, q, pow(m, -1, q), pow(mod, -1, q), mod))
+            mod *= q
+            if mod > (1 << 64):
+                break
+        self.exact = mod > (1 << 64)    # t mod `mod` is every 64-bit t itself
+
+    def __call__(self, tc) -> int:
+        t = 0
+        for j, q, inv_m, inv_mod, mod in self.steps:
+            t += mod * (((int(tc[j]) * inv_m) % q - t) * inv_mod % q)
+        return t
+
+
 def verdict(plan, t: int, surv) -> tuple[list[int], list[int], list[int]]:
     """Host re-verification of a block's kernel survivors (sieve/gpu_sieve_v9.py:551-557):
     (all survivors as n, sorted; the good ones; those with n > k+1 that the exact test rejects)."""
@@ -212,16 +234,23 @@ class GpuSieve:
         self.out_n = _OutN(self)
         self.out = _Out(self)
         self._block = 0
+        self._recover = _BlockRecovery(self.rest_q, self.rest_Mmodq)
         self._set_tconst(self.tconst_h)
 
     # ---------------------------------------------------------------- device plumbing
     def _block_from_tconst(self, tc: np.ndarray) -> int:
-        return block_from_tconst(self.rest_q, self.rest_Mmodq, tc)
+        return self._recover(tc)
 
-    def _set_tconst(self, tc: np.ndarray) -> None:
+    def _set_tconst(self, tc: np.ndarray, t: int | None = None) -> None:
+        """Block constants to the engine; t: their block, when the caller made them from it.  Constants
+        that determine t only modulo a product below 2^64 are first compared with the last block's."""
         tc = np.ascontiguousarray(tc[:max(self.nrest, 1)], dtype=np.uint32)
-        t = self._block if np.array_equal(tc[:self.nrest], N.tconst_for(self.plan, self._block)[:self.nrest]) \
-            else self._block_from_tconst(tc)
+        if t is None:
+            if not self._recover.exact and np.array_equal(tc[:self.nrest],
+                                                          N.tconst_for(self.plan, self._block)[:self.nrest]):
+                t = self._block
+            else:
+                t = self._block_from_tconst(tc)
         self.ctx.set_block(t, tc[:self.nrest] if self.nrest else np.zeros(0, dtype=np.uint32))
 
     def _launch(self, ostart: int, ocount: int) -> None:
@@ -234,7 +263,7 @@ class GpuSieve:
         """Every position of block t; one device sync per block (sieve/gpu_sieve_v9.py:508-525)."""
         self._block = int(t)
         self.tconst_h[:] = N.tconst_for(self.plan, t)[:self.tconst_h.size]
-        self.tconst.set(self.tconst_h)
+        self._set_tconst(self.tconst_h, self._block)
         self.out_n.fill(0)
         ostart = 0
         while ostart < self.R_outer:

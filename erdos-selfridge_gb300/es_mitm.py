@@ -219,6 +219,10 @@ class MitmEngine:
         self.n1, self.n2 = n1.value, n2.value
         self.capacity = capacity
         N.check(L.es_mitm_set_capacity(h, capacity))
+        # survivors as the library returns them, kept from scan to scan (touching new buffers of the full
+        # capacity cost 200 us a scan)
+        self._lo = np.empty(capacity, dtype=np.uint64)
+        self._hi = np.empty(capacity, dtype=np.uint64)
 
     def close(self):
         if getattr(self, "h", None):
@@ -239,8 +243,7 @@ class MitmEngine:
         s1_end = self.n1 if s1_end is None else s1_end
         N.check(L.es_mitm_reset(self.h))
         N.check(L.es_mitm_scan(self.h, B & mask, B >> 64, s1_begin, s1_end))
-        lo = np.zeros(self.capacity, dtype=np.uint64)
-        hi = np.zeros(self.capacity, dtype=np.uint64)
+        lo, hi = self._lo, self._hi
         ns, nc = C.c_uint64(), C.c_uint64()
         N.check(L.es_mitm_results(self.h, lo.ctypes.data_as(C.POINTER(C.c_uint64)),
                                   hi.ctypes.data_as(C.POINTER(C.c_uint64)), self.capacity,

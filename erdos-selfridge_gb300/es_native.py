@@ -404,10 +404,16 @@ class Batch:
 
     def survivors(self) -> np.ndarray:
         cap = self.ctxs[0].capacity
-        out = np.zeros(cap, dtype=SURVIVOR_DTYPE)
         got = C.c_uint64()
-        check(lib().es_batch_survivors(self.h, out.ctypes.data_as(C.POINTER(Survivor)), cap, C.byref(got)))
-        return out[:got.value]
+        room = min(cap, 1024)   # most batches have few; a buffer of the full capacity is tens of megabytes
+        while True:
+            out = np.zeros(room, dtype=SURVIVOR_DTYPE)
+            rc = lib().es_batch_survivors(self.h, out.ctypes.data_as(C.POINTER(Survivor)), room, C.byref(got))
+            if rc == ES_ERR_OVERFLOW and room < got.value <= cap:
+                room = got.value
+                continue
+            check(rc)
+            return out[:got.value]
 
 
 def int_peak(mixed: bool = False) -> tuple[float, float]:
