@@ -675,10 +675,11 @@ static int upload_prod(es_ctx* c, uint32_t F, EsProdImage& img) {
 }
 
 // Candidates per warp-wide ring-1 digit above which a plan's own launches take one more inner table
-// than asked for: the queue's passes then cost more than the table.  k = 260 (4.2 candidates with four
-// tables), 2^32 positions: 498 us, with five 447; k = 378 (5.2): 1439 and 1336; k = 379 (3.0): 1842 and
-// 1857; k = 390 (1.1): 1603 and 1653.
-constexpr double kMoreTables = 3.5;
+// than asked for: the queue's passes then cost more than the table, which few lanes read.  Four and
+// five tables, 2^34 positions: k = 384 (1.8 candidates with four) 1552 and 1494 us, k = 300 (0.6) 1330
+// and 1276, k = 390 (1.1) 1417 and 1415, k = 379 (2.9) 1658 and 1679; 2^30 positions: k = 200 (0.2) 179
+// and 184.
+constexpr double kMoreTables = 0.5;
 
 // Builds the table sets that launches of this shape read, unless they are there already: the
 // plan's own launches (own), or those of a batch of several plans, which share a table count.
@@ -774,8 +775,8 @@ int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes
     info->n_entries = I.n_filters;
     info->row_bytes = I.row_bytes;
     info->key_shift = I.sh;
-    info->bucket_shift = I.bsh;
-    info->band = I.band;
+    info->key_up = I.lsh;
+    info->bucket_log2 = ES_PBUCKET_LOG2;
     info->o_row1 = I.o_R1;
     info->row1_bytes = tables <= 3 ? 16u : 32u;
     info->o_terms1 = I.o_T1;
@@ -787,6 +788,7 @@ int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes
     for (uint32_t i = 0; i < tables; ++i) {
         info->tab_base[i] = I.tab_base[i];
         info->tab_wrap[i] = I.tab_wrap[i];
+        info->tab_mul[i] = I.tab_mul[i];
     }
     uint64_t np = 0;
     for (uint32_t i = 0; i < img.entries.size(); ++i)

@@ -148,16 +148,38 @@ uint32_t prime_of_power(uint32_t q) {
     return q == 1u ? p : 0u;
 }
 
-// -log of the share of candidates that pass "n mod d lies in `proj`", given the wheel: among the
-// residues mod d whose projection to g = gcd(d, M) the set holds at all.
-double value_of(const std::vector<uint8_t>& proj, uint32_t d, uint32_t g) {
-    uint32_t n = 0, ng = 0;
-    for (uint32_t r = 0; r < d; ++r) n += proj[r];
+// 32 packed bits from bit `at` on, of `words` words (0 past them)
+inline uint32_t bits_at(const uint32_t* bits, uint32_t words, uint32_t at) {
+    const uint32_t w = at >> 5, s = at & 31u;
+    const uint64_t lo = w < words ? bits[w] : 0u, hi = w + 1u < words ? bits[w + 1u] : 0u;
+    return (uint32_t)(((hi << 32) | lo) >> s);
+}
+
+// The packed admissible set of a filter (q residues) projected to d | q, packed: word by word.
+void project_bits(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint32_t>& out) {
+    const uint32_t words = (q + 31u) / 32u, n = (d + 31u) / 32u;
+    out.assign(n, 0u);
+    for (uint32_t from = 0; from < q; from += d)
+        for (uint32_t w = 0; w < n; ++w) out[w] |= bits_at(bits, words, from + 32u * w);
+    if (d % 32u) out[n - 1u] &= (1u << (d % 32u)) - 1u;
+}
+
+uint32_t count_bits(const std::vector<uint32_t>& v) {
+    uint32_t n = 0;
+    for (uint32_t w : v) n += (uint32_t)__builtin_popcount(w);
+    return n;
+}
+
+// -log of the share of candidates that pass "n mod d lies in the packed set `proj`", given the wheel:
+// among the residues mod d whose projection to g = gcd(d, M) the set holds at all.
+double value_of(const std::vector<uint32_t>& proj, uint32_t d, uint32_t g, std::vector<uint32_t>& tmp) {
+    const uint32_t n = count_bits(proj);
     if (n == 0) return 64.0;   // nothing is admissible
-    std::vector<uint8_t> pg(g, 0);
-    for (uint32_t r = 0; r < d; r += g)
-        for (uint32_t j = 0; j < g; ++j) pg[j] |= proj[r + j];
-    for (uint32_t j = 0; j < g; ++j) ng += pg[j];
+    uint32_t ng = 1;
+    if (g > 1u) {
+        project_bits(proj.data(), d, g, tmp);
+        ng = count_bits(tmp);
+    }
     return -std::log(((double)n / d) * ((double)g / ng));
 }
 
@@ -180,22 +202,16 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     const double budget = (double)(table_bytes / row_bytes);
     std::vector<EsPart> parts;
     std::vector<double> full(nf, 0.0);   // value of the whole filter
-    std::vector<uint8_t> proj;
+    std::vector<uint32_t> proj, tmp;
     for (uint32_t f = 0; f < nf; ++f) {
         const uint32_t q = P.q[f], gM = gcd32(q, (uint32_t)(P.M % q));
         const uint32_t* bits = P.allowed.data() + P.bit_off[f];
         const uint32_t p = prime_of_power(q);
         for (uint32_t d = p ? p : q;; d *= p) {
             const bool whole = d == q;
-            if (whole && gM == 1u) {
-                uint32_t n = 0;   // (bits past q in the last word are not admissible residues)
-                for (uint32_t w = 0; w < q / 32u; ++w) n += (uint32_t)__builtin_popcount(bits[w]);
-                if (q % 32u) n += (uint32_t)__builtin_popcount(bits[q / 32u] & ((1u << (q % 32u)) - 1u));
-                full[f] = n ? -std::log((double)n / q) : 64.0;
-                if (full[f] > 1e-3 && 2.0 * d <= budget) parts.push_back(EsPart{f, d, full[f]});
-            } else if (whole || 2.0 * d <= budget) {
-                es_project(bits, q, d, proj);
-                const double v = value_of(proj, d, gcd32(d, gM));
+            if (whole || 2.0 * d <= budget) {
+                project_bits(bits, q, d, proj);
+                const double v = value_of(proj, d, gcd32(d, gM), tmp);
                 if (whole) full[f] = v;
                 if (v > 1e-3 && 2.0 * d <= budget) parts.push_back(EsPart{f, d, v});
             }
@@ -207,7 +223,7 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     if (parts.size() > 48) parts.resize(48);
     auto rows = [&](uint32_t d) {
         const uint32_t m = (uint32_t)(P.M % d);
-        return (double)es_table_rows(d, m ? d - m : 0u, pair);
+        return (double)es_table_rows(d, std::max(m ? d - m : 0u, d / 4u), pair);   // (room for spread_of)
     };
     std::vector<Slot> slots;
     const uint32_t np = (uint32_t)parts.size();
@@ -300,6 +316,76 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
 
 namespace {
 
+uint64_t xorshift(uint64_t& s) {
+    s ^= s << 13;
+    s ^= s >> 7;
+    s ^= s << 17;
+    return s;
+}
+
+// The multiplier of an inner table: its rows are indexed by u n mod d, u coprime to d.  The lanes of a
+// warp take consecutive rows of ring 3's digits, so their phases are, wraps apart, an arithmetic
+// progression whose difference is an accident of the wheel: a difference with many factors of two
+// puts all lanes on the same few banks, an odd one spreads them better than chance.  So the library
+// tries multipliers on sampled warps and takes the one with the fewest wavefronts.  2^34 positions:
+// k = 384 2200 -> 1636 us, k = 390 1585 -> 1482, k = 379 1775 -> 1727, k = 300 1356 -> 1323.
+constexpr uint32_t kSampleWarps = 8;
+
+// b3 of the 32 lanes of a few warps (no short scan gains from this: none for blocks below 2^26).
+std::vector<u128> sample_rows(const EsHostPlan& P, uint64_t R, uint64_t& seed) {
+    std::vector<u128> b3;
+    if (R < (1ull << 26)) return b3;
+    for (uint32_t w = 0; w < kSampleWarps; ++w) {
+        const uint64_t row0 = xorshift(seed) >> 24;
+        for (uint32_t l = 0; l < 32; ++l) {
+            uint64_t rem = row0 + l;
+            u128 v = 0;
+            for (size_t j = 3; j < P.radix.size(); ++j) {
+                v += P.terms[P.roff[j] + rem % P.radix[j]];
+                if (v >= P.M) v -= P.M;
+                rem /= P.radix[j];
+            }
+            b3.push_back(v);
+        }
+    }
+    return b3;
+}
+
+uint32_t spread_of(const std::vector<u128>& b3, uint64_t& seed, uint32_t d, uint32_t corr, bool pair, uint32_t row_bytes) {
+    if (row_bytes > 16u || d < 8u || b3.empty()) return 1u;
+    const uint32_t lanes = 128u / row_bytes;   // per wavefront at best; rows across all banks
+    std::vector<uint32_t> res(b3.size()), shift(2 * kSampleWarps);   // shifts: the other rings' terms
+    for (size_t i = 0; i < b3.size(); ++i) res[i] = es_mod(b3[i], d);
+    for (uint32_t& x : shift) x = (uint32_t)(xorshift(seed) % d);
+    uint32_t best = 1, least = ~0u;
+    for (uint32_t t = 0; t < 64; ++t) {
+        const uint32_t u = t == 0 ? 1u : (uint32_t)(xorshift(seed) % (d - 1u)) + 1u;
+        if (gcd32(u, d) != 1u) continue;
+        const uint32_t c = (uint32_t)((uint64_t)u * corr % d);
+        // where the wrapped row is a row of its own it must not need more of them than were planned
+        if (!pair && t && std::min(c, d - c) > std::max(std::min(corr, d - corr), d / 4u)) continue;
+        uint32_t cost = 0;
+        for (uint32_t w = 0; w < kSampleWarps; ++w)
+            for (uint32_t from = 0; from < 32; from += lanes) {
+                uint32_t at[16][16], n[16] = {0}, most = 0;   // distinct rows by bank
+                for (uint32_t l = from; l < from + lanes; ++l) {
+                    const uint32_t x = (uint32_t)(((uint64_t)u * res[32 * w + l] + shift[2 * w]) % d) + shift[2 * w + 1];
+                    const uint32_t bank = x % lanes;
+                    bool seen = false;
+                    for (uint32_t i = 0; i < n[bank]; ++i) seen = seen || at[bank][i] == x;
+                    if (!seen) at[bank][n[bank]++] = x;
+                    most = std::max(most, n[bank]);
+                }
+                cost += most;
+            }
+        if (cost < least) {
+            least = cost;
+            best = u;
+        }
+    }
+    return best;
+}
+
 // Bytes the inner tables may take: what the CTA has left, and no more than staging them is worth.
 // Every CTA copies them at launch, so a plan whose whole block is a short scan keeps them small.
 uint32_t table_bytes(uint64_t R, size_t smem_bytes, size_t small_bytes) {
@@ -353,9 +439,13 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         entries.push_back(EsCascadeEntry{2u, {}});
         fc.push_back(es_filter_consts(M, 2u, ones));
     };
+    uint64_t seed = 0x9e3779b97f4a7c15ull;
+    const std::vector<u128> sample = sample_rows(P, geo.n_outer * r0, seed);
     for (const std::vector<EsPart>& table : C.inner) {
         if (table.empty()) {
+            I.tab_mul[entries.size()] = 1;
             fill();
+            fc.back().off = 1;
             continue;
         }
         EsCascadeEntry e{1u, {}};
@@ -367,8 +457,16 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
             while (p.d > 1u && (uint64_t)u * k % p.d != 1u) ++k;
             e.parts.push_back(EsCascadeEntry::Part{p.f, p.d, p.d > 1u ? (uint32_t)((uint64_t)co * k % e.q) : 0u});
         }
+        // residues are kept times the table's multiplier: limb weights (`off`, which has no use here, is
+        // the lowest limb's), wrap correction and block constant
+        EsFilterC c = es_filter_consts(M, e.q, 0);
+        const uint32_t u = spread_of(sample, seed, e.q, c.corr, pair, row_bytes);
+        I.tab_mul[entries.size()] = u;
+        for (uint32_t* w : {&c.corr, &c.w1, &c.w2, &c.w3}) *w = (uint32_t)((uint64_t)*w * u % e.q);
+        c.off = u;
+        for (EsCascadeEntry::Part& p : e.parts) p.unit = (uint32_t)((uint64_t)p.unit * u % e.q);
         entries.push_back(e);
-        fc.push_back(es_filter_consts(M, e.q, ones));   // no bit table: tested by the inner table alone
+        fc.push_back(c);
     }
     for (int f : C.residue) {
         if (f < 0)
@@ -386,7 +484,7 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     std::vector<uint8_t> adm, one;
     for (uint32_t i = 0; i < F; ++i) {
         const EsCascadeEntry& e = entries[i];
-        const uint32_t d = e.q, corr = fc[i].corr;
+        const uint32_t d = e.q, corr = fc[i].corr, u = I.tab_mul[i];
         adm.assign(d, 1);
         for (const EsCascadeEntry::Part& p : e.parts) {
             const uint32_t q = P.q[p.f];
@@ -399,8 +497,13 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         phase.assign((size_t)d * RS, 0u);
         for (uint32_t s = 0; s < r0; ++s) {
             const uint32_t a = es_mod(R.S0[s], d), wd = s >> 5, at = s & 31u;
-            for (uint32_t ph = 0; ph < d - a; ++ph) phase[(size_t)ph * RS + wd] |= (uint32_t)adm[ph + a] << at;
-            for (uint32_t ph = d - a; ph < d; ++ph) phase[(size_t)ph * RS + wd] |= (uint32_t)adm[ph + a - d] << at;
+            // phase ph is row u ph mod d
+            for (uint32_t ph = 0, r = 0, m = a; ph < d; ++ph) {
+                phase[(size_t)r * RS + wd] |= (uint32_t)adm[m] << at;
+                if (++m == d) m = 0;
+                r += u;
+                if (r >= d) r -= d;
+            }
         }
         const bool up = pair || corr <= d - corr;
         const uint32_t lead = up ? 0u : d - corr, rows = es_table_rows(d, corr, pair);
@@ -420,48 +523,45 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     }
 
     // ---- carry-split buckets -----------------------------------------------------------------
-    // Entry of bucket b = [lo, hi] of the key t of thr = M - b: the slots certainly below thr for
-    // every t of the bucket, and above them the low bits of the one key that lies in it.  Keys of
-    // wheels wider than 32 bits are rounded, t to within +-1: slot keys are stored plus one, so
-    // that a slot is certainly below when its key is < t and certainly not when it is > t + 2.
-    const uint32_t kbits = es_bitlen(M >> sh), nb = 1u << ES_PBUCKET_LOG2;
-    const uint32_t bsh = kbits > ES_PBUCKET_LOG2 ? kbits - ES_PBUCKET_LOG2 : 0, ssh = 32u - bsh;
-    const uint32_t around = sh ? 2u : 0u;
-    const uint64_t flag = ssh >= 32u ? 0xffffffffull : (1ull << ssh) - 1;
+    // Keys are the top 32 bits of values scaled to M's width (shifted up where M is below 2^32), and
+    // t, the key of thr = M - b, is a difference of such keys: exact to within +-1.  Slot keys are
+    // stored plus one, so that a slot is certainly below thr when its key is < t and certainly not
+    // when it is > t + 2.  Entry of bucket [lo, hi] of t: the slots certainly below thr for every t
+    // of the bucket, and above them the low bits of the one key that lies in it.
+    constexpr uint32_t nb = 1u << ES_PBUCKET_LOG2, bsh = 32u - ES_PBUCKET_LOG2, ssh = ES_PBUCKET_LOG2;
+    constexpr uint32_t flag = (1u << ssh) - 1u;
+    const uint32_t lsh = sh ? 0u : 32u - es_bitlen(M);
+    auto key_of = [&](u128 v) { return (uint32_t)(v >> sh) << lsh; };
     std::vector<uint64_t> key(r0);
-    for (uint32_t i = 0; i < r0; ++i)
-        key[i] = std::min<uint64_t>((uint64_t)(R.S0[i] >> sh) + (sh ? 1u : 0u), 0xffffffffull);
+    for (uint32_t i = 0; i < r0; ++i) key[i] = std::min<uint64_t>((uint64_t)key_of(R.S0[i]) + 1u, 0xffffffffull);
     for (uint32_t b = 0, n = 0; b < nb; ++b) {
         const uint64_t lo = (uint64_t)b << bsh, hi = lo + (1ull << bsh) - 1;
         while (n < r0 && key[n] < lo) ++n;
         uint32_t m = n;
-        while (m < r0 && key[m] <= hi + around) ++m;
-        uint32_t v;
-        if (n >= flag)
-            v = (uint32_t)flag;
-        else if (m == n)
+        while (m < r0 && key[m] <= hi + 2) ++m;
+        uint32_t v = flag;   // several keys, or too many slots to hold: found exactly
+        if (n < flag && m == n)
             v = (uint32_t)((((1ull << bsh) - 1) << ssh) | n);
-        else if (bsh == 0 && around == 0)
-            v = n;   // the bucket is one key value: slots at it are not below
-        else if (m == n + 1 && key[n] <= hi)
+        else if (n < flag && m == n + 1 && key[n] <= hi)
             v = (uint32_t)(((key[n] - lo) << ssh) | n);
-        else
-            v = (uint32_t)flag;   // several keys: found exactly
         S.put32(I.o_BK, b, v);
     }
 
     // ---- the rest of the small block ---------------------------------------------------------
+    auto scaled = [&](u128 v, uint32_t f) {   // residue of an inner table, times its multiplier
+        return (uint32_t)((uint64_t)es_mod(v, entries[f].q) * I.tab_mul[f] % entries[f].q);
+    };
     for (uint32_t i = 0; i < r1; ++i) {
         const u128 v = P.terms[P.roff[1] + i];
         S.put128(I.o_T1, i, v);
-        S.put32(I.o_R1 + row1 * i, 0, (uint32_t)(v >> sh));
-        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_R1 + row1 * i, 1 + f, row_bytes * es_mod(v, entries[f].q));
+        S.put32(I.o_R1 + row1 * i, 0, key_of(v));
+        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_R1 + row1 * i, 1 + f, row_bytes * scaled(v, f));
         for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_TQr, 4 * i + f, es_mod(v, entries[F + f].q));
     }
     for (uint32_t i = 0; i < r2; ++i) {
         const u128 v = P.terms[P.roff[2] + i];
         S.put128(I.o_T2, i, v);
-        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_TQ2, i * ds + f, es_mod(v, entries[f].q));
+        for (uint32_t f = 0; f < F; ++f) S.put32(I.o_TQ2, i * ds + f, scaled(v, f));
         for (uint32_t f = 0; f < ES_PRES; ++f) S.put32(I.o_TQ2r, 4 * i + f, es_mod(v, entries[F + f].q));
     }
     for (uint32_t i = 0; i < r0; ++i) {
@@ -497,9 +597,8 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     }
     I.n_filters = (uint32_t)entries.size();
     I.F = F;
-    I.bsh = bsh;
-    I.ssh = ssh;
-    I.band = sh ? 3u << ssh : 0u;   // sh > 0: 32-bit keys, ssh = ES_PBUCKET_LOG2
+    I.lsh = lsh;
+    I.km = key_of(M);
     I.row_bytes = row_bytes;
     I.tab_words = (uint32_t)tabs.size();
     I.small_bytes = (uint32_t)S.b.size();

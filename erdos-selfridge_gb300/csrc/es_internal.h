@@ -80,11 +80,11 @@ struct EsInst {
     uint32_t o_TQ2;       // [r2] ring-2 term residues of the inner tables (rows of 4 or 8 words)
     uint32_t o_TQ2r;      // [r2] ring-2 term residues of the residue-stage filters
     uint32_t o_Qr;        // [r0] inner-ring residues of the residue-stage filters
-    uint32_t ssh;         // 32 - bsh: bucket entries hold the key's low bits above the slot
-    uint32_t band;        // key distance below which the split is found exactly, << ssh
+    uint32_t lsh;         // keys of M below 2^32 are shifted up to 32 bits by this
     uint32_t row_bytes;   // bytes from one phase's row to the next
     uint32_t tab_base[ES_PMAX];   // byte offset of each table's phase-0 row in the staged block
     int32_t tab_wrap[ES_PMAX];    // byte distance from a row to the row a wrap past M selects
+    uint32_t tab_mul[ES_PMAX];    // multiplier of each table's row index (es_cascade.cu)
     uint32_t tab_words;   // words of all inner tables
     uint32_t n_groups;    // groups of rings >= 3, whose sums are ring_terms
     EsGroup group[ES_MAX_GROUPS];

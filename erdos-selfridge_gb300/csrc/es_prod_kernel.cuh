@@ -83,6 +83,20 @@ __device__ __forceinline__ uint32_t shl_c(uint32_t v, uint32_t n) {   // shifts 
     return r;
 }
 
+// The sweep is bound by the ALU pipe next to shared memory, and selects and three-input adds are ALU
+// work: a select between x and x + d is a multiply-add on the FMA pipe instead (k = 390, 2^34
+// positions 1480 -> 1401 us, k = 378 1310 -> 1217).  Inline assembly, so that they stay so.
+__device__ __forceinline__ uint32_t mad_lo(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t zero_or_one(bool p) {
+    uint32_t r;
+    asm("mov.u32 %0, %1;" : "=r"(r) : "r"((uint32_t)p));
+    return r;
+}
+
 // Predicated loads: lanes whose `alive` is 0 load nothing and get an arbitrary value.
 __device__ __forceinline__ uint2 lds64_if(uint32_t a, uint32_t alive) {
     uint2 v;
@@ -95,6 +109,15 @@ __device__ __forceinline__ uint4 lds128_if(uint32_t a, uint32_t alive) {
     asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a), "r"(alive));
     return v;
+}
+
+// x mod q times the multiplier of an inner table (limb weights from `off` on carry it)
+__device__ __forceinline__ uint32_t mod128_times(const U4 x, const EsFilterC& f) {
+    const uint64_t y = (uint64_t)x.x * f.off + (uint64_t)x.y * f.w1 + (uint64_t)x.z * f.w2 + (uint64_t)x.w * f.w3;
+    const uint64_t qt = __umul64hi(y, f.rcp);
+    uint64_t r = y - qt * f.q;
+    if (r >= f.q) r -= f.q;
+    return (uint32_t)r;
 }
 
 // b3 = sum_{j>=3} term_j[d_j] mod M for ring-2 row `row`, from the sums over groups of rings.
@@ -350,8 +373,8 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
     __syncwarp();
 
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint32_t rb = si.row_bytes, KM = si.km, bsh = si.bsh, ssh = si.ssh, band = si.band;
-    const uint32_t smask = ssh >= 32u ? 0xffffffffu : (1u << ssh) - 1u;
+    const uint32_t rb = si.row_bytes, KM = si.km;
+    constexpr uint32_t bsh = 32u - ES_PBUCKET_LOG2, ssh = ES_PBUCKET_LOG2, smask = (1u << ssh) - 1u, band = 3u << ssh;
     const uint32_t bk = sbase + si.o_BK;
     int32_t wrap[F];   // (one- and two-word rings have the wrapped row in the row itself)
 #pragma unroll
@@ -382,7 +405,7 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
             }
             const U4 b3 = decode_row(si, row, Mv);
 #pragma unroll
-            for (int f = 0; f < F; ++f) BQ3[f] = red1(mod128(b3, sFC[f]) + tcv[f], sFC[f].q);
+            for (int f = 0; f < F; ++f) BQ3[f] = red1(mod128_times(b3, sFC[f]) + tcv[f], sFC[f].q);
             uint32_t rv[ES_PRES];
 #pragma unroll
             for (uint32_t j = 0; j < ES_PRES; ++j) rv[j] = red1(mod128(b3, sFC[F + j]) + tcv[F + j], sFC[F + j].q);
@@ -391,8 +414,8 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
         }
         uint32_t wm2;
         const U4 b2 = addmod(ldv128(&Q->rec0[lane]), u4(reinterpret_cast<const uint4*>(smem + si.o_T2)[d2]), Mv, wm2);
-        // shared addresses of the tables' rows at BQ2 without and with the ring-1 wrap
-        uint32_t B[F], Bc[F];
+        // shared addresses of the tables' rows at BQ2, and what the ring-1 wrap adds to them
+        uint32_t B[F], Bw[F];
         constexpr uint32_t DS = F <= 4 ? 4u : 8u;
         const uint32_t* tq2 = reinterpret_cast<const uint32_t*>(smem + si.o_TQ2) + d2 * DS;
 #pragma unroll
@@ -402,12 +425,12 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
             const uint32_t base = sbase + L.stage_off + ldv32(&si.tab_base[f]);
             const uint32_t BQ2 = red2(BQ3[f] + tq2[f] + (corr & wm2), q);
             B[f] = base + rb * BQ2;
-            Bc[f] = base + rb * red1(BQ2 + corr, q);
+            Bw[f] = base + rb * red1(BQ2 + corr, q) - B[f];
         }
         const uint32_t ews = lane | (step << 17);   // entry fields that belong to the step
         // A = M - b2 and its 32-bit key, once per ring-1 cycle
         uint32_t brA;
-        const uint32_t KA = key32(sub128(Mv, b2, brA), si.sh);
+        const uint32_t KA = key32(sub128(Mv, b2, brA), si.sh) << si.lsh;
 
         // ---- ring 1 (a list has one digit per lane) -----------------------------------------
         const uint32_t nd = list ? 1u : r1;
@@ -423,18 +446,43 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
                 load_row<F>(row + v * ProdRow<F>::kBytes, k1, tq);
                 // ring-1 wrap (b2 + T1 >= M, i.e. T1 >= A) from the 32-bit keys, and t, the key of
                 // thr = M - b to within +-1 (0 <= t <= KM away from a key tie)
-                const bool p = k1 > KA;
-                const uint32_t t = KA - k1 + (p ? KM : 0u);
+                const uint32_t p = zero_or_one(k1 > KA);
+                const uint32_t t = mad_lo(p, KM, KA - k1);
                 const uint32_t e4 = lds32(bk + ((t >> bsh) << 2));
-                const uint32_t ts = shl_c(t, ssh);
+                const uint32_t ts = t << ssh;
                 const uint32_t sp = e4 & smask;
                 split[v] = sp + (e4 < ts ? 1u : 0u);
                 rare[v] = (e4 - ts < band) || (sp == smask) || (k1 == KA);
                 any_rare = any_rare || rare[v];
-                wm1[v] = p ? 0xffffffffu : 0u;
+                wm1[v] = 0u - p;
 #pragma unroll
-                for (int f = 0; f < F; ++f) a[v][f] = (p ? Bc[f] : B[f]) + tq[f];
+                for (int f = 0; f < F; ++f) a[v][f] = mad_lo(p, Bw[f], B[f] + tq[f]);
             }
+            // The first table's row is on its way before the vote on the exact path (whose lanes load
+            // theirs again if the wrap was other than the keys said): k = 390, 2^34 positions 1659 ->
+            // 1599 us, k = 384 2312 -> 2202, k = 379 1866 -> 1808, k = 300 1371 -> 1364.  Two rows cost
+            // registers in wide rings (k = 378 1343 -> 1524).
+            constexpr int PRE = WT == 0 ? 0 : 1;
+            uint32_t pre0[NU][PRE + 1][4], pre1[NU][PRE + 1][4];
+            auto load_pair = [&](uint32_t at, int f, uint32_t (&x0)[4], uint32_t (&x1)[4]) {
+                if (WT == 1) {
+                    const uint2 y = lds64(at);
+                    x0[0] = y.x;
+                    x1[0] = y.y;
+                } else if (WT == 2) {
+                    const uint2 y0 = lds64(at), y1 = lds64(at + wrap[f]);
+                    x0[0] = y0.x; x0[1] = y0.y;
+                    x1[0] = y1.x; x1[1] = y1.y;
+                } else {
+                    const uint4 y0 = lds128(at), y1 = lds128(at + wrap[f]);
+                    x0[0] = y0.x; x0[1] = y0.y; x0[2] = y0.z; x0[3] = y0.w;
+                    x1[0] = y1.x; x1[1] = y1.y; x1[2] = y1.z; x1[3] = y1.w;
+                }
+            };
+#pragma unroll
+            for (uint32_t v = 0; v < NU; ++v)
+#pragma unroll
+                for (int f = 0; f < PRE; ++f) load_pair(a[v][f], f, pre0[v][f], pre1[v][f]);
             if (__any_sync(0xffffffffu, any_rare)) {
 #pragma unroll
                 for (uint32_t v = 0; v < NU; ++v) {
@@ -443,9 +491,12 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
                         const uint32_t was = wm1[v], x = prod_split(Q, smem, si, lane, d2, d1 + v);
                         split[v] = x & 0x7fffffffu;
                         wm1[v] = (x >> 31) ? 0xffffffffu : 0u;
+                        if (was != wm1[v]) {
 #pragma unroll
-                        for (int f = 0; f < F; ++f)
-                            if (was != wm1[v]) a[v][f] += wm1[v] ? Bc[f] - B[f] : B[f] - Bc[f];
+                            for (int f = 0; f < F; ++f) a[v][f] += wm1[v] ? Bw[f] : 0u - Bw[f];
+#pragma unroll
+                            for (int f = 0; f < PRE; ++f) load_pair(a[v][f], f, pre0[v][f], pre1[v][f]);
+                        }
                     }
                 }
             }
@@ -487,14 +538,21 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
 #pragma unroll
                     for (int f = 0; f < F; ++f) {
                         uint32_t x0[4], x1[4];
-                        if (WT == 1) {
-                            const uint2 y = f < 2 ? lds64(a[v][f]) : lds64_if(a[v][f], m0[0] | m1[0]);
+                        if (f < PRE) {
+#pragma unroll
+                            for (uint32_t j = 0; j < NW; ++j) {
+                                x0[j] = pre0[v][f < PRE ? f : 0][j];
+                                x1[j] = pre1[v][f < PRE ? f : 0][j];
+                            }
+                        } else if (f < 2) {
+                            load_pair(a[v][f], f, x0, x1);
+                        } else if (WT == 1) {
+                            const uint2 y = lds64_if(a[v][f], m0[0] | m1[0]);
                             x0[0] = y.x;
                             x1[0] = y.y;
                         } else if (WT == 2) {
-                            const uint2 y0 = f < 2 ? lds64(a[v][f]) : lds64_if(a[v][f], m0[0] | m0[NW - 1]);
-                            const uint2 y1 =
-                                f < 2 ? lds64(a[v][f] + wrap[f]) : lds64_if(a[v][f] + wrap[f], m1[0] | m1[NW - 1]);
+                            const uint2 y0 = lds64_if(a[v][f], m0[0] | m0[NW - 1]);
+                            const uint2 y1 = lds64_if(a[v][f] + wrap[f], m1[0] | m1[NW - 1]);
                             x0[0] = y0.x; x0[1] = y0.y;
                             x1[0] = y1.x; x1[1] = y1.y;
                         } else {
@@ -504,8 +562,7 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
                                 l0 |= m0[j];
                                 l1 |= m1[j];
                             }
-                            const uint4 y0 = f < 2 ? lds128(a[v][f]) : lds128_if(a[v][f], l0);
-                            const uint4 y1 = f < 2 ? lds128(a[v][f] + wrap[f]) : lds128_if(a[v][f] + wrap[f], l1);
+                            const uint4 y0 = lds128_if(a[v][f], l0), y1 = lds128_if(a[v][f] + wrap[f], l1);
                             x0[0] = y0.x; x0[1] = y0.y; x0[2] = y0.z; x0[3] = y0.w;
                             x1[0] = y1.x; x1[1] = y1.y; x1[2] = y1.z; x1[3] = y1.w;
                         }

@@ -59,10 +59,10 @@ class BatchItem(C.Structure):
 class CascadeInfo(C.Structure):
     _fields_ = [("small_bytes", C.c_uint64), ("tab_words", C.c_uint64), ("n_parts", C.c_uint64),
                 ("n_entries", C.c_uint32), ("row_bytes", C.c_uint32), ("key_shift", C.c_uint32),
-                ("bucket_shift", C.c_uint32), ("band", C.c_uint32), ("o_row1", C.c_uint32),
+                ("key_up", C.c_uint32), ("bucket_log2", C.c_uint32), ("o_row1", C.c_uint32),
                 ("row1_bytes", C.c_uint32), ("o_terms1", C.c_uint32), ("o_sorted", C.c_uint32),
                 ("o_digits", C.c_uint32), ("o_buckets", C.c_uint32), ("reserved", C.c_uint32),
-                ("tab_base", C.c_uint32 * 6), ("tab_wrap", C.c_int32 * 6)]
+                ("tab_base", C.c_uint32 * 6), ("tab_wrap", C.c_int32 * 6), ("tab_mul", C.c_uint32 * 6)]
 
 
 SURVIVOR_DTYPE = np.dtype([("idx", "<u8"), ("s_lo", "<u8"), ("s_hi", "<u8"), ("t", "<u8"),

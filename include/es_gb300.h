@@ -134,10 +134,11 @@ int es_device_name(char* out, uint32_t cap);
  * it.  Entries 0..tables-1 are the inner tables, the next four the residue stage. */
 typedef struct es_cascade_info {
     uint64_t small_bytes, tab_words, n_parts;
-    uint32_t n_entries, row_bytes, key_shift, bucket_shift, band;
+    uint32_t n_entries, row_bytes, key_shift, key_up, bucket_log2;
     uint32_t o_row1, row1_bytes, o_terms1, o_sorted, o_digits, o_buckets, reserved;
     uint32_t tab_base[6];
     int32_t tab_wrap[6];
+    uint32_t tab_mul[6];   /* a table's rows are indexed by n * tab_mul mod its modulus */
 } es_cascade_info;
 int es_cascade_image(const es_plan_desc* desc, uint32_t tables, uint32_t smem_bytes, es_cascade_info* info,
                      void* small, uint64_t small_cap, uint32_t* tabs, uint64_t tabs_cap, uint32_t* parts,

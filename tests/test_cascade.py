@@ -81,15 +81,13 @@ def test_tables_match_definition(spec):
         W = -(-r0 // 32)
         RS = 4 if W == 3 else W
         assert info.row_bytes == (8 * RS if W <= 1 else 4 * RS)   # one word: both masks in a row
-        sh, bsh, band = info.key_shift, info.bucket_shift, info.band
-        ssh = 32 - bsh
-        mask32 = 0xffffffff
-        flag = (1 << ssh) - 1 if ssh < 32 else mask32
+        sh, up, ssh = info.key_shift, info.key_up, info.bucket_log2
+        bsh, band, flag, mask32 = 32 - ssh, 3 << ssh, (1 << ssh) - 1, 0xffffffff
         t_blk = int(rng.integers(0, 1 << 30))
         for _ in range(6):
             b2 = sum(terms[j][int(rng.integers(radix[j]))] for j in range(2, len(radix))) % P.M
             A = P.M - b2
-            KA, KM = (A >> sh) & mask32, P.M >> sh
+            KA, KM = (A >> sh << up) & mask32, P.M >> sh << up
             for d1 in ([0, r1 - 1] + rng.integers(0, r1, size=6).tolist()):
                 row = info.o_row1 // 4 + d1 * info.row1_bytes // 4
                 k1 = int(u32[row])
@@ -98,7 +96,7 @@ def test_tables_match_definition(spec):
                 bucket = t >> bsh
                 assert bucket < 2048
                 e4 = int(u32[info.o_buckets // 4 + bucket])
-                ts = (t << ssh) & mask32 if ssh < 32 else 0
+                ts = (t << ssh) & mask32
                 split = (e4 & flag) + (1 if e4 < ts else 0)
                 rare = ((e4 - ts) & mask32) < band or (e4 & flag) == flag or k1 == KA
                 exact1 = terms[1][d1] >= A
@@ -108,9 +106,11 @@ def test_tables_match_definition(spec):
                     wrap1, split = exact1, exact_split
                 assert wrap1 == exact1 and split == exact_split
                 for i in range(F):
+                    mul = info.tab_mul[i]
+                    assert np.gcd(mul, q[i]) == 1
                     tc = t_blk * P.M % q[i]
-                    corr = -P.M % q[i]
-                    B = (b2 + tc) % q[i]
+                    corr = -P.M * mul % q[i]
+                    B = (b2 + tc) * mul % q[i]
                     if wrap1:
                         B = (B + corr) % q[i]
                     a = info.tab_base[i] + info.row_bytes * B + int(u32[row + 1 + i])
