@@ -26,7 +26,7 @@
 #define ES_FMAX 8
 #define ES_NBUCKET_LOG2 9
 #define ES_NBUCKET (1u << ES_NBUCKET_LOG2)   // carry-split buckets over the 32-bit keys
-#define ES_QUEUE_BYTES 2592   // per-warp shared slot: entry queue, lane records, tail context
+#define ES_QUEUE_BYTES 2304   // per-warp shared slot: entry queue, lane records, tail context
 #define ES_MAX_RINGS 64
 #define ES_MAX_FILTERS 192   // pi(1024) = 172 residual primes at most
 #define ES_PMAX 6            // inner tables of the production cascade, at most

@@ -67,17 +67,10 @@ struct ProdCtx {
     uint32_t M_big;
 };
 
-#define ES_REST 8
 struct ProdQueue {
     uint4 ent[ES_QCAP];
     uint4 rec0[32];                    // per lane: b3 = sum of the terms of rings >= 3, mod M (limbs)
     uint4 rec1[32];                    // per lane: b3 + block term mod the residue-stage filters
-    struct Rest {
-        U4 s;                          // n mod M
-        uint64_t oidx;
-        uint32_t slot, pad;
-    } rest[ES_REST];                   // candidates for the rest of the cascade, at the unit's end
-    uint32_t n_rest;
     uint16_t own_d2[32];               // per lane: ring-2 digit, where lanes do not share it
     ProdCtx ctx;
 };
@@ -147,16 +140,26 @@ __device__ __noinline__ U4 decode_row(const EsInst& si, uint64_t row, const U4 M
     return acc;
 }
 
-// n mod q_f admissible, from s = n mod M in 128 bits and the block constant
-__device__ __forceinline__ bool tail_filter(const ProdCtx& C, const EsFilterC* sFC, uint32_t f, const U4 s) {
-    const EsFilterC fc = sFC[f];
-    uint32_t r = mod128(s, fc) + C.tc[f];
-    if (r >= fc.q) r -= fc.q;
-    return (__ldg(C.allowed_g + fc.off + (r >> 5)) >> (r & 31u)) & 1u;
-}
-
-__device__ __forceinline__ void prod_emit(const ProdCtx& C, const unsigned char* smem, const EsInst& si, const U4 s,
-                                          uint64_t oidx, uint32_t slot) {
+// The candidates that passed the residue stage: range test, n mod M in 128 bits, the rest of the
+// cascade by limb weights and Barrett, then the emit.
+__device__ __forceinline__ void prod_tail(const ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t f0,
+                                          const U4 b2, uint32_t own, uint32_t d1, uint32_t slot, uint32_t step) {
+    const ProdCtx& C = Q->ctx;
+    const uint64_t e = C.e_base + (uint64_t)own * C.lstride + step;
+    if (e < C.e_min || e >= C.e_max) return;
+    const uint64_t oidx = C.list ? __ldg(C.list + e) : e * C.r1 + d1;
+    if (oidx < C.o_begin || oidx >= C.o_end) return;
+    const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
+    uint32_t wm;
+    const U4 b = addmod(b2, u4(reinterpret_cast<const uint4*>(smem + si.o_T1)[d1]), C.M, wm);
+    const U4 s = addmod(b, u4(reinterpret_cast<const uint4*>(smem + si.o_S0)[slot]), C.M, wm);
+    for (uint32_t f = f0; f < C.nf; ++f) {
+        const EsFilterC fc = sFC[f];
+        uint32_t r = mod128(s, fc) + C.tc[f];
+        if (r >= fc.q) r -= fc.q;
+        const uint32_t wv = __ldg(C.allowed_g + fc.off + (r >> 5));
+        if (!((wv >> (r & 31u)) & 1u)) return;
+    }
     bool good;
     if (C.M_big) {
         good = (C.t_blk > 0) || s.w || s.z || s.y || (s.x > C.kp1);
@@ -175,55 +178,6 @@ __device__ __forceinline__ void prod_emit(const ProdCtx& C, const unsigned char*
         rec->good = good ? 1u : 0u;
     }
     if (good && C.group_found) atomicMin(C.group_found + C.group, (unsigned long long)C.t_blk);
-}
-
-// A candidate that passed the residue stage: range test, n mod M in 128 bits, two more filters by limb
-// weights and Barrett.  What is left (one in thousands) waits for the unit's end, where the warp
-// tests a filter per lane: a true survivor then waits for two or three loads instead of one per
-// filter (59 in a row were half of a short scan's 29 us at k = 300).  Where the list is full the
-// lane goes through the filters itself.  Only for one-word rings (REST): short scans are theirs, and
-// the list costs wider rings registers (k = 379, 2^34 positions 1683 -> 1719 us).
-template <bool REST>
-__device__ __forceinline__ void prod_tail(ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t f0,
-                                          const U4 b2, uint32_t own, uint32_t d1, uint32_t slot, uint32_t step) {
-    const ProdCtx& C = Q->ctx;
-    const uint64_t e = C.e_base + (uint64_t)own * C.lstride + step;
-    if (e < C.e_min || e >= C.e_max) return;
-    const uint64_t oidx = C.list ? __ldg(C.list + e) : e * C.r1 + d1;
-    if (oidx < C.o_begin || oidx >= C.o_end) return;
-    const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
-    uint32_t wm;
-    const U4 b = addmod(b2, u4(reinterpret_cast<const uint4*>(smem + si.o_T1)[d1]), C.M, wm);
-    const U4 s = addmod(b, u4(reinterpret_cast<const uint4*>(smem + si.o_S0)[slot]), C.M, wm);
-    for (uint32_t f = f0; f < C.nf; ++f) {
-        if (REST && f == f0 + 2u) {
-            const uint32_t at = atomicAdd(&Q->n_rest, 1u);
-            if (at < ES_REST) {
-                Q->rest[at].s = s;
-                Q->rest[at].oidx = oidx;
-                Q->rest[at].slot = slot;
-                return;
-            }
-        }
-        if (!tail_filter(C, sFC, f, s)) return;
-    }
-    prod_emit(C, smem, si, s, oidx, slot);
-}
-
-// warp-uniform, at the unit's end: the listed candidates through the filters from f0 on, a lane each
-__device__ __forceinline__ void prod_rest(ProdQueue* Q, const unsigned char* smem, const EsInst& si, uint32_t lane,
-                                          uint32_t f0) {
-    __syncwarp();
-    const uint32_t n = min(Q->n_rest, (uint32_t)ES_REST);
-    const ProdCtx& C = Q->ctx;
-    const EsFilterC* sFC = reinterpret_cast<const EsFilterC*>(smem + si.o_FC);
-    for (uint32_t i = 0; i < n; ++i) {
-        const U4 s = Q->rest[i].s;
-        bool pass = true;
-        for (uint32_t base = f0; base < C.nf && pass; base += 32u)
-            pass = __all_sync(0xffffffffu, tail_filter(C, sFC, min(base + lane, C.nf - 1u), s));
-        if (pass && lane == 0) prod_emit(C, smem, si, s, Q->rest[i].oidx, Q->rest[i].slot);
-    }
 }
 
 // warp-uniform: one pass over up to 32 queued entries.  Each lane takes the lowest candidate of its
@@ -288,7 +242,7 @@ __device__ __forceinline__ void prod_flush(ProdQueue* Q, const unsigned char* sm
             ok = ok && ((wv >> (x & 31u)) & 1u);
         }
     }
-    if (ok) prod_tail<PD>(Q, smem, si, F + ES_PRES, b2, own, d1, slot, step);
+    if (ok) prod_tail(Q, smem, si, F + ES_PRES, b2, own, d1, slot, step);
     __syncwarp();
 }
 
@@ -403,7 +357,6 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
         C.group = item.group;
         C.t_blk = item.t;
         C.lstride = lstride;
-        Q->n_rest = 0;
         C.d2 = rows ? wlo : ES_OWN_DIGIT;
         C.row0 = row0;
         C.list = reinterpret_cast<const unsigned long long*>(item.list);
@@ -645,7 +598,6 @@ __device__ __forceinline__ void prod_unit(const EsLaunch& L, const EsInst& si, u
         if (!rows || step + 1u == nsteps)
             while (qsize) prod_flush<F, PD>(Q, smem, si, lane, qhead, qsize);
     }
-    if (PD) prod_rest(Q, smem, si, lane, F + ES_PRES + 2u);
     __syncwarp();
 }
 
