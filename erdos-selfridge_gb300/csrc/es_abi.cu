@@ -1,6 +1,7 @@
 // Host side of the C ABI (include/es_gb300.h): validates a plan descriptor, derives every
-// device table in C++ (sorted inner ring, carry-split keys and buckets, ring-1 residue table,
-// ring-2 delta table, word-mask phase tables), uploads them in one arena per plan, and drives
+// device table in C++ (the production cascade's in es_cascade.cu; for counting and scalar launches
+// sorted inner ring, carry-split keys and buckets, ring-1 residue table, ring-2 delta table and
+// word-mask phase tables), uploads a table set when a launch first needs it, and drives
 // single-plan launches (the reference GpuSieve._launch surface) and persistent batch launches
 // with CUDA-graph replay.  No exception crosses the ABI: every entry point returns an int.
 #include <cuda_runtime.h>

@@ -34,11 +34,11 @@
 // ready warps (k = 300, 2^34 positions: 1469 against 1369 us), 24 at 80 spill in wide rings (k = 379:
 // 2209 against 1842 us).
 //
-// What bounds it: shared-memory wavefronts (l1tex 78 to 83 % busy) and instruction issue (63 % at
-// k = 300).  Through the drop-in calls, against the caller's cascade by word-mask or pair tables
-// (es_scan_kernel.cuh): k = 300, 2^34 positions 3068 -> 1559 us, 2^30 positions 320 -> 197 us; the
-// three-word k = 379 wheel, 2^34 positions, 5500 -> 1940 us; both k = 390 wheels, 2^35 positions
-// each, 17,068 -> 6297 us (their caller-order tables, 1.75 MB per wheel, came through L2).
+// What bounds it: shared-memory wavefronts (l1tex 82 to 90 % busy), then the ALU pipe (66 to 75 %) and
+// instruction issue (60 to 70 %).  Through the drop-in calls, against the caller's cascade by word-mask
+// or pair tables (es_scan_kernel.cuh): k = 300, 2^34 positions 3060 -> 1348 us, 2^30 positions 318 -> 153
+// us; the three-word k = 379 wheel, 2^34 positions, 5502 -> 1754 us; both k = 390 wheels, 2^35 positions
+// each, 17,050 -> 5585 us (their caller-order tables, 1.75 MB per wheel, came through L2).
 #pragma once
 #include "es_scan_kernel.cuh"
 

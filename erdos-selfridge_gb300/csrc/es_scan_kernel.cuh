@@ -1,6 +1,8 @@
-// The scan kernel of the GB300 Erdős–Selfridge CRT-wheel sieve (sm_103a), as a template that
-// es_scan_wm.cu / es_scan_wmc.cu, es_scan_pair.cu and es_scan_sc.cu instantiate (compiled in
-// parallel); es_scan.cu holds the dispatch, the min-reduction and the peak probe.
+// The scan kernel of the GB300 Erdős–Selfridge CRT-wheel sieve (sm_103a) in the caller's cascade
+// order, as a template that es_scan_wmc.cu, es_scan_pair.cu, es_scan_sm.cu, es_scan_sp.cu (launches
+// that count filter stages) and es_scan_sc.cu (the scalar layout) instantiate; es_scan.cu holds the
+// dispatch, the min-reduction and the peak probe.  Launches that count no stages run the production
+// kernel (es_prod_kernel.cuh) in every other layout.
 //
 // What one launch computes (semantics of the reference kernel, sieve/gpu_sieve_v9.py:240-330,
 // sieve/gpu_sieve_v11.py:250-354, sieve/es_word_masks.py:39-92): for every work item (a plan,

@@ -3,7 +3,8 @@
 Chooses, per plan (or per batch), the fastest of: threads per CTA, strip depth (at most `strip`
 ring-1 cycles per lane per work unit: one balanced window of ring-2 digits), the table layout
 (word masks or pair tables, through L1 or staged in shared memory, or scalar) and the number of
-filters evaluated in the inner-ring stage.  None of
+filters evaluated in the inner-ring stage.  Launches that count no stages take the layout only
+where it is scalar, and their inner tables from the library's own cascade.  None of
 these changes which candidates pass; the tuner only times.  Search: coordinate descent from the
 default shape over one parameter at a time, each candidate timed with CUDA events on a probe
 range (median of a few launches).  Results are cached in a JSON file keyed by the plan (k,

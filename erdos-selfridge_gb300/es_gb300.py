@@ -44,14 +44,15 @@ from es_plan import Plan as _PlanBase  # noqa: E402
 from es_plan import TUNABLES as _PLAN_TUNABLES  # noqa: E402
 
 # Engine tunables on top of the planner's (sieve/gpu_sieve_v9.py:98-120).  Launch shape and
-# table layout never change which candidates pass.
+# table layout never change which candidates pass; the layout (but for "scalar") matters only to
+# launches that count stages.
 TUNABLES = dict(_PLAN_TUNABLES)
 TUNABLES.update({
     "chunk_log2": 34,        # positions per _launch chunk issued by scan_block
     "layout": "auto",        # "auto" (by table bytes) | "wordmask" | "pair" | "smem" | "scalar"
     "threads": 512,          # CTA size
     "strip": 8,              # at most this many ring-1 cycles per lane per warp-unit
-    "smem_kb": 0,            # accepted, no effect (phase tables are read through L1)
+    "smem_kb": 0,            # accepted, no effect (a launch sizes its own shared memory)
     "ctas_per_sm": 4,
     "count_stages": 0,       # per-filter-stage pass counts (es_stage_counts needs 1)
     "search_batch_log2": 34, # positions per multi-block search launch

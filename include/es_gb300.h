@@ -37,6 +37,10 @@ extern "C" {
 #define ES_ERR_STATE (-6)     /* call out of order (e.g. results before a launch) */
 #define ES_ERR_NODEV (-7)     /* no CUDA device / device is not sm_103 */
 
+/* How a launch that counts stages (es_tune.count_stages = 1) reads its filters.  A launch that counts
+ * none finds the same survivors with a cascade of the library's own choice, whose tables always lie
+ * in shared memory: of the layouts below only ES_LAYOUT_SCALAR makes a difference to it.  (A plan
+ * whose tables do not fit shared memory runs its uncounted launches in the scalar layout.) */
 #define ES_LAYOUT_WORDMASK 0  /* phase word-mask tables: 32 candidates per load */
 #define ES_LAYOUT_SCALAR 1    /* per-candidate incremental residue + bit-table test */
 #define ES_LAYOUT_PAIR 2      /* word-mask tables with each phase's wrapped row beside it: one
@@ -85,12 +89,16 @@ typedef struct es_plan_desc {
  * changes which candidates pass. */
 typedef struct es_tune {
     uint32_t layout;        /* ES_LAYOUT_WORDMASK, _SCALAR, _PAIR, _SMEM, _SMEM_PAIR or _AUTO */
-    uint32_t mask_filters;  /* filters in the inner-ring stage, 1..ES_MAX_MASK_FILTERS */
-    uint32_t threads;       /* CTA size, multiple of 32 in [64, 512] */
+    uint32_t mask_filters;  /* filters in the inner-ring stage, 1..ES_MAX_MASK_FILTERS; inner tables
+                               of an uncounted launch, which takes at most 6, and one more than
+                               asked for where many candidates pass */
+    uint32_t threads;       /* CTA size, multiple of 32 in [64, 512]; an uncounted launch of 512
+                               runs 640 */
     uint32_t strip;         /* at most this many ring-1 cycles per thread per work unit: the
                                lanes of a warp take 32 consecutive ring-2 rows over one of
                                ceil(r2 / strip) balanced windows of ring-2 digits; lists and
-                               plans without a ring 2 take `strip` consecutive entries */
+                               plans without a ring 2 take `strip` consecutive entries; short
+                               launches take fewer, in whole waves of units */
     uint32_t smem_kb;       /* accepted, no effect (the staged layouts size their own shared
                                memory) */
     uint32_t ctas_per_sm;   /* persistent grid = SM count * ctas_per_sm */
@@ -218,7 +226,7 @@ int es_batch_destroy(es_batch* b);
  * (*d_count) exceeded out_cap and records were dropped: the minimum is then unknown, d_min[1]
  * is the least block holding a good survivor (exact; UINT64_MAX when none) and the caller
  * retries with fewer blocks or a larger buffer.  Scratch lives in a file-scope device
- * array sized for ES_STATIC_MAX_BLOCKS blocks (about 57 KB, held by every GPU that loads the
+ * array sized for ES_STATIC_MAX_BLOCKS blocks (about 60 KB, held by every GPU that loads the
  * library until exit); larger n_blocks is rejected with ES_ERR_RANGE.  Stage counts are not
  * accumulated.  The first call on a device looks up the scratch array's device address.  The
  * call must not be made while `stream` is capturing (it returns ES_ERR_STATE): its small
