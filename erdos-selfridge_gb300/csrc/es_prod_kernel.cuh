@@ -36,9 +36,9 @@
 //
 // What bounds it: shared-memory wavefronts (l1tex 82 to 90 % busy), then the ALU pipe (66 to 75 %) and
 // instruction issue (60 to 70 %).  Through the drop-in calls, against the caller's cascade by word-mask
-// or pair tables (es_scan_kernel.cuh): k = 300, 2^34 positions 3060 -> 1348 us, 2^30 positions 318 -> 153
-// us; the three-word k = 379 wheel, 2^34 positions, 5502 -> 1754 us; both k = 390 wheels, 2^35 positions
-// each, 17,050 -> 5585 us (their caller-order tables, 1.75 MB per wheel, came through L2).
+// or pair tables (es_scan_kernel.cuh): k = 300, 2^34 positions 3069 -> 1376 us, 2^30 positions 319 -> 155
+// us; the three-word k = 379 wheel, 2^34 positions, 5506 -> 1752 us; both k = 390 wheels, 2^35 positions
+// each, 17,024 -> 5585 us (their caller-order tables, 1.75 MB per wheel, came through L2).
 #pragma once
 #include "es_scan_kernel.cuh"
 
