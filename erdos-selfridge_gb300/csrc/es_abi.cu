@@ -660,10 +660,10 @@ static int build_caller(es_ctx* c) {
 }
 
 // The host image of the production cascade with F inner tables.
-static void prod_image(const es_ctx* c, uint32_t F, EsProdImage& img) {
+static void prod_image(const es_ctx* c, uint32_t F, EsProdImage& img, double max_rate = 1.0) {
     // beside the staged tables: the static shared memory, and the slots of the largest CTA's warps
     es_prod_image(c->plan, c->geo, F,
-                  (uint32_t)g_dev.smem_optin - 2048u - ES_PROD_THREADS / 32u * ES_QUEUE_BYTES, img);
+                  (uint32_t)g_dev.smem_optin - 2048u - ES_PROD_THREADS / 32u * ES_QUEUE_BYTES, img, max_rate);
 }
 
 static int upload_prod(es_ctx* c, uint32_t F, EsProdImage& img) {
@@ -689,9 +689,10 @@ static int ensure_tables(es_ctx* c, const es_tune& t, bool own) {
         uint32_t F = prod_tables(t);
         if (own && !c->own_tables[F]) {
             EsProdImage img;
-            prod_image(c, F, img);
             uint32_t use = F;
-            if (F < ES_PMAX && 32.0 * c->geo.r0 * img.rate > kMoreTables) prod_image(c, use = F + 1, img);
+            const double most = F < ES_PMAX ? kMoreTables / (32.0 * c->geo.r0) : 1.0;
+            prod_image(c, F, img, most);
+            if (img.rate > most) prod_image(c, use = F + 1, img);
             if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)
                 if (int e = upload_prod(c, use, img)) return e;
             c->own_tables[F] = use;

@@ -397,7 +397,8 @@ uint32_t table_bytes(uint64_t R, size_t smem_bytes, size_t small_bytes) {
 }  // namespace
 
 // Tables of the production cascade with F inner tables (es_cascade.h, es_prod_kernel.cuh).
-void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t smem_bytes, EsProdImage& out) {
+void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t smem_bytes, EsProdImage& out,
+                   double max_rate) {
     EsInst& I = out.inst;
     I = geo;
     const u128 M = P.M;
@@ -422,6 +423,7 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     const EsCascade C = es_choose_cascade(P, F, row_bytes, pair, table_bytes(geo.n_outer * r0, smem_bytes, S.b.size()));
 
     out.rate = C.rate;
+    if (C.rate > max_rate) return;
 
     // ---- entries: inner tables, residue stage, tail ----------------------------------------
     std::vector<EsCascadeEntry>& entries = out.entries;

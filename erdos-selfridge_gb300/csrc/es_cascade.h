@@ -126,5 +126,7 @@ int es_check_desc(const es_plan_desc& d, std::string& why);
 int es_parse_plan(const es_plan_desc& d, EsHostPlan& P, EsInst& geo, std::string& why);
 
 // The image of the production cascade with F inner tables; smem_bytes: shared memory for the small
-// block and the inner tables together.
-void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t smem_bytes, EsProdImage& out);
+// block and the inner tables together.  Where more than max_rate of the candidates would pass those
+// tables, only out.rate is set.
+void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t smem_bytes, EsProdImage& out,
+                   double max_rate = 1.0);
