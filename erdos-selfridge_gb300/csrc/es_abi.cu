@@ -541,7 +541,10 @@ static int upload_set(es_ctx* c, TableSet& T, const std::vector<unsigned char>& 
     I.ring_off = reinterpret_cast<const uint32_t*>(arena + a_roff);
     I.radix = reinterpret_cast<const uint32_t*>(arena + a_radix);
     memcpy(&img[a_inst], &I, sizeof(EsInst));
-    const cudaError_t ce = cudaMemcpy(arena, img.data(), aoff, cudaMemcpyHostToDevice);
+    // the copy may still be on its way to the device when it returns, and no stream that reads the
+    // tables is ordered after the default stream: wait for it
+    cudaError_t ce = cudaMemcpy(arena, img.data(), aoff, cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
     if (ce != cudaSuccess) {
         cudaFree(arena);
         return cuda_fail(ce, "table upload");
@@ -744,8 +747,9 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     if (ce == cudaSuccess) ce = cudaMalloc(&c->d_counts, 8ull * std::max<uint32_t>(nf, 1));
     if (ce == cudaSuccess) ce = cudaMalloc(&c->d_surv_n, 8ull * 8);
     if (ce == cudaSuccess) ce = cudaHostAlloc(&c->h_pin, 8ull * 8, cudaHostAllocDefault);
-    if (ce == cudaSuccess) ce = cudaMemset(c->d_counts, 0, 8ull * std::max<uint32_t>(nf, 1));
-    if (ce == cudaSuccess) ce = cudaMemset(c->d_surv_n, 0, 8ull * 8);
+    // on the launches' own stream: nothing orders it after the default stream
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(c->d_counts, 0, 8ull * std::max<uint32_t>(nf, 1), c->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(c->d_surv_n, 0, 8ull * 8, c->stream);
     if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "context setup"); }
     // d_surv_n block: [0] survivor count, [1] unit counter, [2] CTAs done, [3..6] group min
     c->d_unit = c->d_surv_n + 1;
@@ -965,7 +969,8 @@ int es_launch_list(es_ctx* c, const uint64_t* outer, uint64_t n) {
         ES_CUDA(cudaMalloc(&c->d_list, 8ull * n), "cudaMalloc(list)");
         c->list_cap = n;
     }
-    ES_CUDA(cudaMemcpy(c->d_list, outer, 8ull * n, cudaMemcpyHostToDevice), "copy list");
+    ES_CUDA(cudaMemcpyAsync(c->d_list, outer, 8ull * n, cudaMemcpyHostToDevice, c->stream), "copy list");
+    ES_CUDA(cudaStreamSynchronize(c->stream), "copy list");   // the caller's array has been read
     return ctx_launch(c, 0, n, c->d_list);
 }
 

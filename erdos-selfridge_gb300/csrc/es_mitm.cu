@@ -564,7 +564,10 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     if (ce == cudaSuccess) ce = cudaMemcpy(m->d_slices, slices.data(), sizeof(uint4) * slices.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_merged, 4ull * merged.size());
     if (ce == cudaSuccess) ce = cudaMemcpy(m->d_merged, merged.data(), 4ull * merged.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemset(m->d_cnt, 0, 8ull * 4);
+    // the scans' stream is not ordered after the default stream: wait for the copies, and zero the
+    // counters on the former
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(m->d_cnt, 0, 8ull * 4, m->stream);
     if (ce != cudaSuccess) {
         es_mitm_destroy(m);
         return mcuda(ce, "MITM setup");
