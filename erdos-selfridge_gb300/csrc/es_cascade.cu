@@ -187,6 +187,7 @@ double value_of(const std::vector<uint32_t>& proj, uint32_t d, uint32_t g, std::
 struct Slot {
     uint32_t n, part[3];
     double rows, value;
+    uint64_t bytes;   // of its rows, padded as es_prod_image lays them out
 };
 
 }  // namespace
@@ -223,8 +224,10 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     if (parts.size() > 48) parts.resize(48);
     auto rows = [&](uint32_t d) {
         const uint32_t m = (uint32_t)(P.M % d);
-        return (double)es_table_rows(d, std::max(m ? d - m : 0u, d / 4u), pair);   // (room for spread_of)
+        return es_planned_rows(d, m ? d - m : 0u, pair);
     };
+    auto bytes_of = [&](uint32_t n) { return (uint64_t)es_align_up((uint64_t)n * row_bytes, 16); };
+    const uint64_t fill_bytes = bytes_of(es_table_rows(2, 1, pair));
     std::vector<Slot> slots;
     const uint32_t np = (uint32_t)parts.size();
     auto add = [&](uint32_t n, uint32_t a, uint32_t b, uint32_t c) {
@@ -239,8 +242,8 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
             v += x.value;
         }
         if (d >= ES_MAX_Q || 2.0 * (double)d > budget) return;
-        const double r = rows((uint32_t)d);
-        if (r <= budget) slots.push_back(Slot{n, {a, b, c}, r, v});
+        const uint32_t r = rows((uint32_t)d);
+        if (bytes_of(r) <= table_bytes) slots.push_back(Slot{n, {a, b, c}, (double)r, v, bytes_of(r)});
     };
     for (uint32_t a = 0; a < np; ++a) {
         add(1, a, 0, 0);
@@ -255,18 +258,21 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     // by value minus a price per row, over a range of prices.
     std::vector<uint32_t> best;
     double best_value = -1.0;
+    uint64_t spare = 0;
     std::vector<uint8_t> used(nf);
     for (int step = 0; step <= 28; ++step) {
         const double price = step == 0 ? 0.0 : std::exp2(-4.0 - 0.5 * step) * 4000.0 / std::max(budget, 1.0);
         std::fill(used.begin(), used.end(), (uint8_t)0);
         std::vector<uint32_t> pick;
-        double sum = 0.0, left = budget;
+        double sum = 0.0;
+        uint64_t left = table_bytes;
         while (pick.size() < F) {
+            const uint64_t later = fill_bytes * (F - 1 - pick.size());   // the other tables are fill-ins at least
             int at = -1;
             double score = 0.0;
             for (uint32_t i = 0; i < slots.size(); ++i) {
                 const Slot& s = slots[i];
-                if (s.rows > left) continue;
+                if (s.bytes + later > left) continue;
                 const double x = s.value - price * s.rows;
                 if (x <= score) continue;
                 bool free = true;
@@ -279,13 +285,15 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
             if (at < 0) break;
             const Slot& s = slots[at];
             for (uint32_t j = 0; j < s.n; ++j) used[parts[s.part[j]].f] = 1;
-            left -= s.rows;
+            left -= s.bytes;
             sum += s.value;
             pick.push_back((uint32_t)at);
         }
         if (sum > best_value) {
             best_value = sum;
             best = pick;
+            const uint64_t fills = fill_bytes * (F - pick.size());
+            spare = left > fills ? left - fills : 0;
         }
     }
     std::stable_sort(best.begin(), best.end(), [&](uint32_t a, uint32_t b) { return slots[a].value > slots[b].value; });
@@ -305,6 +313,7 @@ EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes,
     }
     C.inner.resize(F);
     C.rate = std::exp(-std::max(best_value, 0.0));
+    C.spare = spare;
     std::vector<uint32_t> order;
     for (uint32_t f = 0; f < nf; ++f)
         if (!settled[f]) order.push_back(f);
@@ -351,7 +360,9 @@ std::vector<u128> sample_rows(const EsHostPlan& P, uint64_t R, uint64_t& seed) {
     return b3;
 }
 
-uint32_t spread_of(const std::vector<u128>& b3, uint64_t& seed, uint32_t d, uint32_t corr, bool pair, uint32_t row_bytes) {
+// reach: how far away the wrapped row may lie, where it is a row of its own.
+uint32_t spread_of(const std::vector<u128>& b3, uint64_t& seed, uint32_t d, uint32_t corr, bool pair, uint32_t row_bytes,
+                   uint32_t reach) {
     if (row_bytes > 16u || d < 8u || b3.empty()) return 1u;
     const uint32_t lanes = 128u / row_bytes;   // per wavefront at best; rows across all banks
     std::vector<uint32_t> res(b3.size()), shift(2 * kSampleWarps);   // shifts: the other rings' terms
@@ -362,8 +373,7 @@ uint32_t spread_of(const std::vector<u128>& b3, uint64_t& seed, uint32_t d, uint
         const uint32_t u = t == 0 ? 1u : (uint32_t)(xorshift(seed) % (d - 1u)) + 1u;
         if (gcd32(u, d) != 1u) continue;
         const uint32_t c = (uint32_t)((uint64_t)u * corr % d);
-        // where the wrapped row is a row of its own it must not need more of them than were planned
-        if (!pair && t && std::min(c, d - c) > std::max(std::min(corr, d - corr), d / 4u)) continue;
+        if (!pair && t && std::min(c, d - c) > reach) continue;
         uint32_t cost = 0;
         for (uint32_t w = 0; w < kSampleWarps; ++w)
             for (uint32_t from = 0; from < 32; from += lanes) {
@@ -443,6 +453,7 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     };
     uint64_t seed = 0x9e3779b97f4a7c15ull;
     const std::vector<u128> sample = sample_rows(P, geo.n_outer * r0, seed);
+    uint64_t spare = C.spare;
     for (const std::vector<EsPart>& table : C.inner) {
         if (table.empty()) {
             I.tab_mul[entries.size()] = 1;
@@ -462,9 +473,15 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         // residues are kept times the table's multiplier: limb weights (`off`, which has no use here, is
         // the lowest limb's), wrap correction and block constant
         EsFilterC c = es_filter_consts(M, e.q, 0);
-        const uint32_t u = spread_of(sample, seed, e.q, c.corr, pair, row_bytes);
+        // the wrapped row no further than its distance with u = 1 or d / 4, and within the bytes left
+        auto bytes_of = [&](uint32_t rows) { return (uint64_t)es_align_up((uint64_t)rows * row_bytes, 16); };
+        const uint64_t room = bytes_of(es_planned_rows(e.q, c.corr, pair)) + spare;
+        const uint32_t near = std::min(c.corr, e.q - c.corr), most = std::max(near, e.q / 4u);
+        const uint32_t reach = (uint32_t)std::min<uint64_t>(most, room / row_bytes - (2u * e.q - 1u));
+        const uint32_t u = spread_of(sample, seed, e.q, c.corr, pair, row_bytes, reach);
         I.tab_mul[entries.size()] = u;
         for (uint32_t* w : {&c.corr, &c.w1, &c.w2, &c.w3}) *w = (uint32_t)((uint64_t)*w * u % e.q);
+        spare = room - bytes_of(es_table_rows(e.q, c.corr, pair));
         c.off = u;
         for (EsCascadeEntry::Part& p : e.parts) p.unit = (uint32_t)((uint64_t)p.unit * u % e.q);
         entries.push_back(e);

@@ -48,6 +48,7 @@ struct EsCascade {
     std::vector<int> residue;
     std::vector<uint32_t> tail;
     double rate = 1.0;    // share of the candidates that pass the inner tables
+    uint64_t spare = 0;   // bytes of table_bytes that the planned rows leave
 };
 
 // Inner rings of one word have the masks of a phase and of the phase a wrap past M selects side by
@@ -67,7 +68,14 @@ inline uint32_t es_table_rows(uint32_t d, uint32_t corr, bool pair) {
 // The admissible set of a filter (packed bits of q residues) as bytes, projected to d | q.
 void es_project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_t>& out);
 
-// Chooses F inner tables whose rows of row_bytes bytes fit table_bytes in all.
+// Rows kept for the table of modulus d when it is chosen, before its multiplier u is: the wrapped row
+// then lies u corr away, at the nearer side.
+inline uint32_t es_planned_rows(uint32_t d, uint32_t corr, bool pair) {
+    return es_table_rows(d, corr > d / 4u ? corr : d / 4u, pair);
+}
+
+// Chooses F inner tables whose planned rows of row_bytes bytes, each table padded to 16 bytes, fit
+// table_bytes in all.  Fill-ins count too; nothing but they can exceed table_bytes.
 EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes);
 
 // An entry of a production cascade: the residue of n mod q is needed.  Its block constant follows

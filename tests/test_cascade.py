@@ -136,6 +136,21 @@ def test_tables_fit_the_room_they_are_given():
             assert info.small_bytes + 4 * info.tab_words <= max(room, info.small_bytes) + 6 * 5 * info.row_bytes
 
 
+def test_tables_never_exceed_their_room():
+    """Whatever multipliers are chosen: not the room, and not what a block of its length may spend on
+    tables.  (The wheels' wrap corrections lie anywhere below their tables' moduli.)"""
+    for spec in PLANS + [(k, None) for k in (192, 212, 258, 294)] + [(382, "primary"), (392, "primary"),
+                                                                     (400, "confirmation")]:
+        P = _plan(spec)
+        most = (12 if P.R < 1 << 22 else 48 if P.R < 1 << 28 else 144) * 1024
+        for tables in range(1, 7):
+            for room in (64 * 1024, 180 * 1024):
+                info, _, _, _ = image(P, tables, room)
+                fill_ins = tables * -(-4 * info.row_bytes // 16) * 16   # four rows each, whatever the room
+                left = max(0, room - info.small_bytes)
+                assert 4 * info.tab_words <= max(min(left, most), fill_ins), (spec, tables, room)
+
+
 # ------------------------------------------------------------------ GPU
 def _ranges(P):
     outer = P.R // P.radix[0]
