@@ -73,10 +73,15 @@ constexpr uint32_t kMitmThreads = 512;
 constexpr uint32_t kMitmChunk = 16;  // values of b per claimed unit, at most (two lanes each for its range)
 constexpr uint32_t kMitmQueue = 64;  // candidates queued per warp
 constexpr uint32_t kMitmTables = 2;  // merged bit tables ahead of the cascade
-constexpr uint32_t kMitmTableBits = 1u << 18;   // bits of both
+// Bits of both: 32 KB less a word that each may round up to, so that with 16 KB of queues the kernel stays
+// within the 48 KB of shared memory that need no opt-in.
+constexpr uint32_t kMitmTableBits = (1u << 18) - 64u;
 constexpr uint64_t kMitmGroup = 1u << 17;       // rings are grouped while their sums stay within this
 constexpr uint64_t kMitmRange = 64;             // values of A per b and slice, at least
 constexpr uint32_t kMitmSlicesLog2 = 12;        // slices at most
+
+static_assert(kMitmThreads / 32u * kMitmQueue * sizeof(uint4) + (kMitmTableBits / 32u + kMitmTables) * 4u <= 48u << 10,
+              "queues and merged tables exceed what a launch has without an opt-in");
 
 struct MitmParams {
     const uint4* S2;              // sorted small half: {lo.x, lo.y, hi.x, hi.y} per entry
@@ -480,7 +485,7 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     hp.bit_off.assign(1, 0);
     for (uint32_t f = 0; f < d->n_filters; ++f) hp.bit_off.push_back(hp.bit_off.back() + (hp.q[f] + 31) / 32);
     if (d->n_filters) hp.allowed.assign(d->allowed, d->allowed + words);
-    // (rows of one byte, two per residue: kMitmTableBits residues in all)
+    // (rows of one byte, two per residue: kMitmTableBits residues in all, padded to 16 rows a table)
     const EsCascade cascade = es_choose_cascade(hp, kMitmTables, 1, true, 2u * kMitmTableBits);
     std::vector<uint32_t> merged;
     std::vector<uint8_t> one;
