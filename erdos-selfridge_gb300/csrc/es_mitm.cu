@@ -540,9 +540,10 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     std::sort(a_index.begin(), a_index.end(), [&](uint32_t x, uint32_t y) { return A[x] < A[y]; });
     std::vector<u128m> a_sorted(A.size());
     for (size_t i = 0; i < A.size(); ++i) a_sorted[i] = A[a_index[i]];
-    // slices of [0, M): a power of two of them, none so thin that a b's range of A is a few values
+    // slices of [0, M): a power of two of them, none so thin that a b's range of A is a few values, and
+    // none empty (an end that is not above the start goes round, so an empty one would hold all of A)
     uint32_t sl = 0;
-    while (sl < kMitmSlicesLog2 && (A.size() >> (sl + 1)) >= kMitmRange) ++sl;
+    while (sl < kMitmSlicesLog2 && (A.size() >> (sl + 1)) >= kMitmRange && (M >> (sl + 1)) != 0) ++sl;
     std::vector<u128m> slices;
     for (uint64_t i = 0; i < (1ull << sl); ++i) slices.push_back((M >> sl) * i);
     slices.push_back(M);

@@ -61,3 +61,16 @@ def test_gpu_filters_of_large_moduli(native, wide):
     for B in (wide.M, wide.M // 3):
         assert e.scan(B) == wide.brute(B)
     e.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [2, 3, 7, 8, 29])
+def test_gpu_modulus_below_the_slices(native, M):
+    """Fewer residues than the value-ordered sweep of S1 would have slices: every s1 counts once."""
+    import es_mitm
+    h = _random(M, [700, 3], [5, 2], [5], M)
+    e = es_mitm.MitmEngine(h)
+    for B in range(1, M + 1):
+        assert e.scan(B) == h.brute(B)
+    assert e.scan(M, 11, 901)[1] == 890 * 10   # B = M: every pair
+    e.close()
