@@ -453,7 +453,26 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
     };
     uint64_t seed = 0x9e3779b97f4a7c15ull;
     const std::vector<u128> sample = sample_rows(P, geo.n_outer * r0, seed);
-    uint64_t spare = C.spare;
+    // The tables' multipliers: a wrapped row no further than its distance with u = 1 or d / 4; where the
+    // tables then exceed their room, also within the bytes that those before it leave.
+    std::vector<uint32_t> mul(F, 1u);
+    for (const bool within : {false, true}) {
+        uint64_t s = seed;
+        int64_t spare = (int64_t)C.spare;
+        for (uint32_t i = 0; i < F; ++i) {
+            if (C.inner[i].empty()) continue;
+            uint32_t d = 1;
+            for (const EsPart& p : C.inner[i]) d *= p.d;
+            const uint32_t corr = (d - es_mod(M, d)) % d;
+            auto bytes_of = [&](uint32_t c) { return (int64_t)es_align_up((uint64_t)c * row_bytes, 16); };
+            const int64_t room = bytes_of(es_planned_rows(d, corr, pair)) + spare;
+            uint32_t reach = std::max(std::min(corr, d - corr), d / 4u);
+            if (within) reach = (uint32_t)std::min<uint64_t>(reach, (uint64_t)room / row_bytes - (2u * d - 1u));
+            mul[i] = spread_of(sample, s, d, corr, pair, row_bytes, reach);
+            spare = room - bytes_of(es_table_rows(d, (uint32_t)((uint64_t)corr * mul[i] % d), pair));
+        }
+        if (spare >= 0) break;
+    }
     for (const std::vector<EsPart>& table : C.inner) {
         if (table.empty()) {
             I.tab_mul[entries.size()] = 1;
@@ -473,15 +492,9 @@ void es_prod_image(const EsHostPlan& P, const EsInst& geo, uint32_t F, uint32_t 
         // residues are kept times the table's multiplier: limb weights (`off`, which has no use here, is
         // the lowest limb's), wrap correction and block constant
         EsFilterC c = es_filter_consts(M, e.q, 0);
-        // the wrapped row no further than its distance with u = 1 or d / 4, and within the bytes left
-        auto bytes_of = [&](uint32_t rows) { return (uint64_t)es_align_up((uint64_t)rows * row_bytes, 16); };
-        const uint64_t room = bytes_of(es_planned_rows(e.q, c.corr, pair)) + spare;
-        const uint32_t near = std::min(c.corr, e.q - c.corr), most = std::max(near, e.q / 4u);
-        const uint32_t reach = (uint32_t)std::min<uint64_t>(most, room / row_bytes - (2u * e.q - 1u));
-        const uint32_t u = spread_of(sample, seed, e.q, c.corr, pair, row_bytes, reach);
+        const uint32_t u = mul[entries.size()];
         I.tab_mul[entries.size()] = u;
         for (uint32_t* w : {&c.corr, &c.w1, &c.w2, &c.w3}) *w = (uint32_t)((uint64_t)*w * u % e.q);
-        spare = room - bytes_of(es_table_rows(e.q, c.corr, pair));
         c.off = u;
         for (EsCascadeEntry::Part& p : e.parts) p.unit = (uint32_t)((uint64_t)p.unit * u % e.q);
         entries.push_back(e);
