@@ -198,6 +198,25 @@ void es_project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_
         for (uint32_t j = 0; j < d; ++j) out[j] |= (bits[(from + j) >> 5] >> ((from + j) & 31u)) & 1u;
 }
 
+void es_and_periodic(const uint32_t* bits, uint32_t q, uint32_t d, uint32_t n, uint32_t* out) {
+    std::vector<uint32_t> proj;
+    project_bits(bits, q, d, proj);
+    // one period and the 32 bits after it, so that a word can start anywhere in the period
+    const uint32_t words = (d + 31u) / 32u + 1u;
+    std::vector<uint32_t> two(words, 0u);
+    for (uint32_t at = 0; at < 32u * words; at += d)
+        for (uint32_t w = 0; w < proj.size(); ++w) {
+            const uint32_t to = at + 32u * w;
+            if (to >= 32u * words) break;
+            two[to / 32u] |= proj[w] << (to % 32u);
+            if (to % 32u && to / 32u + 1u < words) two[to / 32u + 1u] |= proj[w] >> (32u - to % 32u);
+        }
+    for (uint32_t w = 0, at = 0; w < (n + 31u) / 32u; ++w) {
+        out[w] &= bits_at(two.data(), words, at);
+        at = (at + 32u) % d;
+    }
+}
+
 EsCascade es_choose_cascade(const EsHostPlan& P, uint32_t F, uint32_t row_bytes, bool pair, uint32_t table_bytes) {
     const uint32_t nf = (uint32_t)P.q.size();
     const double budget = (double)(table_bytes / row_bytes);

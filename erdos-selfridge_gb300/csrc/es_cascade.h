@@ -68,6 +68,10 @@ inline uint32_t es_table_rows(uint32_t d, uint32_t corr, bool pair) {
 // The admissible set of a filter (packed bits of q residues) as bytes, projected to d | q.
 void es_project(const uint32_t* bits, uint32_t q, uint32_t d, std::vector<uint8_t>& out);
 
+// Packed residues 0 .. n-1 (whole words): those whose residue mod d is not in the filter's admissible set
+// projected to d | q are cleared.
+void es_and_periodic(const uint32_t* bits, uint32_t q, uint32_t d, uint32_t n, uint32_t* out);
+
 // Rows kept for the table of modulus d when it is chosen, before its multiplier u is: the wrapped row
 // then lies u corr away, at the nearer side.
 inline uint32_t es_planned_rows(uint32_t d, uint32_t corr, bool pair) {

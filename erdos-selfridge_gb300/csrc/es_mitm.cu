@@ -76,7 +76,12 @@ constexpr uint32_t kMitmTables = 2;  // merged bit tables ahead of the cascade
 // Bits of both: 32 KB less a word that each may round up to, so that with 16 KB of queues the kernel stays
 // within the 48 KB of shared memory that need no opt-in.
 constexpr uint32_t kMitmTableBits = (1u << 18) - 64u;
-constexpr uint64_t kMitmGroup = 1u << 17;       // rings are grouped while their sums stay within this
+// Rings are grouped while their sums stay within this, and A's within a quarter of S1 as well: sorting a
+// large A costs more than a short scan gains from it.  Creation and one scan, A within 2^17 alone and
+// within a quarter of S1: k = 90 (S1 90,720) 4.19 + 0.080 and 2.53 + 0.080 ms, k = 100 (119,808) 4.89 +
+// 0.092 and 2.86 + 0.083, k = 130 (7.4 million, the same A) 9.50 + 0.263 and 9.45 + 0.270.
+constexpr uint64_t kMitmGroup = 1u << 17;
+constexpr uint64_t kMitmShare = 4;
 constexpr uint64_t kMitmRange = 64;             // values of A per b and slice, at least
 constexpr uint32_t kMitmSlicesLog2 = 12;        // slices at most
 
@@ -280,15 +285,7 @@ __global__ void __launch_bounds__(kMitmThreads) es_mitm_kernel(const __grid_cons
 struct es_mitm {
     cudaStream_t stream = nullptr;
     MitmParams P{};
-    uint4* d_S2 = nullptr;
-    uint32_t* d_dir = nullptr;
-    uint4* d_sums1 = nullptr;
-    EsFilterC* d_filt = nullptr;
-    uint32_t* d_allowed = nullptr;
-    uint32_t* d_merged = nullptr;
-    uint4* d_A = nullptr;
-    uint32_t* d_a_index = nullptr;
-    uint4* d_slices = nullptr;
+    unsigned char* tables = nullptr;   // every array that scans read, in one allocation
     uint4* d_out = nullptr;
     unsigned long long* d_cnt = nullptr;
     unsigned long long* h_cnt = nullptr;
@@ -296,20 +293,35 @@ struct es_mitm {
     int grid = 0;
 };
 
+namespace {
+
+// Sorts items by their keys (below 2^bits): scattered to about one bucket per item (at most
+// 2^16) by the keys' top bits, then the buckets one by one.
+template <class T, class Key>
+void bucket_sort(std::vector<T>& v, uint32_t bits, const Key& key) {
+    const size_t n = v.size();
+    uint32_t P = 0;
+    while (P < std::min(bits, 16u) && ((size_t)1 << P) < n) ++P;
+    const uint32_t sh = bits - P;
+    std::vector<uint32_t> at(((size_t)1 << P) + 1, 0);   // bucket p's items end at at[p], start at at[p - 1]
+    for (const T& x : v) ++at[(size_t)(key(x) >> sh) + 1];
+    for (size_t p = 1; p < at.size(); ++p) at[p] += at[p - 1];
+    std::vector<T> out(n);
+    for (const T& x : v) out[at[(size_t)(key(x) >> sh)]++] = x;
+    for (size_t p = 0, from = 0; p + 1 < at.size(); from = at[p++])
+        if (at[p] - from > 1)
+            std::sort(out.begin() + from, out.begin() + at[p], [&](const T& a, const T& b) { return key(a) < key(b); });
+    v.swap(out);
+}
+
+}  // namespace
+
 extern "C" {
 
 int es_mitm_destroy(es_mitm* m) {
     if (!m) return ES_OK;
     if (m->stream) cudaStreamSynchronize(m->stream);
-    cudaFree(m->d_S2);
-    cudaFree(m->d_dir);
-    cudaFree(m->d_sums1);
-    cudaFree(m->d_filt);
-    cudaFree(m->d_allowed);
-    cudaFree(m->d_merged);
-    cudaFree(m->d_A);
-    cudaFree(m->d_a_index);
-    cudaFree(m->d_slices);
+    cudaFree(m->tables);
     cudaFree(m->d_out);
     cudaFree(m->d_cnt);
     if (m->h_cnt) cudaFreeHost(m->h_cnt);
@@ -327,7 +339,7 @@ void parallel_sort(std::vector<u128m>& v, uint32_t bits) {
     const size_t n = v.size();
     const unsigned T = std::max(1u, std::min(64u, std::thread::hardware_concurrency()));
     if (n < (1u << 16) || T == 1 || bits == 0) {
-        std::sort(v.begin(), v.end());
+        bucket_sort(v, bits, [](u128m x) { return x; });
         return;
     }
     const uint32_t P = std::min<uint32_t>(12, bits);
@@ -488,26 +500,19 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     // (rows of one byte, two per residue: kMitmTableBits residues in all, padded to 16 rows a table)
     const EsCascade cascade = es_choose_cascade(hp, kMitmTables, 1, true, 2u * kMitmTableBits);
     std::vector<uint32_t> merged;
-    std::vector<uint8_t> one;
     for (uint32_t i = 0; i < kMitmTables; ++i) {
         uint32_t q = 1;
         for (const EsPart& p : cascade.inner[i]) q *= p.d;
         if (q == 1) q = 2;   // a fill-in that passes everything
         const uint32_t off = (uint32_t)merged.size();
-        std::vector<uint8_t> adm(q, 1);
-        for (const EsPart& p : cascade.inner[i]) {
-            es_project(hp.allowed.data() + hp.bit_off[p.f], hp.q[p.f], p.d, one);
-            for (uint32_t r = 0, x = 0; r < q; ++r) {
-                adm[r] &= one[x];
-                if (++x == p.d) x = 0;
-            }
-        }
-        merged.resize(off + (q + 31) / 32, 0u);
-        for (uint32_t r = 0; r < q; ++r) merged[off + (r >> 5)] |= (uint32_t)adm[r] << (r & 31u);
+        merged.resize(off + (q + 31) / 32, 0xffffffffu);
+        for (const EsPart& p : cascade.inner[i])
+            es_and_periodic(hp.allowed.data() + hp.bit_off[p.f], hp.q[p.f], p.d, q, &merged[off]);
         m->P.table[i] = es_filter_consts(M, q, off);
     }
     // ---- large half: sums over groups of consecutive rings; the first group is A, sorted -----------
     std::vector<u128m> A(1, 0), sums;
+    const uint64_t a_most = std::min(kMitmGroup, std::max<uint64_t>(n1 / kMitmShare, 1024));
     for (uint32_t j = 0, o = 0; j < d->n_rings1;) {
         uint64_t size = 1;
         const bool first = j == 0;
@@ -523,7 +528,7 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
             sum.swap(next);
             size *= r1[j];
             o += r1[j++];
-        } while (j < d->n_rings1 && size * r1[j] <= kMitmGroup);
+        } while (j < d->n_rings1 && size * r1[j] <= (first ? a_most : kMitmGroup));
         if (first) {
             A.swap(sum);
             continue;
@@ -535,11 +540,20 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
         sums.insert(sums.end(), sum.begin(), sum.end());
     }
     if (sums.empty()) sums.push_back(0);
-    std::vector<uint32_t> a_index(A.size());
-    for (size_t i = 0; i < A.size(); ++i) a_index[i] = (uint32_t)i;
-    std::sort(a_index.begin(), a_index.end(), [&](uint32_t x, uint32_t y) { return A[x] < A[y]; });
+    struct Sum {
+        u128m v;
+        uint32_t index;
+    };
+    std::vector<Sum> by_value(A.size());
+    for (size_t i = 0; i < A.size(); ++i) by_value[i] = Sum{A[i], (uint32_t)i};
+    // (the indices sorted by the values they stand for took 11 ms where this takes 3: 90,720 values)
+    bucket_sort(by_value, bits, [](const Sum& x) { return x.v; });
     std::vector<u128m> a_sorted(A.size());
-    for (size_t i = 0; i < A.size(); ++i) a_sorted[i] = A[a_index[i]];
+    std::vector<uint32_t> a_index(A.size());
+    for (size_t i = 0; i < A.size(); ++i) {
+        a_sorted[i] = by_value[i].v;
+        a_index[i] = by_value[i].index;
+    }
     // slices of [0, M): a power of two of them, none so thin that a b's range of A is a few values, and
     // none empty (an end that is not above the start goes round, so an empty one would hold all of A)
     uint32_t sl = 0;
@@ -549,27 +563,36 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     slices.push_back(M);
     static_assert(sizeof(u128m) == sizeof(uint4), "values are uploaded as they are (little endian)");
     cudaError_t ce = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_S2, sizeof(uint4) * S2.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_dir, 4ull * dir.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_sums1, sizeof(uint4) * sums.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_filt, sizeof(EsFilterC) * std::max<size_t>(fc.size(), 1));
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_allowed, 4ull * std::max<uint32_t>(words, 1));
+    // one allocation and three copies: S2, its directory, and the small arrays in one image
+    size_t total = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = total;
+        total = es_align_up(total + std::max<size_t>(bytes, 16), 256);
+        return at;
+    };
+    std::vector<unsigned char> small;
+    size_t small_at = 0;
+    auto put = [&](const void* src, size_t bytes) {
+        const size_t at = take(bytes);
+        small.resize(total - small_at, 0);
+        if (bytes) memcpy(&small[at - small_at], src, bytes);
+        return at;
+    };
+    const size_t o_S2 = take(sizeof(uint4) * S2.size()), o_dir = take(4 * dir.size());
+    small_at = total;
+    const size_t o_sums = put(sums.data(), sizeof(uint4) * sums.size());
+    const size_t o_filt = put(fc.data(), sizeof(EsFilterC) * fc.size());
+    const size_t o_allowed = put(d->allowed, 4ull * words);
+    const size_t o_A = put(a_sorted.data(), sizeof(uint4) * a_sorted.size());
+    const size_t o_index = put(a_index.data(), 4 * a_index.size());
+    const size_t o_slices = put(slices.data(), sizeof(uint4) * slices.size());
+    const size_t o_merged = put(merged.data(), 4 * merged.size());
+    if (ce == cudaSuccess) ce = cudaMalloc(&m->tables, total);
     if (ce == cudaSuccess) ce = cudaMalloc(&m->d_cnt, 8ull * 4);
     if (ce == cudaSuccess) ce = cudaHostAlloc(&m->h_cnt, 8ull * 4, cudaHostAllocDefault);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_S2, S2.data(), sizeof(uint4) * S2.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_dir, dir.data(), 4ull * dir.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_sums1, sums.data(), sizeof(uint4) * sums.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess && !fc.empty())
-        ce = cudaMemcpy(m->d_filt, fc.data(), sizeof(EsFilterC) * fc.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess && words) ce = cudaMemcpy(m->d_allowed, d->allowed, 4ull * words, cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_A, sizeof(uint4) * A.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_a_index, 4ull * A.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_slices, sizeof(uint4) * slices.size());
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_A, a_sorted.data(), sizeof(uint4) * A.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_a_index, a_index.data(), 4ull * A.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_slices, slices.data(), sizeof(uint4) * slices.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMalloc(&m->d_merged, 4ull * merged.size());
-    if (ce == cudaSuccess) ce = cudaMemcpy(m->d_merged, merged.data(), 4ull * merged.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->tables + o_S2, S2.data(), sizeof(uint4) * S2.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->tables + o_dir, dir.data(), 4 * dir.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(m->tables + small_at, small.data(), small.size(), cudaMemcpyHostToDevice);
     // the scans' stream is not ordered after the default stream: wait for the copies, and zero the
     // counters on the former
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
@@ -579,22 +602,22 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
         return mcuda(ce, "MITM setup");
     }
     MitmParams& P = m->P;
-    P.S2 = m->d_S2;
-    P.dir = m->d_dir;
-    P.sums1 = m->d_sums1;
-    P.filt = m->d_filt;
-    P.allowed = m->d_allowed;
+    P.S2 = reinterpret_cast<const uint4*>(m->tables + o_S2);
+    P.dir = reinterpret_cast<const uint32_t*>(m->tables + o_dir);
+    P.sums1 = reinterpret_cast<const uint4*>(m->tables + o_sums);
+    P.filt = reinterpret_cast<const EsFilterC*>(m->tables + o_filt);
+    P.allowed = reinterpret_cast<const uint32_t*>(m->tables + o_allowed);
     P.counters = m->d_cnt;
     P.n2 = n2;
     P.M_lo = d->M_lo;
     P.M_hi = d->M_hi;
     P.shift = shift;
     P.n_filters = d->n_filters;
-    P.merged = m->d_merged;
-    P.A = m->d_A;
-    P.a_index = m->d_a_index;
+    P.merged = reinterpret_cast<const uint32_t*>(m->tables + o_merged);
+    P.A = reinterpret_cast<const uint4*>(m->tables + o_A);
+    P.a_index = reinterpret_cast<const uint32_t*>(m->tables + o_index);
     P.n_a = (uint32_t)A.size();
-    P.slices = m->d_slices;
+    P.slices = reinterpret_cast<const uint4*>(m->tables + o_slices);
     P.n_slices = 1u << sl;
     P.merged_words = (uint32_t)merged.size();
     int occ = 0;

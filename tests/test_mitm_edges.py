@@ -74,3 +74,22 @@ def test_gpu_modulus_below_the_slices(native, M):
         assert e.scan(B) == h.brute(B)
     assert e.scan(M, 11, 901)[1] == 890 * 10   # B = M: every pair
     e.close()
+
+
+def test_creation_does_not_hang_on_the_size_of_a_small_s1(tmp_path):
+    """An engine of 131,072 s1 is made in about the time of one of 1,024: what a scan of them takes
+    (a tenth of a millisecond) is not worth sorting them."""
+    import time
+    import es_mitm
+    with fake_lib.bound(fake_lib.build(tmp_path)):
+        def best(radix1):
+            h = _random((1 << 89) - 1, radix1, [40, 40], [101, 103], 3)
+            times = []
+            for _ in range(7):
+                t = time.perf_counter()
+                e = es_mitm.MitmEngine(h, capacity=16)
+                times.append(time.perf_counter() - t)
+                e.close()
+            return min(times)
+        small, large = best([32, 32]), best([64, 64, 32])
+        assert large < 4 * small + 1e-3, (small, large)
