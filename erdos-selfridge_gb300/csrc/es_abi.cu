@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -35,6 +36,10 @@ int cuda_fail(cudaError_t e, const char* what) {
     g_err = std::string(what) + ": " + cudaGetErrorString(e);
     return ES_ERR_CUDA;
 }
+
+// The end of an entry point that allocates on the host: nothing throws across the ABI.
+#define ES_CATCH                                                                     \
+    catch (const std::exception&) { return fail(ES_ERR_NOMEM, "host allocation"); }
 
 #define ES_CUDA(call, what)                                  \
     do {                                                     \
@@ -688,35 +693,31 @@ constexpr double kMoreTables = 0.5;
 // Builds the table sets that launches of this shape read, unless they are there already: the
 // plan's own launches (own), or those of a batch of several plans, which share a table count.
 static int ensure_tables(es_ctx* c, const es_tune& t, bool own) {
-    try {
-        uint32_t F = prod_tables(t);
-        if (own && !c->own_tables[F]) {
-            EsProdImage img;
-            uint32_t use = F;
-            const double most = F < ES_PMAX ? kMoreTables / (32.0 * c->geo.r0) : 1.0;
-            prod_image(c, F, img, most);
-            if (img.rate > most) prod_image(c, use = F + 1, img);
-            if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)
-                if (int e = upload_prod(c, use, img)) return e;
-            c->own_tables[F] = use;
-        }
-        if (own) F = c->own_tables[F];
-        if (!c->prod[F].t.d) {
-            EsProdImage img;
-            prod_image(c, F, img);
-            if (int e = upload_prod(c, F, img)) return e;
-        }
-        es_tune s = t;
-        s.count_stages = 0;
-        if ((!is_production(t) || !runs_production(c, s, F)) && !c->caller.d)
-            if (int e = build_caller(c)) return e;
-    } catch (const std::bad_alloc&) {
-        return fail(ES_ERR_NOMEM, "host allocation");
+    uint32_t F = prod_tables(t);
+    if (own && !c->own_tables[F]) {
+        EsProdImage img;
+        uint32_t use = F;
+        const double most = F < ES_PMAX ? kMoreTables / (32.0 * c->geo.r0) : 1.0;
+        prod_image(c, F, img, most);
+        if (img.rate > most) prod_image(c, use = F + 1, img);
+        if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)
+            if (int e = upload_prod(c, use, img)) return e;
+        c->own_tables[F] = use;
     }
+    if (own) F = c->own_tables[F];
+    if (!c->prod[F].t.d) {
+        EsProdImage img;
+        prod_image(c, F, img);
+        if (int e = upload_prod(c, F, img)) return e;
+    }
+    es_tune s = t;
+    s.count_stages = 0;
+    if ((!is_production(t) || !runs_production(c, s, F)) && !c->caller.d)
+        if (int e = build_caller(c)) return e;
     return ES_OK;
 }
 
-int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
+int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) try {
     if (!d || !out) return fail(ES_ERR_ARG, "null descriptor or output pointer");
     *out = nullptr;
     es_tune tune = tune_in ? *tune_in : default_tune();
@@ -725,22 +726,15 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     if (int code = es_check_desc(*d, bad)) return fail(code, bad);
     if (int e = device_facts()) return e;
 
-    es_ctx* c = new (std::nothrow) es_ctx();
-    if (!c) return fail(ES_ERR_NOMEM, "host allocation");
+    std::unique_ptr<es_ctx, int (*)(es_ctx*)> own(new es_ctx(), es_ctx_destroy);
+    es_ctx* c = own.get();
     std::string why;
-    if (int code = es_parse_plan(*d, c->plan, c->geo, why)) {
-        es_ctx_destroy(c);
-        return fail(code, why);
-    }
+    if (int code = es_parse_plan(*d, c->plan, c->geo, why)) return fail(code, why);
     const uint32_t nf = d->n_filters;
     c->tune = tune;
     c->M = c->plan.M;
     c->q = c->plan.q;
-    int e = ensure_tables(c, tune, true);
-    if (e) {
-        es_ctx_destroy(c);
-        return e;
-    }
+    if (int e = ensure_tables(c, tune, true)) return e;
     cudaError_t ce = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaEventCreate(&c->ev0);
     if (ce == cudaSuccess) ce = cudaEventCreate(&c->ev1);
@@ -750,19 +744,19 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) {
     // on the launches' own stream: nothing orders it after the default stream
     if (ce == cudaSuccess) ce = cudaMemsetAsync(c->d_counts, 0, 8ull * std::max<uint32_t>(nf, 1), c->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(c->d_surv_n, 0, 8ull * 8, c->stream);
-    if (ce != cudaSuccess) { es_ctx_destroy(c); return cuda_fail(ce, "context setup"); }
+    if (ce != cudaSuccess) return cuda_fail(ce, "context setup");
     // d_surv_n block: [0] survivor count, [1] unit counter, [2] CTAs done, [3..6] group min
     c->d_unit = c->d_surv_n + 1;
     c->d_done = c->d_surv_n + 2;
     c->d_min = c->d_surv_n + 3;
-    e = es_set_capacity(c, 1u << 20);
-    if (e) { es_ctx_destroy(c); return e; }
-    *out = c;
+    if (int e = es_set_capacity(c, 1u << 20)) return e;
+    *out = own.release();
     return ES_OK;
 }
+ES_CATCH
 
 int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes, es_cascade_info* info, void* small,
-                     uint64_t small_cap, uint32_t* tabs, uint64_t tabs_cap, uint32_t* parts, uint64_t parts_cap) {
+                     uint64_t small_cap, uint32_t* tabs, uint64_t tabs_cap, uint32_t* parts, uint64_t parts_cap) try {
     if (!d || !info) return fail(ES_ERR_ARG, "null argument");
     if (tables < 1 || tables > ES_PMAX) return fail(ES_ERR_ARG, "tables must be in 1..6");
     std::string why;
@@ -771,11 +765,7 @@ int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes
     if (int code = es_check_desc(*d, why)) return fail(code, why);
     if (int code = es_parse_plan(*d, P, geo, why)) return fail(code, why);
     EsProdImage img;
-    try {
-        es_prod_image(P, geo, tables, smem_bytes, img);
-    } catch (const std::bad_alloc&) {
-        return fail(ES_ERR_NOMEM, "host allocation");
-    }
+    es_prod_image(P, geo, tables, smem_bytes, img);
     const EsInst& I = img.inst;
     memset(info, 0, sizeof(*info));
     info->n_entries = I.n_filters;
@@ -811,14 +801,16 @@ int es_cascade_image(const es_plan_desc* d, uint32_t tables, uint32_t smem_bytes
     if (tabs && tabs_cap >= img.tabs.size()) memcpy(tabs, img.tabs.data(), 4ull * img.tabs.size());
     return ES_OK;
 }
+ES_CATCH
 
-int es_ctx_set_tune(es_ctx* c, const es_tune* t) {
+int es_ctx_set_tune(es_ctx* c, const es_tune* t) try {
     if (!c || !t) return fail(ES_ERR_ARG, "null argument");
     if (int e = check_tune(*t)) return e;
     if (int e = ensure_tables(c, *t, true)) return e;
     c->tune = *t;
     return ES_OK;
 }
+ES_CATCH
 
 int es_ctx_get_tune(const es_ctx* c, es_tune* t) {
     if (!c || !t) return fail(ES_ERR_ARG, "null argument");
@@ -1005,7 +997,7 @@ int es_read_survivor_records(es_ctx* c, es_survivor* out, uint64_t cap, uint64_t
     return ES_OK;
 }
 
-int es_read_survivors(es_ctx* c, uint64_t* idx_out, uint64_t cap, uint64_t* n) {
+int es_read_survivors(es_ctx* c, uint64_t* idx_out, uint64_t cap, uint64_t* n) try {
     if (!c || !n) return fail(ES_ERR_ARG, "null argument");
     uint64_t cnt = 0;
     if (int e = es_survivor_count(c, &cnt)) return e;
@@ -1020,6 +1012,7 @@ int es_read_survivors(es_ctx* c, uint64_t* idx_out, uint64_t cap, uint64_t* n) {
     for (uint64_t i = 0; i < cnt; ++i) idx_out[i] = tmp[i].idx;
     return ES_OK;
 }
+ES_CATCH
 
 int es_stage_counts(es_ctx* c, uint64_t* counts, uint32_t n) {
     if (!c || (n && !counts)) return fail(ES_ERR_ARG, "null argument");
@@ -1069,20 +1062,20 @@ int es_batch_destroy(es_batch* b) {
 }
 
 int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* items,
-                    uint32_t n_items, const es_tune* tune_in, es_batch** out) {
+                    uint32_t n_items, const es_tune* tune_in, es_batch** out) try {
     if (!ctxs || !items || !out || n_ctx == 0 || n_items == 0)
         return fail(ES_ERR_ARG, "empty batch");
     *out = nullptr;
     es_tune tune = tune_in ? *tune_in : ctxs[0]->tune;
     if (int e = check_tune(tune)) return e;
     if (int e = device_facts()) return e;
-    es_batch* b = new (std::nothrow) es_batch();
-    if (!b) return fail(ES_ERR_NOMEM, "host allocation");
+    std::unique_ptr<es_batch, int (*)(es_batch*)> own(new es_batch(), es_batch_destroy);
+    es_batch* b = own.get();
     b->tune = tune;
     b->ctxs.assign(ctxs, ctxs + n_ctx);
     for (uint32_t i = 0; i < n_ctx; ++i) {
-        if (!ctxs[i]) { es_batch_destroy(b); return fail(ES_ERR_ARG, "null context in batch"); }
-        if (int e = ensure_tables(ctxs[i], tune, n_ctx == 1)) { es_batch_destroy(b); return e; }
+        if (!ctxs[i]) return fail(ES_ERR_ARG, "null context in batch");
+        if (int e = ensure_tables(ctxs[i], tune, n_ctx == 1)) return e;
     }
     const uint32_t PF = n_ctx == 1 ? ctxs[0]->own_tables[prod_tables(tune)] : prod_tables(tune);
     // the table set a plan's items run on
@@ -1098,14 +1091,12 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     uint32_t max_group = 0;
     for (uint32_t i = 0; i < n_items; ++i) {
         const es_batch_item& s = items[i];
-        if (s.ctx_index >= n_ctx) { es_batch_destroy(b); return fail(ES_ERR_ARG, "item ctx_index out of range"); }
-        if (s.group >= n_items) { es_batch_destroy(b); return fail(ES_ERR_ARG, "item group must be < n_items"); }
+        if (s.ctx_index >= n_ctx) return fail(ES_ERR_ARG, "item ctx_index out of range");
+        if (s.group >= n_items) return fail(ES_ERR_ARG, "item group must be < n_items");
         const es_ctx* c = ctxs[s.ctx_index];
         const EsInst& I = c->geo;
-        if (s.o_begin > s.o_end || s.o_end > I.n_outer) {
-            es_batch_destroy(b);
+        if (s.o_begin > s.o_end || s.o_end > I.n_outer)
             return fail(ES_ERR_RANGE, "item outer range outside [0, R/r0)");
-        }
         EsItem& it = b->h_items[i];
         memset(&it, 0, sizeof(it));
         it.inst = tables(c).d;
@@ -1158,13 +1149,11 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     const size_t n_scalars = 4ull * b->n_groups + 1 + 2ull * n_items + cwords + b->n_groups;
     b->pool = ctxs[0]->pool;
     b->mem = b->pool->take();
-    if (!b->mem) b->mem.reset(new (std::nothrow) BatchMem());
-    if (!b->mem) { es_batch_destroy(b); return fail(ES_ERR_NOMEM, "host allocation"); }
+    if (!b->mem) b->mem.reset(new BatchMem());
     b->surv_cap = ctxs[0]->surv_cap;
     cudaError_t ce = b->mem->need(upload + 8 * n_scalars, upload + 8 * (4ull * b->n_groups + 1), b->surv_cap);
     if (ce != cudaSuccess) {
         b->mem.reset();
-        es_batch_destroy(b);
         return cuda_fail(ce, "batch setup");
     }
     b->stream = b->mem->stream;
@@ -1277,10 +1266,8 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
         L.stage_off = sp.stage_off;
         if (one_ctx) launch_tables(L, tables(ctxs[first_ctx]).h);
         if (int e = grid_for(sub.layout, tune.count_stages, sub.words, F, shape, sp.bytes,
-                             std::max<uint64_t>(units, 1), &sub.grid)) {
-            es_batch_destroy(b);
+                             std::max<uint64_t>(units, 1), &sub.grid))
             return e;
-        }
         b->subs.push_back(sub);
         pos = end;
     }
@@ -1289,10 +1276,11 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     memcpy(stage + items_bytes, launch_items.data(), sizeof(EsItem) * n_items);
     if (!h_tc.empty()) memcpy(stage + 2 * items_bytes, h_tc.data(), 4ull * h_tc.size());
     ce = cudaMemcpyAsync(b->mem->dev, stage, upload, cudaMemcpyHostToDevice, b->stream);
-    if (ce != cudaSuccess) { es_batch_destroy(b); return cuda_fail(ce, "batch upload"); }
-    *out = b;
+    if (ce != cudaSuccess) return cuda_fail(ce, "batch upload");
+    *out = own.release();
     return ES_OK;
 }
+ES_CATCH
 
 static int batch_enqueue(es_batch* b) {
     ES_CUDA(cudaMemsetAsync(b->d_surv_n, 0, b->zero_bytes, b->stream), "memset");

@@ -38,6 +38,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
+#include <functional>
+#include <memory>
 #include <new>
 #include <string>
 #include <thread>
@@ -314,6 +317,21 @@ void bucket_sort(std::vector<T>& v, uint32_t bits, const Key& key) {
     v.swap(out);
 }
 
+// body(0) .. body(T - 1), each on a thread of its own where the system gives one (body must not throw).
+template <class Body>
+void on_threads(unsigned T, const Body& body) {
+    std::vector<std::thread> th;
+    th.reserve(T);
+    unsigned t = 1;
+    try {
+        for (; t < T; ++t) th.emplace_back(std::cref(body), t);
+    } catch (const std::exception&) {   // no more threads: the rest runs here
+    }
+    body(0);
+    for (; t < T; ++t) body(t);
+    for (auto& x : th) x.join();
+}
+
 }  // namespace
 
 extern "C" {
@@ -345,13 +363,8 @@ void parallel_sort(std::vector<u128m>& v, uint32_t bits) {
     const uint32_t P = std::min<uint32_t>(12, bits);
     const uint32_t sh = bits - P;
     const size_t np = (size_t)1 << P;
-    auto run = [T](auto&& body) {
-        std::vector<std::thread> th;
-        for (unsigned t = 0; t < T; ++t) th.emplace_back(body, t);
-        for (auto& x : th) x.join();
-    };
     std::vector<std::vector<size_t>> at(T, std::vector<size_t>(np, 0));
-    run([&](unsigned t) {
+    on_threads(T, [&](unsigned t) {
         for (size_t i = n * t / T, e = n * (t + 1) / T; i < e; ++i) ++at[t][(size_t)(v[i] >> sh)];
     });
     std::vector<size_t> start(np + 1);
@@ -366,11 +379,11 @@ void parallel_sort(std::vector<u128m>& v, uint32_t bits) {
     }
     start[np] = acc;
     std::vector<u128m> out(n);
-    run([&](unsigned t) {
+    on_threads(T, [&](unsigned t) {
         for (size_t i = n * t / T, e = n * (t + 1) / T; i < e; ++i) out[at[t][(size_t)(v[i] >> sh)]++] = v[i];
     });
     std::atomic<size_t> next(0);
-    run([&](unsigned) {
+    on_threads(T, [&](unsigned) {
         for (size_t p = next++; p < np; p = next++) std::sort(out.begin() + start[p], out.begin() + start[p + 1]);
     });
     v.swap(out);
@@ -378,7 +391,7 @@ void parallel_sort(std::vector<u128m>& v, uint32_t bits) {
 
 }  // namespace
 
-int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
+int es_mitm_create(const es_mitm_desc* d, es_mitm** out) try {
     if (!d || !out) return mfail(ES_ERR_ARG, "null descriptor or output pointer");
     *out = nullptr;
     const u128m M = ((u128m)d->M_hi << 64) | d->M_lo;
@@ -464,10 +477,7 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
             if (t + 1 == T)
                 for (; b <= (1ull << D); ++b) dir[b] = (uint32_t)n2;
         };
-        std::vector<std::thread> th;
-        for (unsigned t = 1; t < T; ++t) th.emplace_back(fill, t);
-        fill(0);
-        for (auto& x : th) x.join();
+        on_threads(T, fill);
     }
     // ---- filters ---------------------------------------------------------------------------
     std::vector<EsFilterC> fc(d->n_filters);
@@ -485,8 +495,8 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
         words += (q + 31) / 32;
     }
 
-    es_mitm* m = new (std::nothrow) es_mitm();
-    if (!m) return mfail(ES_ERR_NOMEM, "host allocation");
+    std::unique_ptr<es_mitm, int (*)(es_mitm*)> own(new es_mitm(), es_mitm_destroy);
+    es_mitm* m = own.get();
     m->n1 = n1;
     m->n2 = n2;
     // ---- merged tables: products of projections of filters, tested ahead of the cascade ---------
@@ -597,10 +607,7 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     // counters on the former
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(m->d_cnt, 0, 8ull * 4, m->stream);
-    if (ce != cudaSuccess) {
-        es_mitm_destroy(m);
-        return mcuda(ce, "MITM setup");
-    }
+    if (ce != cudaSuccess) return mcuda(ce, "MITM setup");
     MitmParams& P = m->P;
     P.S2 = reinterpret_cast<const uint4*>(m->tables + o_S2);
     P.dir = reinterpret_cast<const uint32_t*>(m->tables + o_dir);
@@ -622,17 +629,13 @@ int es_mitm_create(const es_mitm_desc* d, es_mitm** out) {
     P.merged_words = (uint32_t)merged.size();
     int occ = 0;
     ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, es_mitm_kernel, kMitmThreads, 4ull * merged.size());
-    if (ce != cudaSuccess || occ < 1) {
-        es_mitm_destroy(m);
-        return mcuda(ce == cudaSuccess ? cudaErrorInvalidConfiguration : ce, "MITM occupancy");
-    }
+    if (ce != cudaSuccess || occ < 1) return mcuda(ce == cudaSuccess ? cudaErrorInvalidConfiguration : ce, "MITM occupancy");
     m->grid = sms * occ;
-    if (int e = es_mitm_set_capacity(m, 1u << 20)) {
-        es_mitm_destroy(m);
-        return e;
-    }
-    *out = m;
+    if (int e = es_mitm_set_capacity(m, 1u << 20)) return e;
+    *out = own.release();
     return ES_OK;
+} catch (const std::exception&) {   // nothing throws across the ABI
+    return mfail(ES_ERR_NOMEM, "host allocation");
 }
 
 int es_mitm_info(const es_mitm* m, uint64_t* n1, uint64_t* n2) {
@@ -687,7 +690,7 @@ int es_mitm_scan(es_mitm* m, uint64_t B_lo, uint64_t B_hi, uint64_t s1_begin, ui
 }
 
 int es_mitm_results(es_mitm* m, uint64_t* n_lo, uint64_t* n_hi, uint64_t cap, uint64_t* n_surv,
-                    uint64_t* n_cand) {
+                    uint64_t* n_cand) try {
     if (!m || !n_surv) return mfail(ES_ERR_ARG, "null argument");
     ES_MCUDA(cudaMemcpyAsync(m->h_cnt, m->d_cnt, 16, cudaMemcpyDeviceToHost, m->stream), "copy");
     ES_MCUDA(cudaStreamSynchronize(m->stream), "MITM kernel execution");
@@ -706,6 +709,8 @@ int es_mitm_results(es_mitm* m, uint64_t* n_lo, uint64_t* n_hi, uint64_t cap, ui
         if (n_hi) n_hi[i] = ((uint64_t)tmp[i].w << 32) | tmp[i].z;
     }
     return ES_OK;
+} catch (const std::exception&) {
+    return mfail(ES_ERR_NOMEM, "host allocation");
 }
 
 }  // extern "C"

@@ -30,6 +30,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -808,13 +810,14 @@ int es_mlp_destroy(es_mlp* M) {
     return ES_OK;
 }
 
-int es_mlp_create(uint32_t in_dim, uint32_t hidden, uint32_t out_dim, uint64_t seed, es_mlp** out) {
+int es_mlp_create(uint32_t in_dim, uint32_t hidden, uint32_t out_dim, uint64_t seed, es_mlp** out) try {
     if (!out) return mlp_fail(ES_ERR_ARG, "null output");
     *out = nullptr;
     if (in_dim < 1 || in_dim > kMaxD || hidden < 8 || hidden > kMaxH || hidden % 32 || out_dim < 1 ||
         out_dim > kMaxO || out_dim > hidden)
         return mlp_fail(ES_ERR_RANGE, "MLP dims must be in <= 64, hidden 32 or 64, out <= 8");
-    es_mlp* M = new es_mlp();
+    std::unique_ptr<es_mlp, int (*)(es_mlp*)> own(new es_mlp(), es_mlp_destroy);
+    es_mlp* M = own.get();
     M->d = Dims{(int)in_dim, (int)hidden, (int)out_dim};
     const int np = M->d.n();
     std::vector<float> h(3 * np, 0.f);   // parameters, then the moments' zeros
@@ -833,12 +836,11 @@ int es_mlp_create(uint32_t in_dim, uint32_t hidden, uint32_t out_dim, uint64_t s
     M->loss = M->g + np;
     M->err = reinterpret_cast<int*>(M->loss + 1);
     if (e == cudaSuccess) e = cudaMemset(M->err, 0, 4);
-    if (e != cudaSuccess) {
-        es_mlp_destroy(M);
-        return mlp_fail(ES_ERR_CUDA, std::string("MLP setup: ") + cudaGetErrorString(e));
-    }
-    *out = M;
+    if (e != cudaSuccess) return mlp_fail(ES_ERR_CUDA, std::string("MLP setup: ") + cudaGetErrorString(e));
+    *out = own.release();
     return ES_OK;
+} catch (const std::exception&) {   // nothing throws across the ABI
+    return mlp_fail(ES_ERR_NOMEM, "host allocation");
 }
 
 int es_mlp_num_params(const es_mlp* M, uint64_t* n) {
@@ -919,7 +921,7 @@ int es_mlp_loss_grad(es_mlp* M, const float* X, const float* T, uint64_t n, floa
 // launch per epoch: the host draws the next epoch's order, and a second stream uploads it, while the
 // cluster works on the last one.
 int es_mlp_train(es_mlp* M, const float* X, const float* T, uint64_t n, uint32_t epochs, uint32_t batch,
-                 float lr, uint64_t seed, float* final_loss) {
+                 float lr, uint64_t seed, float* final_loss) try {
     if (!M || !X || !T || n == 0 || batch == 0) return mlp_fail(ES_ERR_ARG, "null argument or empty set");
     if (n > 0xffffffffull) return mlp_fail(ES_ERR_RANGE, "more than 2^32 samples");
     const Dims d = M->d;
@@ -982,6 +984,8 @@ int es_mlp_train(es_mlp* M, const float* X, const float* T, uint64_t n, uint32_t
     }
     M->trim();
     return e == cudaSuccess ? ES_OK : mlp_fail(ES_ERR_CUDA, cudaGetErrorString(e));
+} catch (const std::exception&) {
+    return mlp_fail(ES_ERR_NOMEM, "host allocation");
 }
 
 }  // extern "C"

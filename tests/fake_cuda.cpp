@@ -9,7 +9,9 @@
 //   fake_faults()   launches while writes wait on the legacy default stream, work counters that are
 //                   not zero, shared memory above what the kernel may use
 //   fake_launches() launches that ran
-//   fake_fail_alloc(n)  the n-th host allocation from now on throws std::bad_alloc (0: none)
+//   fake_fail_alloc(n)  the library's n-th host allocation from now on throws std::bad_alloc (0: none);
+//                   returns how far an earlier request still was from failing (0: it has failed)
+//   fake_live()     device and pinned allocations that have not been freed
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -25,18 +27,29 @@
 
 namespace {
 std::map<cudaStream_t, std::vector<std::function<void()>>> queues;
-int faults = 0, launches = 0;
+int faults = 0, launches = 0, live = 0;
 thread_local long fail_in = 0;
+thread_local int inside = 0;   // in this file: its own allocations neither count nor fail
+struct Inside {
+    Inside() { ++inside; }
+    ~Inside() { --inside; }
+};
 uintptr_t next_handle = 16;
 
 void run(cudaStream_t s) {
+    const Inside here;
     auto q = std::move(queues[s]);
     queues[s].clear();
     for (auto& f : q) f();
 }
-void put(cudaStream_t s, std::function<void()> f) { queues[s].push_back(std::move(f)); }
+template <class F>
+void put(cudaStream_t s, const F& f) {
+    const Inside here;
+    queues[s].push_back(f);
+}
 
 cudaError_t copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t s) {
+    const Inside here;
     if (kind == cudaMemcpyHostToDevice) {   // the host buffer is read now, the device written later
         std::vector<unsigned char> b((const unsigned char*)src, (const unsigned char*)src + n);
         put(s, [=] { memcpy(dst, b.data(), n); });
@@ -47,6 +60,7 @@ cudaError_t copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cuda
 }
 // What a launch on stream s finds, apart from its arguments.
 void launched(cudaStream_t s) {
+    const Inside here;
     if (s != nullptr && !queues[nullptr].empty()) ++faults;
     ++launches;
 }
@@ -55,7 +69,8 @@ void launched(cudaStream_t s) {
 extern "C" {
 int fake_faults() { return faults; }
 int fake_launches() { return launches; }
-void fake_fail_alloc(long n) { fail_in = n; }
+int fake_live() { return live; }
+long fake_fail_alloc(long n) { const long left = fail_in; fail_in = n; return left; }
 void fake_drain() { for (auto& q : queues) run(q.first); }
 
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
@@ -70,11 +85,12 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
     *p = aligned_alloc(256, (n + 511) / 256 * 256);
     if (*p && n <= (64u << 20)) memset(*p, 0xcd, n);
+    live += *p != nullptr;
     return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }
-cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { live -= p != nullptr; free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
-cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f) {
     if (f != cudaStreamNonBlocking) ++faults;
     *s = (cudaStream_t)(next_handle += 16);
@@ -165,7 +181,7 @@ int es_launch_min(const es_survivor*, const unsigned long long*, uint64_t, const
 int es_launch_int_peak(unsigned long long*, int, int, int, int, void*) { return 0; }
 
 // ---- host allocations that fail on request ------------------------------------------------------
-static bool fails() { return fail_in > 0 && --fail_in == 0; }
+static bool fails() { return !inside && fail_in > 0 && --fail_in == 0; }
 void* operator new(size_t n) {
     void* p = fails() ? nullptr : malloc(n ? n : 1);
     if (!p) throw std::bad_alloc();

@@ -28,7 +28,7 @@ def bound(so: str):
     N._lib, N.LIB_PATH = None, so
     try:
         L = N.lib()
-        L.fake_fail_alloc.argtypes = [C.c_long]
+        L.fake_fail_alloc.argtypes, L.fake_fail_alloc.restype = [C.c_long], C.c_long
         yield L
     finally:
         N._lib, N.LIB_PATH = kept
