@@ -684,11 +684,16 @@ static int upload_prod(es_ctx* c, uint32_t F, EsProdImage& img) {
 }
 
 // Candidates per warp-wide ring-1 digit above which a plan's own launches take one more inner table
-// than asked for: the queue's passes then cost more than the table, which few lanes read.  Four and
-// five tables, 2^34 positions: k = 384 (1.8 candidates with four) 1552 and 1494 us, k = 300 (0.6) 1330
-// and 1276, k = 390 (1.1) 1417 and 1415, k = 379 (2.9) 1658 and 1679; 2^30 positions: k = 200 (0.2) 179
-// and 184.
-constexpr double kMoreTables = 0.5;
+// than asked for: the queue's passes then cost more than the table, which few lanes read.  A wider ring
+// reads more of it, two rows of its words instead of one, so the line lies higher there.  With four
+// tables and with five, 2^32 positions, us by candidates with four:
+//   one word       0.28: 340, 354   0.44: 468, 460   0.51: 469, 436   0.80: 448, 429   1.09: 400, 368
+//   two words      0.57: 516, 537   1.01: 373, 385   1.10: 391, 390   1.19: 387, 371   1.90: 481, 391
+//   three or four  1.47: 358, 380   2.24: 360, 363   2.88: 432, 439   3.41: 393, 382   5.66: 430, 391
+//   five and more  1.1 a word: 548, 595   1.6: 556, 621   2.1: 575, 644   2.5: 483, 428   4.4: 1228, 1003
+// (k = 160..400 and the recorded wheels; for five and more words wheels of k = 220..390 around one large
+// prime, of which 2.5 and 5.1 candidates a word also lost 4 and 10 %).
+static double more_tables(uint32_t words) { return words == 1 ? 0.5 : words == 2 ? 1.15 : words <= 4 ? 3.2 : 2.3 * words; }
 
 // Builds the table sets that launches of this shape read, unless they are there already: the
 // plan's own launches (own), or those of a batch of several plans, which share a table count.
@@ -697,7 +702,7 @@ static int ensure_tables(es_ctx* c, const es_tune& t, bool own) {
     if (own && !c->own_tables[F]) {
         EsProdImage img;
         uint32_t use = F;
-        const double most = F < ES_PMAX ? kMoreTables / (32.0 * c->geo.r0) : 1.0;
+        const double most = F < ES_PMAX ? more_tables(c->geo.W) / (32.0 * c->geo.r0) : 1.0;
         prod_image(c, F, img, most);
         if (img.rate > most) prod_image(c, use = F + 1, img);
         if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)

@@ -8,7 +8,7 @@
 // looks, when its stream runs, at what it was given and counts what is wrong:
 //   fake_faults()   launches while writes wait on the legacy default stream, work counters that are
 //                   not zero, shared memory above what the kernel may use
-//   fake_launches() launches that ran
+//   fake_launches() launches that ran; fake_tables() the inner tables of the last scan
 //   fake_fail_alloc(n)  the library's n-th host allocation from now on throws std::bad_alloc (0: none);
 //                   returns how far an earlier request still was from failing (0: it has failed)
 //   fake_live()     device and pinned allocations that have not been freed
@@ -27,7 +27,7 @@
 
 namespace {
 std::map<cudaStream_t, std::vector<std::function<void()>>> queues;
-int faults = 0, launches = 0, live = 0;
+int faults = 0, launches = 0, live = 0, tables = 0;
 thread_local long fail_in = 0;
 thread_local int inside = 0;   // in this file: its own allocations neither count nor fail
 struct Inside {
@@ -70,6 +70,7 @@ extern "C" {
 int fake_faults() { return faults; }
 int fake_launches() { return launches; }
 int fake_live() { return live; }
+int fake_tables() { return tables; }
 long fake_fail_alloc(long n) { const long left = fail_in; fail_in = n; return left; }
 void fake_drain() { for (auto& q : queues) run(q.first); }
 
@@ -161,6 +162,7 @@ int es_scan_occupancy(int, int, uint32_t, uint32_t, int threads, int smem, int* 
 int es_launch_scan(const EsLaunch& L, int layout, int, uint32_t, int, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     launched(s);
+    tables = (int)L.mask_filters;
     EsLaunch l = L;
     if (!l.items) put(s, [=] {
         if (*l.unit_counter != 0 || *l.ctas_done != 0) ++faults;

@@ -151,6 +151,25 @@ def test_tables_never_exceed_their_room():
                 assert 4 * info.tab_words <= max(min(left, most), fill_ins), (spec, tables, room)
 
 
+# plans whose candidates per digit with four tables lie on either side of the line of their ring's words
+@pytest.mark.parametrize("spec,want", [
+    ((316, None), 4), ((196, None), 4), ((340, None), 5), ((394, "primary"), 5), ((244, None), 4),
+    ((390, "confirmation"), 4), ((395, "confirmation"), 5), ((384, "primary"), 5), ((380, "confirmation"), 4),
+    ((379, "primary"), 4), ((400, "primary"), 5), ((378, "primary"), 5), ((391, "primary"), 5),
+    ((250, [[199, 1], [7, 3], [137, 1], [89, 1], [17, 2], [131, 1], [37, 1], [43, 1], [2, 8], [127, 1], [11, 1], [23, 1],
+            [3, 2]]), 4)], ids=str)
+def test_one_more_table_where_it_pays(spec, want, tmp_path):
+    import es_native as N
+    import fake_lib
+    with fake_lib.bound(fake_lib.build(tmp_path)) as L:
+        ctx = N.Context(_plan(spec), N.make_tune(layout=N.LAYOUT_AUTO, mask_filters=4, count_stages=0))
+        ctx.set_block(0)
+        ctx.launch(0, 1)
+        ctx.sync()
+        ctx.close()
+        assert L.fake_tables() == want
+
+
 # ------------------------------------------------------------------ GPU
 def _ranges(P):
     outer = P.R // P.radix[0]
