@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -120,9 +121,9 @@ struct ProdSet {
     std::vector<EsCascadeEntry> entries;
 };
 
-// Device and pinned memory, stream and events of one batch.  A destroyed batch hands them to the
-// pool of its first context, which keeps one such set for the next batch: a block-ordered search
-// makes a batch per launch, and allocating and freeing these took 200 of its 254 us.
+// Device and pinned memory, stream and events of one batch.  A destroyed batch hands them to its
+// device's pool for the next batch: a block-ordered search makes a batch per launch, and allocating
+// and freeing these took 200 of its 254 us.
 struct BatchMem {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -133,6 +134,7 @@ struct BatchMem {
     BatchMem() = default;
     BatchMem(const BatchMem&) = delete;
     BatchMem& operator=(const BatchMem&) = delete;
+    size_t bytes() const { return dev_cap + pin_cap + sizeof(es_survivor) * surv_cap; }
     ~BatchMem() {
         cudaFree(dev);
         cudaFree(surv);
@@ -171,19 +173,39 @@ struct BatchMem {
     }
 };
 
-// Shared by a context and the batches made on it, so that either may go first.
+// One per device, held by its contexts and their batches and gone with the last of them.
 struct BatchPool {
-    static constexpr size_t kKeep = 256u << 20;   // a larger set is freed instead of kept
+    static constexpr size_t kKeep = 256u << 20;   // idle bytes at most; what is beyond is freed
     std::mutex mu;
-    std::unique_ptr<BatchMem> idle;
-    std::unique_ptr<BatchMem> take() {
+    std::vector<std::unique_ptr<BatchMem>> idle;
+    // a set whose survivor buffer holds `cap` records, if there is one, else any
+    std::unique_ptr<BatchMem> take(uint64_t cap) {
         std::lock_guard<std::mutex> lock(mu);
-        return std::move(idle);
+        if (idle.empty()) return nullptr;
+        size_t at = idle.size() - 1;
+        for (size_t i = 0; i < idle.size(); ++i)
+            if (idle[i]->surv_cap >= cap) at = i;
+        std::unique_ptr<BatchMem> m = std::move(idle[at]);
+        idle.erase(idle.begin() + (ptrdiff_t)at);
+        return m;
     }
     void give(std::unique_ptr<BatchMem> m) {
-        if (m->dev_cap + m->pin_cap + sizeof(es_survivor) * m->surv_cap > kKeep) return;
         std::lock_guard<std::mutex> lock(mu);
-        if (!idle) idle = std::move(m);
+        size_t bytes = m->bytes();
+        for (const std::unique_ptr<BatchMem>& x : idle) bytes += x->bytes();
+        if (bytes > kKeep) return;
+        try {
+            idle.push_back(std::move(m));
+        } catch (const std::exception&) {   // no memory for the list: the set is freed
+        }
+    }
+    static std::shared_ptr<BatchPool> of_device(int dev) {
+        static std::mutex mu;
+        static std::map<int, std::weak_ptr<BatchPool>> pools;
+        std::lock_guard<std::mutex> lock(mu);
+        std::shared_ptr<BatchPool> p = pools[dev].lock();
+        if (!p) pools[dev] = p = std::make_shared<BatchPool>();
+        return p;
     }
 };
 
@@ -216,7 +238,7 @@ struct es_ctx {
     // the survivor count read since the last launch or reset, if any
     bool count_known = false;
     uint64_t count = 0;
-    std::shared_ptr<BatchPool> pool = std::make_shared<BatchPool>();
+    std::shared_ptr<BatchPool> pool;   // the device's
 };
 
 struct es_batch {
@@ -733,6 +755,7 @@ int es_ctx_create(const es_plan_desc* d, const es_tune* tune_in, es_ctx** out) t
 
     std::unique_ptr<es_ctx, int (*)(es_ctx*)> own(new es_ctx(), es_ctx_destroy);
     es_ctx* c = own.get();
+    c->pool = BatchPool::of_device(g_dev.dev);
     std::string why;
     if (int code = es_parse_plan(*d, c->plan, c->geo, why)) return fail(code, why);
     const uint32_t nf = d->n_filters;
@@ -1153,7 +1176,7 @@ int es_batch_create(es_ctx* const* ctxs, uint32_t n_ctx, const es_batch_item* it
     const size_t upload = 2 * items_bytes + es_align_up(4ull * h_tc.size(), 16);
     const size_t n_scalars = 4ull * b->n_groups + 1 + 2ull * n_items + cwords + b->n_groups;
     b->pool = ctxs[0]->pool;
-    b->mem = b->pool->take();
+    b->mem = b->pool->take(ctxs[0]->surv_cap);
     if (!b->mem) b->mem.reset(new BatchMem());
     b->surv_cap = ctxs[0]->surv_cap;
     cudaError_t ce = b->mem->need(upload + 8 * n_scalars, upload + 8 * (4ull * b->n_groups + 1), b->surv_cap);
