@@ -696,6 +696,12 @@ static void prod_image(const es_ctx* c, uint32_t F, EsProdImage& img, double max
                   (uint32_t)g_dev.smem_optin - 2048u - ES_PROD_THREADS / 32u * ES_QUEUE_BYTES, img, max_rate);
 }
 
+// Whether a CTA of any size has room for it (runs_production asks for the launch's own).
+static bool image_fits(const EsProdImage& img) {
+    return img.small.size() + es_align_up(4 * img.tabs.size(), 16) + ES_PROD_THREADS / 32u * ES_QUEUE_BYTES <=
+           (size_t)g_dev.smem_optin - 1024u;
+}
+
 static int upload_prod(es_ctx* c, uint32_t F, EsProdImage& img) {
     TableSet T;
     T.h = img.inst;
@@ -726,7 +732,10 @@ static int ensure_tables(es_ctx* c, const es_tune& t, bool own) {
         uint32_t use = F;
         const double most = F < ES_PMAX ? more_tables(c->geo.W) / (32.0 * c->geo.r0) : 1.0;
         prod_image(c, F, img, most);
-        if (img.rate > most) prod_image(c, use = F + 1, img);
+        if (img.rate > most) {
+            prod_image(c, use = F + 1, img);
+            if (!image_fits(img)) prod_image(c, use = F, img);   // (its ring-1 and step rows may be twice as long)
+        }
         if (!c->prod[use].t.d)   // (counting contexts too: es_search_blocks_static never counts)
             if (int e = upload_prod(c, use, img)) return e;
         c->own_tables[F] = use;

@@ -8,7 +8,8 @@
 // looks, when its stream runs, at what it was given and counts what is wrong:
 //   fake_faults()   launches while writes wait on the legacy default stream, work counters that are
 //                   not zero, shared memory above what the kernel may use
-//   fake_launches() launches that ran; fake_tables() the inner tables of the last scan
+//   fake_launches() launches that ran; fake_tables(), fake_layout() the inner
+//                   tables and the layout of the last scan
 //   fake_fail_alloc(n)  the library's n-th host allocation from now on throws std::bad_alloc (0: none);
 //                   returns how far an earlier request still was from failing (0: it has failed)
 //   fake_live()     device and pinned allocations that have not been freed
@@ -27,7 +28,7 @@
 
 namespace {
 std::map<cudaStream_t, std::vector<std::function<void()>>> queues;
-int faults = 0, launches = 0, live = 0, tables = 0;
+int faults = 0, launches = 0, live = 0, tables = 0, layouts = 0;
 thread_local long fail_in = 0;
 thread_local int inside = 0;   // in this file: its own allocations neither count nor fail
 struct Inside {
@@ -71,6 +72,7 @@ int fake_faults() { return faults; }
 int fake_launches() { return launches; }
 int fake_live() { return live; }
 int fake_tables() { return tables; }
+int fake_layout() { return layouts; }
 long fake_fail_alloc(long n) { const long left = fail_in; fail_in = n; return left; }
 void fake_drain() { for (auto& q : queues) run(q.first); }
 
@@ -163,6 +165,7 @@ int es_launch_scan(const EsLaunch& L, int layout, int, uint32_t, int, void* stre
     cudaStream_t s = (cudaStream_t)stream;
     launched(s);
     tables = (int)L.mask_filters;
+    layouts = layout;
     EsLaunch l = L;
     if (!l.items) put(s, [=] {
         if (*l.unit_counter != 0 || *l.ctas_done != 0) ++faults;

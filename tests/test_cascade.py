@@ -170,6 +170,28 @@ def test_one_more_table_where_it_pays(spec, want, tmp_path):
         assert L.fake_tables() == want
 
 
+@pytest.mark.parametrize("r1,want", [(2000, (16, 4)), (3300, (16, 3))])
+def test_one_more_table_only_where_it_fits(r1, want, tmp_path):
+    """Three tables of weak filters, which ask for a fourth; its rows of a long ring 1 may not fit a CTA
+    where the three tables' do (16: the production cascade, 1: the scalar layout)."""
+    import es_native as N
+    import fake_lib
+    rng = np.random.default_rng(r1)
+    M, radix, q = (1 << 89) - 1, [32, r1, 4, 5], [11, 13, 17, 19, 23, 29]
+    terms = [int(x) * int(y) % M for x, y in zip(rng.integers(1, 1 << 62, size=sum(radix)), rng.integers(1, 1 << 62, size=sum(radix)))]
+    arrays = N.PlanArrays.from_arrays(
+        30, np.array(radix, dtype=np.uint32), np.array([t & (1 << 64) - 1 for t in terms], dtype=np.uint64),
+        np.array([t >> 64 for t in terms], dtype=np.uint64), np.array(q, dtype=np.uint32),
+        np.concatenate([N.bit_table(x, range(1, x)) for x in q]), M)
+    with fake_lib.bound(fake_lib.build(tmp_path)) as L:
+        ctx = N.Context.from_arrays(arrays, N.make_tune(layout=N.LAYOUT_AUTO, mask_filters=3, count_stages=0), len(q))
+        ctx.set_block(0, np.zeros(len(q), dtype=np.uint32))
+        ctx.launch(0, 1)
+        ctx.sync()
+        ctx.close()
+        assert (L.fake_layout(), L.fake_tables()) == want
+
+
 # ------------------------------------------------------------------ GPU
 def _ranges(P):
     outer = P.R // P.radix[0]
