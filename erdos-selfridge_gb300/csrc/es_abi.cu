@@ -408,8 +408,8 @@ uint32_t longest_of(const EsInst& I, uint32_t strip) {
 // Ring-1 cycles per lane and warp-unit of a launch of `steps` warp-wide cycles, at most the caller's;
 // units(s) is the number of units at s, longest(s) the longest of them.  A unit costs about half a
 // cycle to set up, so long ones are better; but a warp takes as long for a unit when the SM is half
-// empty as when it is full, so a launch of few waves takes whole ones.  Measured (3040 resident
-// warps): k = 300, 2^30 positions 103 us in 1.9 waves of 7 cycles, 117 in 4.4 of 3, 141 in 13.3 of 1;
+// empty as when it is full, so a launch of few waves takes whole ones.  Measured when the rule was made
+// (3040 resident warps): k = 300, 2^30 positions 103 us in 1.9 waves of 7 cycles, 117 in 4.4 of 3, 141 in 13.3 of 1;
 // 2^34 positions 1470 at 7, 1723 at 2; k = 384, 2^28 positions 67 us in 1.5 waves of 1, 127 in 0.2 of 8.
 template <class Units, class Longest>
 uint32_t launch_strip(uint64_t steps, const es_tune& t, const Units& units, const Longest& longest) {

@@ -355,7 +355,8 @@ uint64_t xorshift(uint64_t& s) {
 // warp take consecutive rows of ring 3's digits, so their phases are, wraps apart, an arithmetic
 // progression whose difference is an accident of the wheel: a difference with many factors of two
 // puts all lanes on the same few banks, an odd one spreads them better than chance.  So the library
-// tries multipliers on sampled warps and takes the one with the fewest wavefronts.  2^34 positions:
+// tries multipliers on sampled warps and takes the one with the fewest wavefronts.  2^34 positions,
+// without and with them:
 // k = 384 2200 -> 1636 us, k = 390 1585 -> 1482, k = 379 1775 -> 1727, k = 300 1356 -> 1323.
 constexpr uint32_t kSampleWarps = 8;
 
@@ -416,7 +417,12 @@ uint32_t spread_of(const std::vector<u128>& b3, uint64_t& seed, uint32_t d, uint
 }
 
 // Bytes the inner tables may take: what the CTA has left, and no more than staging them is worth.
-// Every CTA copies them at launch, so a plan whose whole block is a short scan keeps them small.
+// Every CTA copies them at launch, so a plan whose whole block is a short scan keeps them small.  One
+// block alone, and 64 in one launch, with 12, 48 and 144 KB, us: 2^15.1 positions (k = 92) 20.7, 18.7, 19.2
+// and 46, 39, 42; 2^17.2 (k = 124) 21.7, 20.4, 21.1 and 43, 39, 47; 2^20.8 (k = 112) 21.2, 20.8, 21.0 and 64, 65,
+// 64; 2^22.4 (k = 152) 24.5, 23.7, 24.6 and 152, 137, 124; one block of 2^26.2 (k = 168) 34.5, 33.3, 31.4, of
+// 2^28.0 (k = 176) 53.5, 43.3, 44.1, of 2^29.8 (k = 212) 125, 117, 97.  (So the lower line could lie at 2^21
+// and the middle step matters little; single blocks hardly tell 12 from 144 KB below 2^25.)
 uint32_t table_bytes(uint64_t R, size_t smem_bytes, size_t small_bytes) {
     const size_t left = smem_bytes > small_bytes ? smem_bytes - small_bytes : 0;
     const size_t want = R < (1ull << 22) ? 12u << 10 : (R < (1ull << 28) ? 48u << 10 : 144u << 10);

@@ -34,11 +34,13 @@
 // ready warps (k = 300, 2^34 positions: 1469 against 1369 us), 24 at 80 spill in wide rings (k = 379:
 // 2209 against 1842 us).
 //
-// What bounds it: shared-memory wavefronts (l1tex 82 to 90 % busy), then the ALU pipe (66 to 75 %) and
-// instruction issue (60 to 70 %).  Through the drop-in calls, against the caller's cascade by word-mask
-// or pair tables (es_scan_kernel.cuh): k = 300, 2^34 positions 3069 -> 1376 us, 2^30 positions 319 -> 155
-// us; the three-word k = 379 wheel, 2^34 positions, 5506 -> 1752 us; both k = 390 wheels, 2^35 positions
-// each, 17,024 -> 5585 us (their caller-order tables, 1.75 MB per wheel, came through L2).
+// What bounds it: shared-memory wavefronts (l1tex 87 to 90 % busy, a third of them bank conflicts), then
+// the ALU pipe (57 to 66 %) and instruction issue (62 to 72 %).  Through the drop-in calls, against the caller's cascade by word-mask
+// or pair tables (es_scan_kernel.cuh): k = 300, 2^34 positions 3069 -> 1359 us (1290 of
+// them the kernel), 2^30 positions 319 -> 155 (102); the three-word k = 379 wheel, 2^34 positions, 5506 ->
+// 1730 (1661); both k = 390 wheels, 2^35 positions each, 17,024 -> 5580 us (5497; their caller-order
+// tables, 1.75 MB per wheel, came through L2).  Figures beside single choices, here and in the host
+// code, compare their two sides with the kernel of the day and are not its time now.
 #pragma once
 #include "es_scan_kernel.cuh"
 
