@@ -873,6 +873,7 @@ int es_set_capacity(es_ctx* c, uint64_t cap) {
     ES_CUDA(cudaStreamSynchronize(c->stream), "sync");
     cudaFree(c->d_surv);
     c->d_surv = nullptr;
+    c->surv_cap = 0;   // until there is a new one, launches count and store nothing
     ES_CUDA(cudaMalloc(&c->d_surv, sizeof(es_survivor) * cap), "cudaMalloc(survivors)");
     c->surv_cap = cap;
     return ES_OK;
@@ -995,6 +996,7 @@ int es_launch_list(es_ctx* c, const uint64_t* outer, uint64_t n) {
     if (n > c->list_cap) {
         cudaFree(c->d_list);
         c->d_list = nullptr;
+        c->list_cap = 0;
         ES_CUDA(cudaMalloc(&c->d_list, 8ull * n), "cudaMalloc(list)");
         c->list_cap = n;
     }

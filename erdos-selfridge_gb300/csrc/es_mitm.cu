@@ -649,7 +649,8 @@ int es_mitm_set_capacity(es_mitm* m, uint64_t cap) {
     if (!m || cap == 0 || cap > (1ull << 32)) return mfail(ES_ERR_ARG, "capacity must be in [1, 2^32]");
     ES_MCUDA(cudaStreamSynchronize(m->stream), "sync");
     cudaFree(m->d_out);
-    m->d_out = nullptr;
+    m->d_out = m->P.out = nullptr;
+    m->cap = m->P.out_cap = 0;   // until there is a new one, scans count and store nothing
     ES_MCUDA(cudaMalloc(&m->d_out, sizeof(uint4) * cap), "cudaMalloc(survivors)");
     m->cap = cap;
     m->P.out = m->d_out;

@@ -12,6 +12,7 @@
 //                   tables and the layout of the last scan
 //   fake_fail_alloc(n)  the library's n-th host allocation from now on throws std::bad_alloc (0: none);
 //                   returns how far an earlier request still was from failing (0: it has failed)
+//   (device allocations of 32 GB and more are refused)
 //   fake_live()     device and pinned allocations that have not been freed
 #include <cuda_runtime.h>
 
@@ -86,7 +87,7 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) { memset(p, 0, sizeo
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-    *p = aligned_alloc(256, (n + 511) / 256 * 256);
+    *p = n < 32ull << 30 ? aligned_alloc(256, (n + 511) / 256 * 256) : nullptr;
     if (*p && n <= (64u << 20)) memset(*p, 0xcd, n);
     live += *p != nullptr;
     return *p ? cudaSuccess : cudaErrorMemoryAllocation;
@@ -168,6 +169,7 @@ int es_launch_scan(const EsLaunch& L, int layout, int, uint32_t, int, void* stre
     layouts = layout;
     EsLaunch l = L;
     if (!l.items) put(s, [=] {
+        if (!l.surv && l.surv_cap) ++faults;   // records would go to a null pointer
         if (*l.unit_counter != 0 || *l.ctas_done != 0) ++faults;
         // the plan's header and tables are there
         const EsInst& I = *l.item0.inst;

@@ -49,3 +49,24 @@ def test_failed_allocations_come_back_as_codes(tmp_path, what, at_least):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
     assert int(r.stdout.split()[-1]) >= at_least
+
+
+def test_a_capacity_that_does_not_fit_leaves_no_buffer_to_write_to(tmp_path):
+    """The old buffer is gone when the new one is refused: launches then count survivors and store none,
+    and reading them says so."""
+    import es_gb300
+    import es_native as N
+    with fake_lib.bound(fake_lib.build(tmp_path)) as L:
+        ctx = N.Context(es_gb300.Plan(60), N.make_tune(mask_filters=2, count_stages=0))
+        ctx.set_block(0)
+        before = L.fake_faults()
+        with pytest.raises(N.EsError):
+            ctx.set_capacity(1 << 32)
+        ctx.launch(0, ctx.n_outer)
+        ctx.sync()
+        assert L.fake_faults() == before
+        ctx.set_capacity(1 << 10)
+        ctx.launch(0, ctx.n_outer)
+        ctx.sync()
+        assert L.fake_faults() == before
+        ctx.close()
