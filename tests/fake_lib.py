@@ -2,6 +2,7 @@
 bound to it for the length of a `with` block.  Test infrastructure only."""
 import contextlib
 import ctypes as C
+import importlib.util
 import os
 import subprocess
 
@@ -9,8 +10,10 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def build(out_dir) -> str:
-    import es_native
-    es_native.lib()   # the objects below are those of the built library
+    spec = importlib.util.spec_from_file_location("es_build", os.path.join(ROOT, "erdos-selfridge_gb300", "build.py"))
+    es_build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(es_build)
+    es_build.build()   # the objects below are those of the library
     obj = os.path.join(ROOT, "erdos-selfridge_gb300", "_build")
     so = os.path.join(str(out_dir), "libfake.so")
     cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
